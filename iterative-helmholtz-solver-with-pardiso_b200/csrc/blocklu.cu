@@ -8,12 +8,15 @@
 // D_j tridiagonal (x couplings cmx/cpx, diagonal -(cmx+cpx) - (cmy+cpy)
 // + omega^2 s0^2 (1 + i beta) - kz^2).  The y couplings are scalars per line
 // (alpha_y depends on j only), so the Schur recurrence is
-//   S_0 = D_0,   S_j = D_j - cmy[j] cpy[j-1] G_{j-1},   G_j = S_j^{-1}.
+//   S_0 = D_0,   S_j = D_j - cmy[j] cpy[j-1] G_{j-1},   G_j = S_j^{-1},
+// run from both ends towards the middle line (chain.cuh): one launch factors
+// the two halves of every kz as independent chains, a second one the middle
+// lines, each from its two neighbours' G.
 // Each G_j is formed by Gauss-Jordan elimination with partial pivoting
 // (rows chosen among the not yet pivoted ones by max |re| + |im|) and
 // stored transposed (G_j^T row-major) for the sweep.
 //
-// Execution: one thread-block cluster of C CTAs per kz, all ny lines in
+// Execution: one thread-block cluster of C CTAs per (kz, half), its lines in
 // sequence.  The NP x NP block (n padded with an identity) lives in
 // registers: lane l of every warp owns rows l, l+32, ...; CTA q, warp w owns
 // columns q*NPC + w*CB + [0, CB).  At pivot step k the warp owning column k
@@ -30,6 +33,7 @@
 
 #include <cstdint>
 
+#include "chain.cuh"
 #include "cplx.cuh"
 #include "helm3d_internal.h"
 #include "ptx.cuh"
@@ -54,15 +58,16 @@ template <typename R> struct FactorK {
     const cplx<R> *kz2;  // complex shift of mode kz
     int *status;
     const int *kzslot;   // >= 0: a skipped mode (nothing to do), or null
+    int middle;          // 0: the halves, 1: the middle lines
 };
 
 template <typename R> __device__ __forceinline__ R cabs1(cplx<R> a) { return fabs(a.x) + fabs(a.y); }
 
-// bounded wait on a local mbarrier; cluster-scope acquire only when other
-// CTAs of the cluster arrive on it
+// bounded wait of a warp on a local mbarrier; cluster-scope acquire only when
+// other CTAs of the cluster arrive on it
 template <int C> __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity) {
-    if constexpr (C == 1) return mbar_wait_bounded_cta(addr, parity, kWaitLimit);
-    else return mbar_wait_bounded_cluster(addr, parity, kWaitLimit);
+    if constexpr (C == 1) return mbar_wait_warp_cta(addr, parity, kWaitLimit);
+    else return mbar_wait_warp_cluster(addr, parity, kWaitLimit);
 }
 
 // Predicated selects in inline PTX.  Written as plain `if (a == q) x = S[q]`
@@ -138,16 +143,19 @@ __global__ void __launch_bounds__(NW * 32, MB) factor_kernel(FactorK<R> a) {
     Smem<R> sm = carve<R, NP, NPC>(smem_raw);
 
     const uint32_t rank = (C > 1) ? cluster_ctarank() : 0u;
-    const int kz = blockIdx.x / C;
+    const int piece = blockIdx.x / C;
+    const int kz = a.middle ? piece : piece >> 1;
+    const HalfChain hc(a.ny, a.middle ? 0 : piece & 1);
     if (a.kzslot && a.kzslot[kz] >= 0) return;   // a skipped mode (kz_skip_ratio): not factored / swept
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int n = a.n, ny = a.ny;
+    const int lane = threadIdx.x & 31, warp = warp_index();
+    const int n = a.n, lines = a.middle ? 1 : hc.K;
+    const Cx *cin = hc.half ? a.cpy : a.cmy, *cout = hc.half ? a.cmy : a.cpy;
     const int col0 = (int)rank * NPC + warp * CB;
     bool dead = false;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kRing; s++) {
-            mbar_init(&sm.full[s], 32);
+            mbar_init(&sm.full[s], 1);
             mbar_init(&sm.empty[s], NW * C);
         }
         fence_mbar_init_cluster();
@@ -159,11 +167,18 @@ __global__ void __launch_bounds__(NW * 32, MB) factor_kernel(FactorK<R> a) {
     Cx S[RB][CB];
     long t = 0;  // global pivot step counter (line * n + k)
 
-    for (int line = 0; line < ny; line++) {
-        // ---- S_line = D_line - cmy[line] cpy[line-1] G_{line-1}
+    for (int ls = 0; ls < lines; ls++) {
+        const int line = a.middle ? hc.mid : hc.line(ls);
+        // ---- S_line = D_line - cin[line] cout[prev] G_prev; the middle
+        // line: minus both neighbours' terms, their G read from global memory
         {
             const Cx cyd = mkc<R>(-(a.cmy[line].x + a.cpy[line].x), -(a.cmy[line].y + a.cpy[line].y));
-            const Cx cc = line > 0 ? cmul(a.cmy[line], a.cpy[line - 1]) : mkc<R>(0, 0);
+            const Cx cc = ls > 0 ? cmul(cin[line], cout[hc.line(ls - 1)]) : mkc<R>(0, 0);
+            const bool lo = a.middle && line > 0, hi = a.middle && line + 1 < a.ny;
+            const Cx clo = lo ? cmul(a.cmy[line], a.cpy[line - 1]) : mkc<R>(0, 0);
+            const Cx chi = hi ? cmul(a.cpy[line], a.cmy[line + 1]) : mkc<R>(0, 0);
+            const Cx *glo = a.Gt + ((long)kz * a.ny + line - 1) * (long)n * a.ldg;
+            const Cx *ghi = glo + 2 * (long)n * a.ldg;
 #pragma unroll
             for (int ra = 0; ra < RB; ra++) {
                 const int i = lane + 32 * ra;
@@ -174,10 +189,12 @@ __global__ void __launch_bounds__(NW * 32, MB) factor_kernel(FactorK<R> a) {
                     if (i >= n || j >= n) {
                         if (i == j) v = mkc<R>(1, 0);
                     } else {
-                        if (line > 0) {
+                        if (ls > 0) {
                             Cx gij = sm.sGT[(warp * CB + b) * NP + i];
                             v = mkc<R>(-(cc.x * gij.x - cc.y * gij.y), -(cc.x * gij.y + cc.y * gij.x));
                         }
+                        if (lo) v = cfms(clo, glo[(long)j * a.ldg + i], v);
+                        if (hi) v = cfms(chi, ghi[(long)j * a.ldg + i], v);
                         if (i == j) {
                             Cx d = cadd(cadd(cyd, a.base2d[(long)line * n + i]), kzv);
                             d.x -= a.cmx[i].x + a.cpx[i].x;
@@ -243,7 +260,7 @@ __global__ void __launch_bounds__(NW * 32, MB) factor_kernel(FactorK<R> a) {
                     sm.ringr[s] = r;
                     sm.perm[k] = r;
                 }
-                mbar_arrive_local(&sm.full[s]);
+                mbar_arrive_warp(&sm.full[s]);
             } else {
                 const uint32_t a_col = smem_u32(&sm.ringcol[s * NP]);
                 const uint32_t a_pv = smem_u32(&sm.ringpv[s]);
@@ -263,7 +280,7 @@ __global__ void __launch_bounds__(NW * 32, MB) factor_kernel(FactorK<R> a) {
                     }
                 }
 #pragma unroll
-                for (int q = 0; q < C; q++) mbar_arrive_cluster(mapa_u32(a_full, q));
+                for (int q = 0; q < C; q++) mbar_arrive_warp_cluster(mapa_u32(a_full, q));
             }
         };
         auto owns = [&](int k) { return (int)rank == k / NPC && warp == (k % NPC) / CB; };
@@ -325,18 +342,17 @@ __global__ void __launch_bounds__(NW * 32, MB) factor_kernel(FactorK<R> a) {
 #pragma unroll
             for (int b = 0; b < CB; b++)
                 if (!ahead || b != obn) update_col(b);
-            __syncwarp();
             // Release slot s on the `empty` barrier of every CTA: whichever CTA
             // produces the next step that uses slot s, its barrier has then
             // completed exactly one phase per use of the slot, so the producer
             // can wait on the parity of the global step count.
-            if (lane == 0 && (t + kRing) / n < ny) {
+            if (t + kRing < (long)lines * n) {
                 if constexpr (C == 1) {
-                    mbar_arrive_local(&sm.empty[s]);
+                    mbar_arrive_warp(&sm.empty[s]);
                 } else {
                     const uint32_t a_empty = smem_u32(&sm.empty[s]);
 #pragma unroll
-                    for (int q = 0; q < C; q++) mbar_arrive_cluster(mapa_u32(a_empty, (uint32_t)q));
+                    for (int q = 0; q < C; q++) mbar_arrive_warp_cluster(mapa_u32(a_empty, (uint32_t)q));
                 }
             }
         }
@@ -371,7 +387,7 @@ __global__ void __launch_bounds__(NW * 32, MB) factor_kernel(FactorK<R> a) {
         }
         if (C > 1) cluster_sync_all();
         else __syncthreads();
-        cplx<R> *gout = a.Gt + ((long)kz * ny + line) * (long)n * a.ldg;
+        cplx<R> *gout = a.Gt + ((long)kz * a.ny + line) * (long)n * a.ldg;
         for (int idx = threadIdx.x; idx < NPC * n; idx += NW * 32) {
             const int jl = idx / n, i = idx - jl * n;
             const int jg = (int)rank * NPC + jl;
@@ -384,6 +400,7 @@ __global__ void __launch_bounds__(NW * 32, MB) factor_kernel(FactorK<R> a) {
 template <typename R, int NP, int NW, int CB, int C, int MB>
 static int launch_cfg(const FactorArgs &fa, cudaStream_t st) {
     FactorK<R> k;
+    k.middle = fa.middle;
     k.n = fa.n;
     k.ny = fa.ny;
     k.nz = fa.nz;
@@ -402,7 +419,7 @@ static int launch_cfg(const FactorArgs &fa, cudaStream_t st) {
     if (!smem_limit_max(kern, smem))
         return HELM3D_ERR_CUDA;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(fa.nz * C), 1, 1);
+    cfg.gridDim = dim3((unsigned)((fa.middle ? 1 : 2) * fa.nz * C), 1, 1);
     cfg.blockDim = dim3(NW * 32, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -471,7 +488,7 @@ int factor_variants(bool c64, int n) {
 
 bool factor_supported(bool c64, int n) { return n >= 1 && factor_variants(c64, n) > 0; }
 
-int launch_factor(bool c64, const FactorArgs &fa, cudaStream_t s, int variant) {
+static int launch_factor_part(bool c64, const FactorArgs &fa, cudaStream_t s, int variant) {
     int first, count;
     if (c64) shapes_for(kShapes64, fa.n, first, count);
     else shapes_for(kShapes128, fa.n, first, count);
@@ -480,6 +497,16 @@ int launch_factor(bool c64, const FactorArgs &fa, cudaStream_t s, int variant) {
     if (variant == count && factor_tc2_supported(c64, fa.n)) return launch_factor_tc2(fa, s);
     if (variant < 0 || variant >= count) variant = 0;
     return (c64 ? kShapes64 : kShapes128)[first + variant].fn(fa, s);
+}
+
+// the halves of every kz, then the middle lines, which read both halves' last G
+int launch_factor(bool c64, const FactorArgs &fa, cudaStream_t s, int variant) {
+    FactorArgs part = fa;
+    part.middle = 0;
+    const int rc = launch_factor_part(c64, part, s, variant);
+    if (rc) return rc;
+    part.middle = 1;
+    return launch_factor_part(c64, part, s, variant);
 }
 
 }  // namespace h3d

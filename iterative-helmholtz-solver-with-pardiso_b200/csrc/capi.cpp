@@ -512,10 +512,6 @@ int helm3d_apply_prec_batch(helm3d_ctx *c, const double *x, double *y, int nrhs,
     if (xa.rc) return xa.rc;
     VecArg ya(c, y, cnt, false, &c->d_u, &c->u_cap);
     if (ya.rc) return ya.rc;
-    // the sweep shape: forced (HELM3D_FORCE_SWEEP), else the one the last
-    // solve of this context was tuned to
-    const int forced = tune_forced("SWEEP");
-    if (forced >= 0) c->tv_sweep[adjoint ? 1 : 0] = forced < kSweepVariants ? forced : 0;
     const VecBatch xb{xa.dev, c->N}, yb{ya.dev, c->N};
     const ScaleBatch one{nullptr, 0};
     int rc = adjoint ? apply_prec_adjoint(c, xb, 1.0, one, yb, nrhs) : apply_prec(c, xb, 1.0, one, yb, nrhs);

@@ -4,8 +4,9 @@
 // updates on the 5th-generation tensor cores (tcgen05, kind::tf32, 3xTF32).
 // Same recurrence (replacing PARDISO phases 11/22, Source/FGMRES.cpp:274-284,
 // and DirFactFastDiagStructOnline, Source/HODLR/BinaryTreesHODLR.cpp:
-// 2870-2969): S_0 = D_0, S_j = D_j - cmy[j] cpy[j-1] G_{j-1}, G_j = S_j^{-1},
-// by Gauss-Jordan with partial pivoting (the pivot of column k is the row,
+// 2870-2969), from both ends towards the middle line (chain.cuh: one launch
+// for the halves, one for the middle lines): S_0 = D_0, S_j = D_j - cin[j]
+// cout[prev] G_prev, G_j = S_j^{-1}, by Gauss-Jordan with partial pivoting (the pivot of column k is the row,
 // among those not yet pivoted, with the largest |re| + |im|; ties to the
 // lowest row), G_j^T written row-major for the sweep.
 //
@@ -20,7 +21,7 @@
 // block in TMEM; the panel's own columns, which that product does not
 // describe, are then rewritten from registers.
 //
-// Layout per CTA (one CTA per kz, all ny lines in sequence):
+// Layout per CTA (one CTA per (kz, half), its lines in sequence):
 //   TMEM (512 columns x 128 lanes): the block M (lane i = row i, column
 //     2j / 2j + 1 = Re / Im M[i][j]) at [0, 256); X hi at [256, 288), X lo at
 //     [288, 320) (lane i, column 2kk + re/im);
@@ -37,6 +38,7 @@
 
 #include <cstdint>
 
+#include "chain.cuh"
 #include "cplx.cuh"
 #include "helm3d_internal.h"
 #include "ptx.cuh"
@@ -100,13 +102,19 @@ __device__ __forceinline__ void ft_row_barrier() {
     asm volatile("bar.sync 1, %0;" ::"n"(kFtRowWarps * 32) : "memory");
 }
 
+// MID: the middle lines (one launch) instead of the halves: a kernel of its
+// own, so that the halves' loop does not carry the middle line\'s code
+template <bool MID>
 __global__ void __launch_bounds__(kFtThreads, 1) factor_tc_kernel(FactorTcK a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     FtSmem sm = ft_carve(smem_raw);
-    const int n = a.n, ny = a.ny;
-    const int kz = blockIdx.x;
+    const int n = a.n;
+    const int kz = MID ? blockIdx.x : blockIdx.x >> 1;
+    const HalfChain hc(a.ny, MID ? 0 : blockIdx.x & 1);
+    const int lines = MID ? 1 : hc.K;
+    const float2 *cin = hc.half ? a.cpy : a.cmy, *cout = hc.half ? a.cmy : a.cpy;
     if (a.kzslot && a.kzslot[kz] >= 0) return;   // a skipped mode (kz_skip_ratio): not factored / swept
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
     const int npan = (n + kFtB - 1) / kFtB;
     const int ncol = ((n + 7) / 8) * 8;          // complex columns the GEMM covers (N = 2 ncol, a multiple of 16)
 
@@ -136,7 +144,7 @@ __global__ void __launch_bounds__(kFtThreads, 1) factor_tc_kernel(FactorTcK a) {
             const uint32_t sbo = (uint32_t)(2 * kFtB / 4) * 128u;
             const uint32_t bhi = smem_u32(sm.Bhi), blo = smem_u32(sm.Blo);
             uint32_t ph = 0;
-            for (int line = 0; line < ny; line++) {
+            for (int ls = 0; ls < lines; ls++) {
                 for (int p = 0; p < npan; p++) {
                     wait(sm.b_ready, ph);
                     tc_fence_after();
@@ -162,11 +170,18 @@ __global__ void __launch_bounds__(kFtThreads, 1) factor_tc_kernel(FactorTcK a) {
         const uint32_t trow = tmem + ((uint32_t)(32 * warp) << 16);
         uint32_t ph = 0;
         const float2 kzv = a.kz2[kz];
-        for (int line = 0; line < ny; line++) {
-            // ---- S_line = D_line - cmy[line] cpy[line-1] G_{line-1} into TMEM
+        for (int ls = 0; ls < lines; ls++) {
+            const int line = MID ? hc.mid : hc.line(ls);
+            // ---- S_line = D_line - cin[line] cout[prev] G_prev into TMEM; the
+            // middle line: minus both neighbours' terms, their G from global memory
             {
                 const float2 cyd = make_float2(-(a.cmy[line].x + a.cpy[line].x), -(a.cmy[line].y + a.cpy[line].y));
-                const float2 cc = line > 0 ? cmul(a.cmy[line], a.cpy[line - 1]) : make_float2(0.f, 0.f);
+                const float2 cc = ls > 0 ? cmul(cin[line], cout[hc.line(ls - 1)]) : make_float2(0.f, 0.f);
+                const bool lo = MID && line > 0, hi = MID && line + 1 < a.ny;
+                const float2 clo = lo ? cmul(a.cmy[line], a.cpy[line - 1]) : make_float2(0.f, 0.f);
+                const float2 chi = hi ? cmul(a.cpy[line], a.cmy[line + 1]) : make_float2(0.f, 0.f);
+                const float2 *glo = a.Gt + ((long)kz * a.ny + line - 1) * (long)n * a.ldg;
+                const float2 *ghi = glo + 2 * (long)n * a.ldg;
                 float2 diag = make_float2(0.f, 0.f), sub = diag, sup = diag;
                 if (t < n) {
                     diag = cadd(cadd(cyd, a.base2d[(long)line * n + t]), kzv);
@@ -186,10 +201,12 @@ __global__ void __launch_bounds__(kFtThreads, 1) factor_tc_kernel(FactorTcK a) {
                         if (t >= n || j >= n) {
                             if (t == j) s = make_float2(1.f, 0.f);
                         } else {
-                            if (line > 0) {
+                            if (ls > 0) {
                                 const float2 g = grow[j];
                                 s = make_float2(-(cc.x * g.x - cc.y * g.y), -(cc.x * g.y + cc.y * g.x));
                             }
+                            if (lo) s = cfms(clo, glo[(long)j * a.ldg + t], s);
+                            if (hi) s = cfms(chi, ghi[(long)j * a.ldg + t], s);
                             if (j == t) s = cadd(s, diag);
                             else if (j == t + 1) s = cadd(s, sup);
                             else if (j == t - 1) s = cadd(s, sub);
@@ -372,10 +389,12 @@ __global__ void __launch_bounds__(kFtThreads, 1) factor_tc_kernel(FactorTcK a) {
                     reinterpret_cast<float4 *>(sm.Blo)[u] = l;
                 }
                 fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_local(sm.b_ready);
+                mbar_arrive_warp(sm.b_ready);
                 // ---- M += X B^T done: rewrite the panel's own columns
-                wait(sm.mma_done, ph);
+                if (!dead && !mbar_wait_warp_cta(smem_u32(sm.mma_done), ph, kFtWaitLimit)) {
+                    dead = true;
+                    atomicOr(a.status, 2);
+                }
                 ph ^= 1u;
                 tc_fence_after();
                 {
@@ -413,7 +432,7 @@ __global__ void __launch_bounds__(kFtThreads, 1) factor_tc_kernel(FactorTcK a) {
             ft_row_barrier();
             // ---- G_line^T to global: row m of G^T = column m of G
             if (t < n) {
-                float2 *gout = a.Gt + ((long)kz * ny + line) * (long)n * a.ldg;
+                float2 *gout = a.Gt + ((long)kz * a.ny + line) * (long)n * a.ldg;
                 const float2 *grow = sm.G + (size_t)t * kFtGld;
                 for (int m = 0; m < n; m++) gout[(long)m * a.ldg + t] = grow[m];
             }
@@ -443,9 +462,9 @@ int launch_factor_tc(const FactorArgs &fa, cudaStream_t st) {
     k.kz2 = (const float2 *)fa.kz2;
     k.status = fa.status;
     k.kzslot = fa.kzslot;
-    if (!smem_limit_max(factor_tc_kernel, kFtSmemBytes))
-        return HELM3D_ERR_CUDA;
-    factor_tc_kernel<<<dim3((unsigned)fa.nz), kFtThreads, kFtSmemBytes, st>>>(k);
+    void (*kern)(FactorTcK) = fa.middle ? factor_tc_kernel<true> : factor_tc_kernel<false>;
+    if (!smem_limit_max(kern, kFtSmemBytes)) return HELM3D_ERR_CUDA;
+    kern<<<dim3((unsigned)((fa.middle ? 1 : 2) * fa.nz)), kFtThreads, kFtSmemBytes, st>>>(k);
     return cudaGetLastError() == cudaSuccess ? HELM3D_OK : HELM3D_ERR_CUDA;
 }
 

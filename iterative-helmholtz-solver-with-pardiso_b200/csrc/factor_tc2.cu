@@ -1,11 +1,13 @@
 // factor_tc2.cu -- the block-tridiagonal factor of blocklu.cu for complex64
-// blocks of 128 < n <= 224 on a pair of CTAs per kz (a thread-block cluster
+// blocks of 128 < n <= 224 on a pair of CTAs per (kz, half) (a thread-block cluster
 // of 2), the block resident in the two CTAs' tensor memory and the trailing
 // updates of the panel-blocked Gauss-Jordan elimination on the tensor cores
 // (tcgen05, kind::tf32, 3xTF32).  Same recurrence as blocklu.cu and
 // factor_tc.cu (replacing PARDISO phases 11/22, Source/FGMRES.cpp:274-284, and
 // DirFactFastDiagStructOnline, Source/HODLR/BinaryTreesHODLR.cpp:2870-2969):
-// S_0 = D_0, S_j = D_j - cmy[j] cpy[j-1] G_{j-1}, G_j = S_j^{-1}, by
+// from both ends towards the middle line (chain.cuh: one launch for the
+// halves, one for the middle lines),
+// S_0 = D_0, S_j = D_j - cin[j] cout[prev] G_prev, G_j = S_j^{-1}, by
 // Gauss-Jordan with partial pivoting, G_j^T written row-major for the sweep.
 //
 // Rows.  CTA 0 of the pair holds physical rows [0, n0), CTA 1 rows [n0, n)
@@ -61,6 +63,7 @@
 
 #include <cstdint>
 
+#include "chain.cuh"
 #include "cplx.cuh"
 #include "helm3d_internal.h"
 #include "ptx.cuh"
@@ -168,14 +171,21 @@ __device__ __forceinline__ uint32_t f2_key(float2 v, bool cand, int g) {
     return (__float_as_uint(av) & 0xFFFFFF00u) | (uint32_t)(255 - g);
 }
 
+// MID: the middle lines (one launch) instead of the halves: a kernel of its
+// own, so that the halves' loop does not carry the middle line\'s code
+template <bool MID>
 __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     F2Smem sm = f2_carve(smem_raw);
-    const int n = a.n, ny = a.ny;
-    const uint32_t rank = cluster_ctarank(), peer = rank ^ 1u;
-    const int kz = blockIdx.x >> 1;
+    const int n = a.n;
+    const uint32_t rank = blockIdx.x & 1u, peer = rank ^ 1u;   // the rank in the cluster of two
+    const int piece = blockIdx.x >> 1;
+    const int kz = MID ? piece : piece >> 1;
+    const HalfChain hc(a.ny, MID ? 0 : piece & 1);
+    const int lines = MID ? 1 : hc.K;
+    const float2 *cin = hc.half ? a.cpy : a.cmy, *cout = hc.half ? a.cmy : a.cpy;
     if (a.kzslot && a.kzslot[kz] >= 0) return;   // a skipped mode (kz_skip_ratio): not factored / swept
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
     const int n0 = (n + 1) >> 1;
     const int nr = rank == 0 ? n0 : n - n0;       // rows of this CTA
     const int gbase = rank == 0 ? 0 : n0;
@@ -211,8 +221,15 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
             atomicOr(a.status, 2);
         }
     };
+    // the row warps' waits, whole warps
+    auto wait_warp = [&](uint64_t *bar, uint32_t parity) {
+        if (!dead && !mbar_wait_warp_cta(smem_u32(bar), parity, kF2WaitLimit)) {
+            dead = true;
+            atomicOr(a.status, 2);
+        }
+    };
     auto wait_cluster = [&](uint64_t *bar, uint32_t parity) {
-        if (!dead && !mbar_wait_bounded_cluster(smem_u32(bar), parity, kF2WaitLimit)) {
+        if (!dead && !mbar_wait_warp_cluster(smem_u32(bar), parity, kF2WaitLimit)) {
             dead = true;
             atomicOr(a.status, 2);
         }
@@ -244,7 +261,7 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                 }
             };
             uint32_t ph = 0;
-            for (int line = 0; line < ny; line++) {
+            for (int ls = 0; ls < lines; ls++) {
                 for (int p = 0; p < npan; p++) {
                     wait_cta(sm.b_ready, ph);
                     ph ^= 1u;
@@ -279,9 +296,16 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
         uint32_t ph_pan = 0, ph_y = 0, ph_next = 0, ph_rest = 0;
         int cur = 0;
 
-        // ---- S_0 = D_0 (identity frame)
-        {
-            F2Drow d = f2_drow(a, 0, valid ? g : 0, kzv);
+        // ---- the first line's block in the identity frame: D, and for the
+        // middle line both neighbours' terms, their G from global memory
+        if (lines > 0) {
+            const int line = MID ? hc.mid : hc.line(0);
+            F2Drow d = f2_drow(a, line, valid ? g : 0, kzv);
+            const bool lo = MID && line > 0, hi = MID && line + 1 < a.ny;
+            const float2 clo = lo ? cmul(a.cmy[line], a.cpy[line - 1]) : make_float2(0.f, 0.f);
+            const float2 chi = hi ? cmul(a.cpy[line], a.cmy[line + 1]) : make_float2(0.f, 0.f);
+            const float2 *glo = a.Gt + ((long)kz * a.ny + line - 1) * (long)n * a.ldg + g;
+            const float2 *ghi = glo + 2 * (long)n * a.ldg;
 #pragma unroll 1
             for (int c = 0; c < ncol / 16; c++) {
                 float f[32];
@@ -293,6 +317,8 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                         if (q == g) s = d.diag;
                         else if (q == g - 1) s = d.sub;
                         else if (q == g + 1) s = d.sup;
+                        if (lo) s = cfms(clo, glo[(long)q * a.ldg], s);
+                        if (hi) s = cfms(chi, ghi[(long)q * a.ldg], s);
                     }
                     f[2 * e] = s.x;
                     f[2 * e + 1] = s.y;
@@ -302,12 +328,13 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
             tmem_wait_st();
         }
 
-        for (int line = 0; line < ny; line++) {
+        for (int ls = 0; ls < lines; ls++) {
+            const int line = MID ? hc.mid : hc.line(ls);
             bool used0 = false, used1 = false;
             for (int p = 0; p < npan; p++) {
                 const int k0 = p * kF2B, bl = min(kF2B, n - k0);
                 if (p > 0) {
-                    wait_cta(sm.next_ready, ph_next);
+                    wait_warp(sm.next_ready, ph_next);
                     ph_next ^= 1u;
                 }
                 // ---- this CTA's rows of the panel into both CTAs' PF
@@ -326,8 +353,7 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                             st_cluster_v4f32(rdst + 16u * (uint32_t)e, q4);
                         }
                     }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive_cluster(panbar_peer);
+                    mbar_arrive_warp_cluster(panbar_peer);
                 }
                 f2_row_barrier();
                 wait_cluster(sm.pan_bar, ph_pan);
@@ -468,7 +494,7 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                 // ---- the previous panel's trailing GEMM is done: X and the
                 // panel's own columns of this CTA's rows into TMEM
                 if (p > 0) {
-                    wait_cta(sm.rest_done, ph_rest);
+                    wait_warp(sm.rest_done, ph_rest);
                     ph_rest ^= 1u;
                 }
                 tc_fence_after();
@@ -539,8 +565,7 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                     }
                 }
                 tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(ybar_peer);
+                mbar_arrive_warp_cluster(ybar_peer);
                 f2_row_barrier();
                 wait_cluster(sm.y_bar, ph_y);
                 ph_y ^= 1u;
@@ -569,12 +594,11 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                     bl4[1] = make_float4(l.y, l.x, l.w, l.z);
                 }
                 fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_local(sm.b_ready);
+                mbar_arrive_warp(sm.b_ready);
             }
 
             // ---- the line's last GEMM done: the next frame
-            wait_cta(sm.rest_done, ph_rest);
+            wait_warp(sm.rest_done, ph_rest);
             ph_rest ^= 1u;
             tc_fence_after();
             f2_row_barrier();
@@ -598,18 +622,19 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
             // ---- G_line^T to global in the new frame, and S_{line+1} in place
             {
                 const int i = valid ? rho2[g] : 0;
-                const bool more = line + 1 < ny;
+                const bool more = ls + 1 < lines;
                 float2 cc = make_float2(0.f, 0.f);
                 F2Drow d = {};
                 int qd = -1, qs = -1, qp = -1;
                 if (more) {
-                    cc = cmul(a.cmy[line + 1], a.cpy[line]);
-                    d = f2_drow(a, line + 1, i, kzv);
+                    const int nl = hc.line(ls + 1);
+                    cc = cmul(cin[nl], cout[line]);
+                    d = f2_drow(a, nl, i, kzv);
                     qd = sm.kapinv[i];
                     qs = i > 0 ? sm.kapinv[i - 1] : -1;
                     qp = i + 1 < n ? sm.kapinv[i + 1] : -1;
                 }
-                float2 *gout = a.Gt + ((long)kz * ny + line) * (long)n * a.ldg;
+                float2 *gout = a.Gt + ((long)kz * a.ny + line) * (long)n * a.ldg;
 #pragma unroll 1
                 for (int c = 0; c < ncol / 16; c++) {
                     float f[32];
@@ -661,21 +686,8 @@ int launch_factor_tc2(const FactorArgs &fa, cudaStream_t st) {
     k.kz2 = (const float2 *)fa.kz2;
     k.status = fa.status;
     k.kzslot = fa.kzslot;
-    if (!smem_limit_max(factor_tc2_kernel, kF2SmemBytes)) return HELM3D_ERR_CUDA;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(2 * fa.nz), 1, 1);
-    cfg.blockDim = dim3(kF2Threads, 1, 1);
-    cfg.dynamicSmemBytes = kF2SmemBytes;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, factor_tc2_kernel, k) != cudaSuccess) return HELM3D_ERR_CUDA;
-    return cudaGetLastError() == cudaSuccess ? HELM3D_OK : HELM3D_ERR_CUDA;
+    return launch_pairs(fa.middle ? factor_tc2_kernel<true> : factor_tc2_kernel<false>, (fa.middle ? 1 : 2) * fa.nz,
+                        kF2Threads, kF2SmemBytes, k, st);
 }
 
 }  // namespace h3d

@@ -100,6 +100,7 @@ struct FactorArgs {
     const void *kz2;          // cplx<P>[nz]: complex shift of mode k (-kz^2 or lambda_k)
     int *status;              // device flag: bit 0 = zero pivot
     const int *kzslot = nullptr;   // [nz]: >= 0 for a skipped mode (not factored), or null
+    int middle = 0;           // set by launch_factor: 0 the two halves of every kz, 1 the middle lines (chain.cuh)
 };
 // variant: one of the factor_variants(c64, n) launch shapes (0: the default)
 int launch_factor(bool c64, const FactorArgs &a, cudaStream_t s, int variant = 0);
@@ -123,12 +124,11 @@ struct SweepArgs {
     int R;
     const void *dxy;          // null: S^{-1}; else S^{-H} with the [2][ny][n] alpha_x alpha_y table
     int *status;              // device flag: bit 2 = a bounded wait expired
-    int stage_kb = 16;        // bulk-copy stage of G^T rows (KB, about)
+    int stage_kb = 32;        // bulk-copy stage of G^T rows (KB, about)
     int ring_kb = 200;        // shared-memory ring of stages (KB, at most)
-    int tc_mc = 0;            // complex64, n <= 256: the tensor-core sweep with G^T chunks of tc_mc rows (16, 32)
-    int tc_f16 = 0;           // ... with FP16 hi/lo products (K = 16 per MMA), scaled by gscale
     const float *gscale = nullptr;   // [nz][ny] power-of-two scales of the blocks (launch_gscale)
-    int tc_pack = 0;          // the tensor-core sweep on the packed factor (sweep_tcp.cu)
+    int tc_occ = 0;           // 1, 2: the tensor-core sweep on the packed factor, planned for so many CTAs per SM
+    int tc_stages = 8;        // ... its ring's depth at most
     const void *gpack = nullptr;     // the packed factor (launch_gpack), or null
     // skipped modes (kz_skip_ratio): kzslot[kz] >= 0 marks one (the sweep
     // kernels leave it), kzlist[slot] = kz, kzinv[slot] its inverse diagonal
@@ -147,15 +147,13 @@ int launch_kzinv(bool c64, const int *kzlist, int nskip, int nx, int ny, const v
                  cudaStream_t s);
 int launch_kzskip_apply(bool c64, const SweepArgs &a, cudaStream_t s);
 // the sweep's launch variants the autotuner times: stage and ring sizes of
-// the CUDA-core kernels (0-5), the tensor-core kernel's chunk (6, 7), the
-// tensor-core kernel with FP16 products (8), the tensor-core kernel on the
-// packed factor (9)
+// the CUDA-core kernel (0-5), the tensor-core kernel on the packed factor
+// planned for two CTAs per SM (6, 7) or one (8, 9), ring depths 8 and 4
 constexpr int kSweepVariants = 10;
+int sweep_default(bool c64, int n);   // the variant of an untuned batch
 // power-of-two scale of every complex64 block G_j for the FP16 products
 int launch_gscale(const void *Gt, int n, int ny, int nz, int ldg, float *gscale, cudaStream_t s);
 void sweep_variant(int v, SweepArgs &a);
-bool sweep_tc_supported(const SweepArgs &a);   // shape and shared memory fit
-int launch_sweep_tc(const SweepArgs &a, int mc, cudaStream_t s);
 // the complex64 factor (n <= 256) packed once into FP16 hi/lo tiles of
 // s_j G_j (s_j = gscale) in the tensor core's operand layout, gpack_bytes
 // bytes (about those of the complex64 factor), for launch_sweep_tcp
@@ -301,6 +299,26 @@ template <typename K> inline bool smem_limit_max(K kern, size_t need) {
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap) == cudaSuccess;
 }
 
+// a launch of `pairs` clusters of two CTAs
+template <typename K, typename A>
+inline int launch_pairs(K kern, int pairs, int threads, size_t smem, const A &arg, cudaStream_t st) {
+    if (!smem_limit_max(kern, smem)) return HELM3D_ERR_CUDA;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
+    cfg.blockDim = dim3((unsigned)threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, kern, arg) != cudaSuccess) return HELM3D_ERR_CUDA;
+    return cudaGetLastError() == cudaSuccess ? HELM3D_OK : HELM3D_ERR_CUDA;
+}
+
 // ------------------------------------------------------------- autotuner
 // The fastest of nvariants launch shapes of a kernel family for a problem
 // shape: launch(v) runs variant v once on the context's stream; the choice is
@@ -415,6 +433,7 @@ struct helm3d_ctx {
     // red_blocks)
     int tv_factor = 0;
     int tv_sweep[2] = {0, 0};
+    int tv_sweep_R[2] = {0, 0};                 // the batch tv_sweep was chosen for (0: none yet, sweep_default)
     int tv_stencil = 0;
     int tv_update = 0;
     size_t f_cap = 0, u_cap = 0;                // staging capacities (vectors) of d_f, d_u

@@ -24,6 +24,11 @@ __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+__device__ __forceinline__ void cluster_arrive() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
@@ -80,6 +85,24 @@ __device__ __forceinline__ void bulk_g2s(void *dst_smem, const void *src_gmem, u
         : "memory");
 }
 
+// One element (8 or 16 bytes) copied global -> shared asynchronously by this
+// thread; zero where !valid (the source is then not read)
+template <int B> __device__ __forceinline__ void cp_async_el(void *dst_smem, const void *src, bool valid);
+template <> __device__ __forceinline__ void cp_async_el<16>(void *dst_smem, const void *src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst_smem)), "l"(src),
+                 "r"(valid ? 16 : 0)
+                 : "memory");
+}
+template <> __device__ __forceinline__ void cp_async_el<8>(void *dst_smem, const void *src, bool valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst_smem)), "l"(src),
+                 "r"(valid ? 8 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 __device__ __forceinline__ void st_cluster_v2f32(uint32_t addr, float x, float y) {
     asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(x), "f"(y) : "memory");
 }
@@ -103,6 +126,75 @@ __device__ __forceinline__ bool mbar_wait_bounded_cta(uint32_t addr, uint32_t pa
         if (mbar_try_wait_cta(addr, parity)) return true;
     return false;
 }
+
+// Barrier operations of a whole converged warp, by one predicated lane: a poll
+// or arrive executed by all 32 lanes is done lane by lane (137 cycles for a
+// poll of a completed phase on a B200, and ~190 for one lane's under a branch
+// with the reconvergence after it; 22 this way).  The outcome of a poll is the
+// warp's, and the __syncwarp orders the other lanes' accesses with lane 0's.
+__device__ __forceinline__ bool mbar_poll_warp_cta(uint32_t addr, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.eq.u32 q, %3, 0;\n\t"
+        "setp.ne.u32 p, %3, %3;\n\t"
+        "@q mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(addr), "r"(parity), "r"((uint32_t)(threadIdx.x & 31))
+        : "memory");
+    return __any_sync(0xffffffffu, ok != 0);
+}
+__device__ __forceinline__ bool mbar_poll_warp_cluster(uint32_t addr, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.eq.u32 q, %3, 0;\n\t"
+        "setp.ne.u32 p, %3, %3;\n\t"
+        "@q mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(addr), "r"(parity), "r"((uint32_t)(threadIdx.x & 31))
+        : "memory");
+    return __any_sync(0xffffffffu, ok != 0);
+}
+__device__ __forceinline__ bool mbar_wait_warp_cta(uint32_t addr, uint32_t parity, uint32_t limit) {
+    for (uint32_t it = 0; it < limit; ++it)
+        if (mbar_poll_warp_cta(addr, parity)) {
+            __syncwarp();
+            return true;
+        }
+    return false;
+}
+__device__ __forceinline__ bool mbar_wait_warp_cluster(uint32_t addr, uint32_t parity, uint32_t limit) {
+    for (uint32_t it = 0; it < limit; ++it)
+        if (mbar_poll_warp_cluster(addr, parity)) {
+            __syncwarp();
+            return true;
+        }
+    return false;
+}
+// one arrive for the warp, after every lane's earlier accesses
+__device__ __forceinline__ void mbar_arrive_warp(uint64_t *bar) {
+    __syncwarp();
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.eq.u32 q, %1, 0;\n\t"
+        "@q mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(smem_u32(bar)),
+        "r"((uint32_t)(threadIdx.x & 31))
+        : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_warp_cluster(uint32_t cluster_addr) {
+    __syncwarp();
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.eq.u32 q, %1, 0;\n\t"
+        "@q mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n\t}" ::"r"(cluster_addr),
+        "r"((uint32_t)(threadIdx.x & 31))
+        : "memory");
+}
+// this thread's warp in its (1-D) block, in a form the compiler knows to be warp-uniform
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 
 // A position in a ring of `size` slots: the slot, and the parity of the
 // current pass over the ring (the phase an mbarrier of the slot completes

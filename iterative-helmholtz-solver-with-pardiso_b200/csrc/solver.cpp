@@ -204,7 +204,12 @@ static SweepArgs sweep_args(helm3d_ctx *c, int R, bool adjoint) {
         s.nskip = c->nskip;
         s.kzinv = c->d_kzinv;
     }
-    sweep_variant(c->tv_sweep[adjoint ? 1 : 0], s);
+    // the forced shape, or the one the last solve was tuned to; a batch of one
+    // or two sources (the last of a solve's whose others have retired) whose
+    // lines fit one row block is faster on the CUDA cores
+    const int adj = adjoint ? 1 : 0, forced = tune_forced("SWEEP");
+    const bool tuned = c->tv_sweep_R[adj] > 0 && (R == c->tv_sweep_R[adj] || R >= 3 || s.n > 128);
+    sweep_variant(forced >= 0 ? forced : tuned ? c->tv_sweep[adj] : sweep_default(c->c64, s.n), s);
     return s;
 }
 
@@ -570,7 +575,7 @@ int tune_solve(helm3d_ctx *c, int R, bool adjoint) {
     const bool any_forced = std::getenv("HELM3D_FORCE_SWEEP") || std::getenv("HELM3D_FORCE_STENCIL") ||
                             std::getenv("HELM3D_FORCE_REDUCE") || std::getenv("HELM3D_FORCE_UPDATE");
     if (!tune_enabled() && !any_forced) {
-        c->tv_sweep[0] = c->tv_sweep[1] = 0;
+        c->tv_sweep_R[0] = c->tv_sweep_R[1] = 0;   // sweep_default
         c->tv_stencil = 0;
         c->tv_update = 0;
         c->red_blocks = reduce_blocks(0);
@@ -583,13 +588,16 @@ int tune_solve(helm3d_ctx *c, int R, bool adjoint) {
     // the sweep, in place on zeroed planes of R right-hand sides
     RC(cuda_check(c, cudaMemsetAsync(c->d_planes, 0, (c->c64 ? 8 : 16) * (size_t)N * R, c->stream), "tune planes"));
     const int adj = adjoint ? 1 : 0;
-    std::snprintf(shape, sizeof(shape), "%d|%d|%d|%d|%d|%d", c->c64 ? 64 : 128, g.nx, g.ny, g.nz, R, adj);
+    // (t2: the second numbering of the variants, so that a cache file written
+    // with the first one is not read as this one)
+    std::snprintf(shape, sizeof(shape), "t2|%d|%d|%d|%d|%d|%d", c->c64 ? 64 : 128, g.nx, g.ny, g.nz, R, adj);
     const SweepArgs s0 = sweep_args(c, R, adjoint);
     c->tv_sweep[adj] = tune_pick(c, "SWEEP", shape, kSweepVariants, [&](int v) {
         SweepArgs t = s0;
         sweep_variant(v, t);
         return launch_sweep(c->c64, t, c->stream);
     });
+    c->tv_sweep_R[adj] = tune_enabled() ? R : 0;
     if (c->opts.mode == HELM3D_MODE_N) {
         // the stencil from Z_0 (its FGMRES input: complex64 when the
         // context keeps Z so) into V_1 of every right-hand side

@@ -15,12 +15,9 @@
 
 #include "cplx.cuh"
 #include "helm3d_internal.h"
+#include "ptx.cuh"
 
 namespace h3d {
-
-__device__ __forceinline__ uint32_t smem_u32_st(const void *p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
 
 constexpr int kStX = 32, kStY = 8;
 
@@ -119,23 +116,6 @@ __global__ void __launch_bounds__(kStX *kStY) stencil_kernel(StencilArgs a) {
 // the tile, the z neighbours from the tiles of planes k - 1 (kept in a
 // register) and k + 1.  One CTA barrier per plane.
 constexpr int kSsX = 32, kSsY = 8, kSsHX = kSsX + 2, kSsHY = kSsY + 2, kSsBuf = 4;
-
-// one element of x (B = 16 bytes complex128, 8 bytes complex64)
-template <int B> __device__ __forceinline__ void cp_async_el(void *dst_smem, const void *src, bool valid);
-template <> __device__ __forceinline__ void cp_async_el<16>(void *dst_smem, const void *src, bool valid) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32_st(dst_smem)), "l"(src),
-                 "r"(valid ? 16 : 0)
-                 : "memory");
-}
-template <> __device__ __forceinline__ void cp_async_el<8>(void *dst_smem, const void *src, bool valid) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32_st(dst_smem)), "l"(src),
-                 "r"(valid ? 8 : 0)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
 
 template <bool ADJ, typename TX>
 __global__ void __launch_bounds__(kSsX *kSsY) stencil_smem_kernel(StencilArgs a) {

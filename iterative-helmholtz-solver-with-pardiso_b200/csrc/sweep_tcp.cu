@@ -2,17 +2,16 @@
 // factor packed once, after the block LU factor, into FP16 hi/lo tiles in
 // the tensor core's shared-memory operand layout, so that the sweep streams
 // them by bulk copies straight into the MMAs' A operand: no per-sweep
-// conversion of G and no TMEM copy of it.  Same recurrence as sweep.cu and
-// sweep_tc.cu (the per-kz 2D solve replacing PARDISO phase 33,
+// conversion of G and no TMEM copy of it.  Same two-ended recurrence as
+// sweep.cu (chain.cuh; the per-kz 2D solve replacing PARDISO phase 33,
 // Source/functions.cpp:5959, and DirSolveFastDiagStruct,
-// Source/HODLR/BinaryTreesHODLR.cpp:2971-3018):
-//   forward   y_0 = G_0 f_0,   y_j = G_j (f_j - cmy[j] y_{j-1})
-//   backward  x_{ny-1} = y_{ny-1},   x_j = y_j - cpy[j] G_j x_{j+1}
-// and the same real GEMM per line as sweep_tc.cu,
+// Source/HODLR/BinaryTreesHODLR.cpp:2971-3018): a cluster of two CTAs per kz,
+// CTA h taking half h's lines.  Per line one real GEMM
 //   D[i][2r + c] = sum_K A[i][K] B[2r + c][K],   K = 2m + (re, im),
-// A = s_j G_j (s_j the block's power-of-two scale) as FP16 hi + lo, B the
-// real form of the line's input v scaled per right-hand side by a power of
-// two, as FP16 hi + lo; D = a_hi b_hi + a_hi b_lo + a_lo b_hi in FP32
+// A = s_j G_j (s_j the block's power-of-two scale, so that the largest scaled
+// entry lies in [2^13, 2^14) and the lo halves stay normal) as FP16 hi + lo,
+// B the real form of the line's input v scaled per right-hand side by a power
+// of two, as FP16 hi + lo; D = a_hi b_hi + a_hi b_lo + a_lo b_hi in FP32
 // (kind::f16, K = 16 per MMA), unscaled exactly in the epilogue.
 //
 // Packed factor (launch_gpack): block (kz, j), chunk c (complex m in
@@ -24,10 +23,13 @@
 // rows takes its last rows from whatever shared memory follows; those rows
 // of D are never read.
 //
-// Roles (11 warps): warps 0-7 epilogue (as sweep_tc.cu: D from TMEM, finish
-// the line, the next B), warp 8 one lane: bulk copies of the packed chunks
+// Roles (11 warps): warps 0-7 epilogue (D from TMEM, finish the line, the
+// next B; the line's plane stores after the next B is handed over, off the
+// line-to-line chain), warp 8 one lane: bulk copies of the packed chunks
 // into a ring of stages, warps 9-10 one lane each: the MMAs (A and B from
-// shared memory), split between the two issuers as in sweep_tc.cu, each
+// shared memory; a thread waits ~70 cycles per tcgen05.mma it issues whatever
+// N, and two issuers' MMAs overlap: row block u to issuer u, or with one row
+// block the a_hi and the a_lo products into separate accumulators), each
 // chunk's MMAs committed to the stage's empty barrier.  Every wait is
 // bounded; on expiry bit 2 of *status is set, the producer stops issuing and
 // drains its copies, the issuers wait (bounded) for their MMAs, TMEM is freed
@@ -37,6 +39,7 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "chain.cuh"
 #include "cplx.cuh"
 #include "helm3d_internal.h"
 #include "ptx.cuh"
@@ -83,19 +86,21 @@ template <bool ADJ> __device__ __forceinline__ float2 tp_adj_out(const SweepTpK 
 // RR right-hand sides (8 or 16, padded), MB row blocks of 128 rows.  TMEM:
 // the accumulator of row block rb at columns [2 NR rb, 2 NR (rb + 1)); with
 // one row block the a_lo b_hi products in their own at [2 NR, 3 NR).
-template <int RR, int MB, bool ADJ>
-__global__ void __launch_bounds__(kTpThreads, 1) sweep_tcp_kernel(SweepTpK a) {
+// OCC: CTAs per SM the registers (and, in tp_shape, the ring) are planned for.
+template <int RR, int MB, bool ADJ, int OCC>
+__global__ void __launch_bounds__(kTpThreads, OCC) sweep_tcp_kernel(SweepTpK a) {
     constexpr int NR = 2 * RR;        // B rows = D columns
     constexpr int RH = RR / 2;        // right-hand sides per epilogue warp
     static_assert((MB == 2 ? 4 * NR : 3 * NR) <= (int)kTpCols, "TMEM layout");
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    const int n = a.n, ny = a.ny, Rn = a.nrhs, npad = a.npad, cpl = a.cpl;
+    const int n = a.n, Rn = a.nrhs, npad = a.npad, cpl = a.cpl;
     const int Kp = 2 * npad;
-    const int kz = blockIdx.x;
-    if (a.kzslot && a.kzslot[kz] >= 0) return;   // a skipped mode (kz_skip_ratio): not factored / swept
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nsteps = 2 * ny - 1;
-    const long nseq = (long)nsteps * cpl;
+    const int kz = blockIdx.x >> 1;
+    if (a.kzslot && a.kzslot[kz] >= 0) return;   // a skipped mode (kz_skip_ratio), in both CTAs
+    const uint32_t rank = blockIdx.x & 1u, peer = rank ^ 1u;   // the rank in the cluster of two
+    const HalfChain hc(a.ny, (int)rank);
+    const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
+    const int nsteps = hc.steps();
     const uint32_t stage_bytes = 2 * a.tile_bytes;
 
     unsigned char *ring = smem_raw;
@@ -109,8 +114,9 @@ __global__ void __launch_bounds__(kTpThreads, 1) sweep_tcp_kernel(SweepTpK a) {
     uint64_t *b_full = empty + a.nstage;
     uint64_t *d_full = b_full + 1;
     uint64_t *fin = d_full + 1;                                        // [kTpMmaWarps]
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(fin + kTpMmaWarps);
-    float2 *P = a.planes + (long)kz * ny * Rn * n;   // line j, rhs r, row i at ((j*Rn + r)*n + i)
+    uint64_t *met = fin + kTpMmaWarps, *read = met + 1;                // the peer's epilogue warps arrive on them
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(read + 1);
+    float2 *P = a.planes + (long)kz * a.ny * Rn * n;   // line j, rhs r, row i at ((j*Rn + r)*n + i)
 
     if (warp == 0) tmem_alloc(tslot, kTpCols);
     if (tid == 0) {
@@ -121,10 +127,12 @@ __global__ void __launch_bounds__(kTpThreads, 1) sweep_tcp_kernel(SweepTpK a) {
         mbar_init(b_full, kTpEpiWarps);
         mbar_init(d_full, kTpMmaWarps);
         for (int u = 0; u < kTpMmaWarps; u++) mbar_init(&fin[u], 1);
+        mbar_init(met, kTpEpiWarps);
+        mbar_init(read, kTpEpiWarps);
         fence_mbar_init_cluster();
     }
     tc_fence_before();
-    __syncthreads();
+    cluster_sync_all();   // the peer's barriers exist before the first remote arrive
     tc_fence_after();
     const uint32_t tmem = *tslot;
     bool dead = false;
@@ -139,28 +147,20 @@ __global__ void __launch_bounds__(kTpThreads, 1) sweep_tcp_kernel(SweepTpK a) {
     if (warp == kTpProducerWarp) {
         // ---------------------------------------------------- producer
         if (lane == 0) {
-            // chunk c of step t: forward lines 0..ny-1, then backward lines
-            // ny-2..0; its hi and lo tiles into the first and second half of
-            // the stage
+            // chunk c of step t: its hi and lo tiles into the first and second
+            // half of the stage
             const size_t block_bytes = (size_t)cpl * 2 * a.tile_bytes;
             RingPos rp;
-            int t = 0, c = 0;
             long issued = 0;
-            for (long seq = 0; seq < nseq; seq++) {
-                if (seq >= a.nstage) wait(&empty[rp.slot], rp.phase ^ 1u);
-                if (dead) break;   // stop issuing once a wait has expired
-                const int line = t < ny ? t : 2 * ny - 2 - t;
-                const unsigned char *src =
-                    a.Gp + ((size_t)kz * ny + line) * block_bytes + (size_t)c * 2 * a.tile_bytes;
-                unsigned char *dst = ring + (size_t)rp.slot * stage_bytes;
-                mbar_expect_tx(&full[rp.slot], 2 * a.tile_bytes);
-                bulk_g2s(dst, src, a.tile_bytes, &full[rp.slot]);
-                bulk_g2s(dst + a.tile_bytes, src + a.tile_bytes, a.tile_bytes, &full[rp.slot]);
-                rp.next(a.nstage);
-                issued++;
-                if (++c == cpl) {
-                    c = 0;
-                    t++;
+            for (int t = 0; t < nsteps && !dead; t++) {
+                const unsigned char *src = a.Gp + ((size_t)kz * a.ny + hc.step_line(t)) * block_bytes;
+                for (int c = 0; c < cpl; c++, src += 2 * a.tile_bytes) {
+                    if (issued >= a.nstage) wait(&empty[rp.slot], rp.phase ^ 1u);
+                    if (dead) break;   // stop issuing once a wait has expired
+                    mbar_expect_tx(&full[rp.slot], 2 * a.tile_bytes);
+                    bulk_g2s(ring + (size_t)rp.slot * stage_bytes, src, 2 * a.tile_bytes, &full[rp.slot]);
+                    rp.next(a.nstage);
+                    issued++;
                 }
             }
             // the copies still in flight land before the CTA exits: the
@@ -267,8 +267,7 @@ __global__ void __launch_bounds__(kTpThreads, 1) sweep_tcp_kernel(SweepTpK a) {
                 reinterpret_cast<uint4 *>(Blo)[u] = make_uint4(p0.y, p1.y, p2.y, p3.y);
             }
             fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_local(b_full);
+            mbar_arrive_warp(b_full);
         };
         // this warp's per-right-hand-side maxima of the next v into vmax[q][r]
         // (one writer per entry; every reader of the previous values is past
@@ -283,24 +282,60 @@ __global__ void __launch_bounds__(kTpThreads, 1) sweep_tcp_kernel(SweepTpK a) {
         };
         float sv_cur[RH];   // scales of the v this thread's line is multiplied with
 
-        // line 0's input: f_0 of this thread's rows and right-hand sides
+        const float2 *cin = hc.half ? a.cpy : a.cmy, *cout = hc.half ? a.cmy : a.cpy;
+        // the halves meet at the middle line: this warp's rows of the last
+        // forward y are in the planes; after the peer's, its y may be read
+        auto arrive_peer = [&](uint64_t *bar) { mbar_arrive_warp_cluster(mapa_u32(smem_u32(bar), peer)); };
+        auto wait_cluster = [&](uint64_t *bar) {
+            if (!dead && !mbar_wait_warp_cluster(smem_u32(bar), 0u, kTpWaitLimit)) fail();
+        };
+        // the middle line's input: f minus both neighbours' terms, in one order
+        auto mid_in = [&](float2 f, float2 own, float2 other) {
+            const float2 lo = hc.half ? other : own, hi = hc.half ? own : other;
+            return cfms(a.cpy[hc.mid], hi, cfms(a.cmy[hc.mid], lo, f));
+        };
+        auto peer_y = [&](int r, int row) {
+            return hc.peer_lines() ? P[((long)hc.peer_last() * Rn + r) * n + row] : make_float2(0.f, 0.f);
+        };
+
+        // the first line's input: f of this thread's rows and right-hand sides
+        // (a half without lines starts with the middle one)
         {
             float am[RH];
+            float2 f[MB][RH];
 #pragma unroll
             for (int k = 0; k < RH; k++) am[k] = 0.f;
 #pragma unroll
             for (int rb = 0; rb < MB; rb++) {
-                const int m = i + 128 * rb;
-                if (m >= npad) continue;
+                const int m = i + 128 * rb, line = hc.line(0);
 #pragma unroll
                 for (int k = 0; k < RH; k++) {
                     const int r = wg * RH + k;
-                    const float2 f = (r < Rn && m < n) ? tp_adj_in<ADJ>(a, 0, m, P[(long)r * n + m])
-                                                       : make_float2(0.f, 0.f);
-                    vst[(size_t)r * vld + m] = f;
-                    am[k] = fmaxf(am[k], fmaxf(fabsf(f.x), fabsf(f.y)));
+                    f[rb][k] = r < Rn && m < n ? tp_adj_in<ADJ>(a, line, m, P[((long)line * Rn + r) * n + m])
+                                               : make_float2(0.f, 0.f);
                 }
             }
+            if (hc.K == 0) {
+                arrive_peer(met);
+                wait_cluster(met);
+#pragma unroll
+                for (int rb = 0; rb < MB; rb++)
+#pragma unroll
+                    for (int k = 0; k < RH; k++) {
+                        const int r = wg * RH + k, m = i + 128 * rb;
+                        if (r < Rn && m < n) f[rb][k] = mid_in(f[rb][k], make_float2(0.f, 0.f), peer_y(r, m));
+                    }
+            }
+#pragma unroll
+            for (int rb = 0; rb < MB; rb++) {
+                const int m = i + 128 * rb;
+#pragma unroll
+                for (int k = 0; k < RH; k++) {
+                    if (m < npad) vst[(size_t)(wg * RH + k) * vld + m] = f[rb][k];
+                    am[k] = fmaxf(am[k], fmaxf(fabsf(f[rb][k].x), fabsf(f[rb][k].y)));
+                }
+            }
+            if (hc.K == 0) arrive_peer(read);
             put_vmax(am);
         }
         tp_epilogue_barrier();
@@ -309,26 +344,22 @@ __global__ void __launch_bounds__(kTpThreads, 1) sweep_tcp_kernel(SweepTpK a) {
         build_b();
 
         // What finishing step t needs besides G v, loaded one step ahead (the
-        // planes do not fit in L2): f_{line+1} forward (and its adjoint
+        // planes do not fit in L2): the next line's f forward (and its adjoint
         // scale), y_line backward.  Written by this same thread earlier, or
         // untouched input.  Row i + 128 rb of row block rb.
         auto load_pre = [&](int t, float2 (&v)[MB][RH], float2 (&dx)[MB]) {
-            const bool fwd = t < ny;
-            const int line = fwd ? t : 2 * ny - 2 - t;
-            const bool nxt = fwd && line + 1 < ny;
+            const bool nxt = t < hc.K;
+            const int line = nxt ? hc.line(t + 1) : hc.step_line(t);
 #pragma unroll
             for (int rb = 0; rb < MB; rb++) {
                 const int row = i + 128 * rb;
 #pragma unroll
                 for (int k = 0; k < RH; k++) {
                     const int r = wg * RH + k;
-                    v[rb][k] = make_float2(0.f, 0.f);
-                    if (row < n && r < Rn) {
-                        if (nxt) v[rb][k] = P[((long)(line + 1) * Rn + r) * n + row];
-                        else if (!fwd) v[rb][k] = P[((long)line * Rn + r) * n + row];
-                    }
+                    v[rb][k] = row < n && r < Rn && t != hc.K ? P[((long)line * Rn + r) * n + row]
+                                                             : make_float2(0.f, 0.f);
                 }
-                dx[rb] = (ADJ && nxt && row < n) ? a.dxy[(long)(line + 1) * n + row] : make_float2(0.f, 0.f);
+                dx[rb] = (ADJ && nxt && row < n) ? a.dxy[(long)line * n + row] : make_float2(0.f, 0.f);
             }
         };
         float2 pv[MB][RH], pvn[MB][RH], dx[MB], dxn[MB];
@@ -336,26 +367,34 @@ __global__ void __launch_bounds__(kTpThreads, 1) sweep_tcp_kernel(SweepTpK a) {
 
         for (int t = 0; t < nsteps; t++) {
             if (t + 1 < nsteps) load_pre(t + 1, pvn, dxn);
-            const bool fwd = t < ny;
-            const int line = fwd ? t : 2 * ny - 2 - t;
-            const bool last_fwd = fwd && line + 1 == ny;
-            const float2 cn = (fwd && !last_fwd) ? a.cmy[line + 1] : make_float2(0.f, 0.f);
-            const float2 cp = fwd ? make_float2(0.f, 0.f) : a.cpy[line];
-            const float igs = pow2_inv(a.gscale[(long)kz * ny + line]);
+            const bool fwd = t <= hc.K;
+            const int line = hc.step_line(t);
+            const float2 cc = t + 1 < hc.K ? cin[hc.line(t + 1)] : !fwd ? cout[line] : make_float2(0.f, 0.f);
+            const float igs = pow2_inv(a.gscale[(long)kz * a.ny + line]);
             float us[RH];   // exact unscaling: 1 / (block scale * right-hand-side scale)
 #pragma unroll
             for (int k = 0; k < RH; k++) us[k] = igs * pow2_inv(sv_cur[k]);
             float am[RH];
 #pragma unroll
             for (int k = 0; k < RH; k++) am[k] = 0.f;
-            wait(d_full, (uint32_t)(t & 1));
+            if (!dead && !mbar_wait_warp_cta(smem_u32(d_full), (uint32_t)(t & 1), kTpWaitLimit)) fail();
             tc_fence_after();
             // this line's y / x, stored to the planes after the next B is
             // handed over (the stores are off the line-to-line chain)
             float2 outs[MB][RH];
+            auto store_outs = [&](int to) {
+#pragma unroll
+                for (int rb = 0; rb < MB; rb++) {
+                    const int row = i + 128 * rb;
+#pragma unroll
+                    for (int k = 0; k < RH; k++) {
+                        const int r = wg * RH + k;
+                        if (row < n && r < Rn) P[((long)to * Rn + r) * n + row] = outs[rb][k];
+                    }
+                }
+            };
 #pragma unroll
             for (int rb = 0; rb < MB; rb++) {
-                const int row = i + 128 * rb;
                 // D = a_hi b_hi (+ a_lo b_hi with two row blocks) (columns c) +
                 // a_hi b_lo (columns NR + c); with one row block a_lo b_hi at 2 NR + c
                 const uint32_t dcol = (uint32_t)(rb * 2 * NR + wg * RR);
@@ -378,28 +417,37 @@ __global__ void __launch_bounds__(kTpThreads, 1) sweep_tcp_kernel(SweepTpK a) {
                 }
 #pragma unroll
                 for (int k = 0; k < RH; k++) {
-                    const int r = wg * RH + k;
-                    const float2 pk = pv[rb][k];
-                    const float2 pre = (ADJ && fwd && !last_fwd) ? cmul(dx[rb], make_float2(pk.x, -pk.y)) : pk;
                     const float2 acc = make_float2((d[2 * k] + d[RR + 2 * k] + d3[2 * k]) * us[k],
                                                    (d[2 * k + 1] + d[RR + 2 * k + 1] + d3[2 * k + 1]) * us[k]);
-                    float2 out, vn;
-                    bool fin_x;   // out is this line's final x
-                    if (fwd) {
-                        out = acc;                                        // y_line
-                        fin_x = last_fwd;
-                        vn = fin_x ? out : cfms(cn, out, pre);            // f_{line+1} - cmy y_line, or x_{ny-1}
-                    } else {
-                        out = cfms(cp, acc, pre);                         // x_line = y_line - cpy G x_{line+1}
-                        fin_x = true;
-                        vn = out;
-                    }
+                    // y_line, x_mid, or x_line = y_line - cout G x_next
+                    outs[rb][k] = fwd ? acc : cfms(cc, acc, pv[rb][k]);
+                }
+            }
+            if (t == hc.K - 1) {
+                store_outs(line);
+                arrive_peer(met);
+                wait_cluster(met);
+            }
+#pragma unroll
+            for (int rb = 0; rb < MB; rb++) {
+                const int row = i + 128 * rb;
+#pragma unroll
+                for (int k = 0; k < RH; k++) {
+                    const int r = wg * RH + k;
+                    const float2 out = outs[rb][k];
                     const bool valid = row < n && r < Rn;
-                    outs[rb][k] = fin_x ? tp_adj_out<ADJ>(a, line, row, out) : out;
+                    float2 vn = out;
+                    if (t < hc.K) {   // the next line's input
+                        const float2 pk = pv[rb][k];
+                        const float2 f = ADJ ? cmul(dx[rb], make_float2(pk.x, -pk.y)) : pk;
+                        vn = t + 1 < hc.K ? cfms(cc, out, f) : valid ? mid_in(f, out, peer_y(r, row)) : out;
+                    }
+                    if (t >= hc.K) outs[rb][k] = tp_adj_out<ADJ>(a, line, row, out);
                     if (row < npad) vst[(size_t)r * vld + row] = valid ? vn : make_float2(0.f, 0.f);
                     if (valid) am[k] = fmaxf(am[k], fmaxf(fabsf(vn.x), fabsf(vn.y)));
                 }
             }
+            if (t == hc.K - 1) arrive_peer(read);
             tc_fence_before();
             if (t + 1 < nsteps) {
                 put_vmax(am);
@@ -408,15 +456,9 @@ __global__ void __launch_bounds__(kTpThreads, 1) sweep_tcp_kernel(SweepTpK a) {
                 for (int k = 0; k < RH; k++) sv_cur[k] = v_scale(wg * RH + k);
                 build_b();
             }
-#pragma unroll
-            for (int rb = 0; rb < MB; rb++) {
-                const int row = i + 128 * rb;
-#pragma unroll
-                for (int k = 0; k < RH; k++) {
-                    const int r = wg * RH + k;
-                    if (row < n && r < Rn) P[((long)line * Rn + r) * n + row] = outs[rb][k];
-                }
-            }
+            // the peer has read this half's last y before it is overwritten
+            if (t == hc.K + 1) wait_cluster(read);
+            if (t != hc.K - 1 && (t != hc.K || hc.half == 0)) store_outs(line);
 #pragma unroll
             for (int rb = 0; rb < MB; rb++) {
 #pragma unroll
@@ -426,12 +468,41 @@ __global__ void __launch_bounds__(kTpThreads, 1) sweep_tcp_kernel(SweepTpK a) {
         }
     }
     tc_fence_before();
-    __syncthreads();
+    __syncwarp();
+    cluster_sync_all();   // no CTA leaves while the peer may arrive on its barriers
     tc_fence_after();
     if (warp == 0) tmem_dealloc(tmem, kTpCols);
 }
 
-// ------------------------------------------------------------- the packing
+// ------------------------------------------------------ scales and packing
+// ------------------------------------------------------------------- host
+// Power-of-two scale of every block G_j (kz, line) for the FP16 products:
+// its largest |re| or |im| scaled into [2^13, 2^14).
+__global__ void __launch_bounds__(256) gscale_kernel(const float2 *Gt, int n, int ldg, float *gscale) {
+    __shared__ float wmax[8];
+    const float2 *g = Gt + (long)blockIdx.x * n * ldg;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float mx = 0.f;
+    for (int m = warp; m < n; m += 8)
+        for (int i = lane; i < n; i += 32) {
+            const float2 v = g[(long)m * ldg + i];
+            mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)));
+        }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+    if (lane == 0) wmax[warp] = mx;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) mx = fmaxf(mx, wmax[w]);
+        gscale[blockIdx.x] = pow2_scale_13(mx);
+    }
+}
+
+int launch_gscale(const void *Gt, int n, int ny, int nz, int ldg, float *gscale, cudaStream_t s) {
+    gscale_kernel<<<dim3((unsigned)(ny * nz)), 256, 0, s>>>((const float2 *)Gt, n, ldg, gscale);
+    return cudaGetLastError() == cudaSuccess ? HELM3D_OK : HELM3D_ERR_CUDA;
+}
+
 // One CTA per block (kz, j): 16-byte units (row i, chunk c, K core kc) =
 // complex m = 16 c + 4 kc + [0, 4) of row i, as (re, im) FP16 pairs of the
 // hi parts and of the lo parts of s_j G[i][m] (s_j = gscale).  Consecutive
@@ -482,7 +553,7 @@ int launch_gpack(const void *Gt, int n, int ny, int nz, int ldg, const float *gs
 // The launch shape of a batch: RR right-hand sides (8 or 16), MB row blocks,
 // ring depth and shared memory; false when it does not fit.
 struct TpShape {
-    int RR, MB, npad, cpl, nstage;
+    int RR, MB, OCC, npad, cpl, nstage;
     uint32_t tile_bytes;
     size_t smem;
 };
@@ -499,18 +570,20 @@ static bool tp_shape(const SweepArgs &sa, TpShape &sh) {
     const size_t NR = 2 * (size_t)sh.RR, Kp = 2 * (size_t)sh.npad;
     const size_t bbytes = 2 * NR * Kp * 2;   // B hi and lo, FP16
     const size_t vbytes = sizeof(float2) * (size_t)sh.RR * (sh.npad + 2) + sizeof(float) * 4 * sh.RR;
-    const size_t fixed = bbytes + vbytes + sizeof(uint64_t) * (2 + kTpMmaWarps) + 16;
+    const size_t fixed = bbytes + vbytes + sizeof(uint64_t) * (4 + kTpMmaWarps) + 16;
     // a row block read through the last stage's lo tile runs past the ring
     // by (128 MB - n8) rows: that much must be allocated after it
     const size_t tail = std::max(fixed, (size_t)(128 * sh.MB - n8) * kTpRowBytes);
     const size_t optin = device_info().smem_optin;
     const size_t per_stage = stage + 2 * sizeof(uint64_t);
-    if (tail + 2 * per_stage > optin) return false;
-    int nst = (int)((optin - tail) / per_stage);
-    const int ring_cap = (int)(((size_t)sa.ring_kb * 1024) / stage);
-    if (nst > ring_cap) nst = ring_cap;
-    if (nst > 8) nst = 8;
-    if (nst < 2) return false;
+    // two CTAs per SM (one row block): half an SM's shared memory less the
+    // 1 KB the system keeps per CTA, at least 3 stages
+    const size_t half_sm = (optin - 1024) / 2;
+    sh.OCC = sa.tc_occ == 2 && sh.MB == 1 && tail + 3 * per_stage <= half_sm ? 2 : 1;
+    const size_t avail = sh.OCC == 2 ? half_sm : optin;
+    if (tail + 2 * per_stage > avail) return false;
+    int nst = (int)((avail - tail) / per_stage);
+    if (nst > sa.tc_stages) nst = sa.tc_stages;
     sh.nstage = nst;
     sh.smem = (size_t)nst * stage + tail + 2 * sizeof(uint64_t) * nst;
     return true;
@@ -521,7 +594,7 @@ bool sweep_tcp_supported(const SweepArgs &sa) {
     return tp_shape(sa, sh);
 }
 
-template <int RR, int MB, bool ADJ> static int sweep_tcp_impl(const SweepArgs &sa, const TpShape &sh, cudaStream_t st) {
+template <int RR, int MB, bool ADJ, int OCC> static int sweep_tcp_impl(const SweepArgs &sa, const TpShape &sh, cudaStream_t st) {
     SweepTpK k;
     k.n = sa.n;
     k.ny = sa.ny;
@@ -538,15 +611,16 @@ template <int RR, int MB, bool ADJ> static int sweep_tcp_impl(const SweepArgs &s
     k.dxy = (const float2 *)sa.dxy;
     k.status = sa.status;
     k.kzslot = sa.kzslot;
-    auto kern = sweep_tcp_kernel<RR, MB, ADJ>;
-    if (!smem_limit_max(kern, sh.smem)) return HELM3D_ERR_CUDA;
-    kern<<<dim3((unsigned)sa.nz), kTpThreads, sh.smem, st>>>(k);
-    return cudaGetLastError() == cudaSuccess ? HELM3D_OK : HELM3D_ERR_CUDA;
+    return launch_pairs(sweep_tcp_kernel<RR, MB, ADJ, OCC>, sa.nz, kTpThreads, sh.smem, k, st);
+}
+
+template <int RR, bool ADJ> static int sweep_tcp_rr(const SweepArgs &sa, const TpShape &sh, cudaStream_t s) {
+    if (sh.MB == 2) return sweep_tcp_impl<RR, 2, ADJ, 1>(sa, sh, s);
+    return sh.OCC == 2 ? sweep_tcp_impl<RR, 1, ADJ, 2>(sa, sh, s) : sweep_tcp_impl<RR, 1, ADJ, 1>(sa, sh, s);
 }
 
 template <bool ADJ> static int sweep_tcp_adj(const SweepArgs &sa, const TpShape &sh, cudaStream_t s) {
-    if (sh.MB == 2) return sh.RR == 8 ? sweep_tcp_impl<8, 2, ADJ>(sa, sh, s) : sweep_tcp_impl<16, 2, ADJ>(sa, sh, s);
-    return sh.RR == 8 ? sweep_tcp_impl<8, 1, ADJ>(sa, sh, s) : sweep_tcp_impl<16, 1, ADJ>(sa, sh, s);
+    return sh.RR == 8 ? sweep_tcp_rr<8, ADJ>(sa, sh, s) : sweep_tcp_rr<16, ADJ>(sa, sh, s);
 }
 
 int launch_sweep_tcp(const SweepArgs &sa, cudaStream_t s) {
