@@ -193,25 +193,14 @@ int launch_stencil(const StencilArgs &a, bool adjoint, cudaStream_t s);
 // dimension ldv) per right-hand side r, with real scales vs (basis vector i
 // of r is vs[r][i] V_r[i]).
 struct Reduce {
-    double2 *partials;        // [rmax][nblocks][cap] scratch
+    double2 *partials;        // of right-hand side r at r * stride
+    long stride;
+    int *tickets;             // [rmax + 1], zero between launches (krylov.cu last_to_finish)
     int nblocks;
-    int cap;
+    int cap;                  // sums per right-hand side at most
     int rmax;
     int update = 0;           // DCGS2 update pass variant (0: loads one by one, 1: 8 basis loads batched)
 };
-// out[r][i] = <vs_r[i] V_r[i], w_r>   (i < nv); with wnorm also out[r][nv].x = ||w_r||^2
-// (pred: when given and *pred == 0 on the device, the kernels do nothing)
-int launch_dots(const VecBatch &V, long ldv, const ScaleBatch &vs, int nv, const VecBatch &w, long N, int R,
-                const Reduce &red, double2 *out, long sOut, cudaStream_t s, bool wnorm = false,
-                const int *pred = nullptr);
-// w_r -= sum_i coef[r][i] vs_r[i] V_r[i]; post 1: out[r].x = ||w_r||^2
-int launch_update(const VecBatch &V, long ldv, const ScaleBatch &vs, int nv, const double2 *coef, long sCoef,
-                  const VecBatch &w, long N, int R, int post, const Reduce &red, double2 *out, long sOut,
-                  cudaStream_t s, const int *pred = nullptr);
-// x_r += sum_i y[r][i] zs_r[i] Z_r[i]  (i < min(nzv, *nzv_dev) when nzv_dev is given)
-int launch_combine(const VecBatch &Z, long ldz, const ScaleBatch &zs, int nzv, const double2 *y, long sY,
-                   const VecBatch &x, long N, int R, cudaStream_t s, const int *nzv_dev = nullptr);
-
 // ------------------------------------------- device-side Arnoldi bookkeeping
 // Per right-hand side p of a lockstep batch of B (the host FGMRES state, on
 // the device so that a whole restart cycle runs without the host):
@@ -231,36 +220,46 @@ struct ArnState {
     double *vs;        // basis scales [B][M2]
 };
 constexpr int kArnFlags = 8;
-// flags[0] = any unfrozen p with ||w||^2 after the first pass < 1/2 of before
-int launch_reorth_check(const ArnState &a, int j, cudaStream_t s);
-// column j of H (h1 + h2 when flags[0]), rotations, g, est, frozen, k, it,
-// vs[j + 1]; sets `next` (if has_next) to "some p is still unfrozen"
-int launch_givens(const ArnState &a, int j, bool has_next, cudaGraphConditionalHandle next, cudaStream_t s);
+// out[r][i] = <vs_r[i] V_r[i], w_r>   (i < nv); with wnorm also out[r][nv].x = ||w_r||^2
+// (pred: when given and *pred == 0 on the device, the pass does nothing)
+int launch_dots(const VecBatch &V, long ldv, const ScaleBatch &vs, int nv, const VecBatch &w, long N, int R,
+                const Reduce &red, double2 *out, long sOut, cudaStream_t s, bool wnorm = false,
+                const int *pred = nullptr);
+// w_r -= sum_i coef[r][i] vs_r[i] V_r[i]; post 1: out[r].x = ||w_r||^2.  With
+// arn the end of classical Gram-Schmidt's step j too: after the first pass
+// (no pred) flags[0] = any unfrozen r with ||w||^2 < 1/2 of before, after the
+// second (taken when *pred) column j of H (h1 + h2 when flags[0]), rotations,
+// g, est, frozen, k, it, vs[j + 1], and `next` (if has_next) set to "some r is
+// still unfrozen".
+int launch_update(const VecBatch &V, long ldv, const ScaleBatch &vs, int nv, const double2 *coef, long sCoef,
+                  const VecBatch &w, long N, int R, int post, const Reduce &red, double2 *out, long sOut,
+                  cudaStream_t s, const int *pred = nullptr, const ArnState *arn = nullptr, int j = 0,
+                  bool has_next = false, cudaGraphConditionalHandle next = 0);
+// x_r += sum_i y[r][i] zs_r[i] Z_r[i]  (i < min(nzv, *nzv_dev) when nzv_dev is given)
+int launch_combine(const VecBatch &Z, long ldz, const ScaleBatch &zs, int nzv, const double2 *y, long sY,
+                   const VecBatch &x, long N, int R, cudaStream_t s, const int *nzv_dev = nullptr);
 // DCGS2 (low-synchronization Gram-Schmidt with delayed reorthogonalization,
 // flexible FGMRES): per step j one reduction (dots2) and one update pass
 // (update2) over the basis.  Krylov scalars per right-hand side: dots at h
 // (2 j + 2 slots), ||w'||^2 at 2 M2, update coefficients alpha at 4 M2 and
-// delta at 5 M2.
+// delta at 5 M2.  With arn: frozen right-hand sides are left out, dots2 ends
+// by finalizing column j - 1 and writing column j and the update coefficients,
+// update2 by beta, vs[j + 1], flags[4..5] and the condition of step j + 1.
 int launch_dots2(const VecBatch &V, long ldv, const ScaleBatch &vs, int j, const VecBatch &w, long N, int R,
-                 const Reduce &red, double2 *out, long sOut, cudaStream_t s, const int *pred, const int *skip);
+                 const Reduce &red, double2 *out, long sOut, cudaStream_t s, const ArnState *arn);
 int launch_update2(const VecBatch &V, long ldv, int j, const double2 *coef, long sCoef, int M2, const VecBatch &w,
-                   long N, int R, const Reduce &red, double2 *out, long sOut, cudaStream_t s, const int *pred,
-                   const int *skip);
-// reorthogonalization dots of the cycle's last tentative vector V_{jl+1},
-// jl = *jl on the device (tmax: the largest jl + 1)
-int launch_dots_tail(const VecBatch &V, long ldv, const ScaleBatch &vs, int tmax, const int *jl, long N, int R,
-                     const Reduce &red, double2 *out, long sOut, cudaStream_t s, const int *pred, const int *skip);
-// finalize column j - 1, write column j and the update coefficients
-int launch_lagged(const ArnState &a, int j, cudaStream_t s);
-// beta, vs[j + 1], flags[4..5] and the condition of step j + 1
-int launch_post(const ArnState &a, int j, bool has_next, cudaGraphConditionalHandle next, cudaStream_t s);
-// finalize the open column of the cycle's last step
-int launch_lagged_final(const ArnState &a, cudaStream_t s);
-// y = R^{-1} g (k x k per p, zero padded to m) into h at 3 M2; flags[2] = max k
-int launch_backsub(const ArnState &a, cudaStream_t s);
-// out[r].x = ||x_r||^2 over the box [x0,x1) x [y0,y1) x [z0,z1)
-int launch_norm2_box(const VecBatch &x, int R, int nx, int ny, int nz, const int box[6], const Reduce &red,
-                     double2 *out, long sOut, cudaStream_t s);
+                   long N, int R, const Reduce &red, double2 *out, long sOut, cudaStream_t s, const ArnState *arn,
+                   bool has_next = false, cudaGraphConditionalHandle next = 0);
+// End of a cycle: with tail (DCGS2) the reorthogonalization dots of the last
+// tentative vector V_{jl+1}, jl = flags[4], and the open column they close;
+// then y = R^{-1} g (k x k per p, zero padded to m) into h at 3 M2 and
+// flags[2] = max k.
+int launch_cycle_end(const VecBatch &V, long ldv, const ArnState &arn, bool tail, long N, int R, const Reduce &red,
+                     cudaStream_t s);
+// out[r * sOut].x = ||x_r||^2 and, with box, out[r * sOut + 1].x over the box
+// [x0,x1) x [y0,y1) x [z0,z1)
+int launch_norm2(const VecBatch &x, int R, int nx, int ny, int nz, const int *box, const Reduce &red, double2 *out,
+                 long sOut, cudaStream_t s);
 // y_r = a x_r + b y_r
 int launch_axpby(double2 a, const VecBatch &x, double2 b, const VecBatch &y, long N, int R, cudaStream_t s);
 // y = x - dl * t  (mode R's K x from t = L0^{-1} x)
@@ -440,7 +439,9 @@ struct helm3d_ctx {
     double *d_vs = nullptr;
     double2 *d_h = nullptr;        // small device scalars
     double2 *d_partials = nullptr;
+    int *d_tickets = nullptr;      // zero between launches (krylov.cu last_to_finish)
     int red_blocks = 0, red_cap = 0;
+    long red_stride = 0;           // partials of one right-hand side
     double2 *d_f = nullptr, *d_u = nullptr, *d_r = nullptr, *d_t = nullptr, *d_t2 = nullptr;
     double2 *d_bic = nullptr;      // BiCGStab vectors
     size_t bytes = 0;

@@ -46,6 +46,8 @@ static VecBatch one(const double2 *p) { return VecBatch{const_cast<double2 *>(p)
 static Reduce reducer(helm3d_ctx *c) {
     Reduce r;
     r.partials = c->d_partials;
+    r.stride = c->red_stride;
+    r.tickets = c->d_tickets;
     r.nblocks = c->red_blocks;
     r.cap = c->red_cap;
     r.rmax = c->r_alloc;
@@ -104,9 +106,10 @@ static void drop_graphs(helm3d_ctx *c) {
 
 static void free_krylov(helm3d_ctx *c) {
     drop_graphs(c);
-    void *bufs[] = {c->d_V, c->d_Z, c->d_vs, c->d_h, c->d_partials, c->d_Fw, c->d_Uw, c->d_arn};
+    void *bufs[] = {c->d_V, c->d_Z, c->d_vs, c->d_h, c->d_partials, c->d_tickets, c->d_Fw, c->d_Uw, c->d_arn};
     for (void *p : bufs)
         if (p) cudaFree(p);
+    c->d_tickets = nullptr;
     c->d_V = c->d_Z = c->d_h = c->d_partials = c->d_Fw = c->d_Uw = nullptr;
     c->d_arn = nullptr;
     c->d_vs = nullptr;
@@ -139,6 +142,8 @@ int ensure_krylov(helm3d_ctx *c, int m, int R) {
         (rc = get((void **)&c->d_vs, sizeof(double) * (m + 2) * R, "basis scales")) ||
         (rc = get((void **)&c->d_h, sizeof(double2) * scalars_per_rhs(m) * R, "Krylov scalars")) ||
         (rc = get((void **)&c->d_partials, sizeof(double2) * c->red_cap * red_max * R, "partials")) ||
+        (rc = get((void **)&c->d_tickets, sizeof(int) * (R + 1), "tickets")) ||
+        (rc = cuda_check(c, cudaMemsetAsync(c->d_tickets, 0, sizeof(int) * (R + 1), c->stream), "tickets")) ||
         (rc = get((void **)&c->d_Fw, vb * R, "packed right-hand sides")) ||
         (rc = get((void **)&c->d_Uw, vb * R, "packed iterates")) ||
         (rc = get(&c->d_arn, arn_bytes(m, R), "Arnoldi state"))) {
@@ -148,6 +153,7 @@ int ensure_krylov(helm3d_ctx *c, int m, int R) {
     }
     c->m_alloc = m;
     c->r_alloc = R;
+    c->red_stride = (long)c->red_cap * red_max;
     c->kry_bytes = total;
     c->bytes += total;
     return HELM3D_OK;
@@ -333,15 +339,6 @@ static int fetch(helm3d_ctx *c, const double2 *d, size_t n, double2 *h, const ch
     return cuda_check(c, cudaStreamSynchronize(c->stream), what);
 }
 
-static void full_box(helm3d_ctx *c, int box[6]) {
-    box[0] = 0;
-    box[1] = c->grid.nx;
-    box[2] = 0;
-    box[3] = c->grid.ny;
-    box[4] = 0;
-    box[5] = c->grid.nz;
-}
-
 // the physical domain: the grid without its PML (and mode R's sponge) layers
 static void phys_box(helm3d_ctx *c, int box[6]) {
     const helm3d_grid &g = c->grid;
@@ -357,16 +354,11 @@ static void phys_box(helm3d_ctx *c, int box[6]) {
 // ||x_r||^2 into out[r * sOut].x (full grid) and, with phys, out[r * sOut + 1].x
 // (physical domain); no host synchronization
 static int norms(helm3d_ctx *c, const VecBatch &x, int R, bool phys, double2 *out, long sOut) {
-    const Reduce red = reducer(c);
     int box[6];
-    full_box(c, box);
-    RC(timed(c, HELM3D_K_KRYLOV, 2, [&] {
-        return launch_norm2_box(x, R, c->grid.nx, c->grid.ny, c->grid.nz, box, red, out, sOut, c->stream);
-    }));
-    if (!phys) return HELM3D_OK;
     phys_box(c, box);
-    return timed(c, HELM3D_K_KRYLOV, 2, [&] {
-        return launch_norm2_box(x, R, c->grid.nx, c->grid.ny, c->grid.nz, box, red, out + 1, sOut, c->stream);
+    return timed(c, HELM3D_K_KRYLOV, 1, [&] {
+        return launch_norm2(x, R, c->grid.nx, c->grid.ny, c->grid.nz, phys ? box : nullptr, reducer(c), out, sOut,
+                            c->stream);
     });
 }
 
@@ -435,29 +427,27 @@ static int arnoldi_step(helm3d_ctx *c, int m, int B, int j, bool adjoint, const 
     }
     if (lowsync(c)) {
         // DCGS2: one reduction (w against V_0..V_j, the lagged second
-        // projection of V_j), the bookkeeping, one update pass
-        RC(timed(c, HELM3D_K_KRYLOV, 2, [&] {
-            return launch_dots2(Vall, N, vsb, j, w, N, B, red, d_h1, SH, c->stream, nullptr, a.frozen);
-        }));
-        RC(timed(c, HELM3D_K_KRYLOV, 1, [&] { return launch_lagged(a, j, c->stream); }));
-        RC(timed(c, HELM3D_K_KRYLOV, 2, [&] {
-            return launch_update2(Vall, N, j, Hd + 4 * M2, SH, M2, w, N, B, red, d_nrm, SH, c->stream, nullptr,
-                                  a.frozen);
-        }));
-        return timed(c, HELM3D_K_KRYLOV, 1, [&] { return launch_post(a, j, has_next, next, c->stream); });
+        // projection of V_j) ending with the bookkeeping, one update pass
+        // ending with the next step's condition
+        RC(timed(c, HELM3D_K_KRYLOV, 1,
+                 [&] { return launch_dots2(Vall, N, vsb, j, w, N, B, red, d_h1, SH, c->stream, &a); }));
+        return timed(c, HELM3D_K_KRYLOV, 1, [&] {
+            return launch_update2(Vall, N, j, Hd + 4 * M2, SH, M2, w, N, B, red, d_nrm, SH, c->stream, &a, has_next,
+                                  next);
+        });
     }
-    RC(timed(c, HELM3D_K_KRYLOV, 2,
+    RC(timed(c, HELM3D_K_KRYLOV, 1,
              [&] { return launch_dots(Vall, N, vsb, j + 1, w, N, B, red, d_h1, SH, c->stream, true); }));
-    RC(timed(c, HELM3D_K_KRYLOV, 2,
-             [&] { return launch_update(Vall, N, vsb, j + 1, d_h1, SH, w, N, B, 1, red, d_nrm, SH, c->stream); }));
-    RC(timed(c, HELM3D_K_KRYLOV, 1, [&] { return launch_reorth_check(a, j, c->stream); }));
-    RC(timed(c, HELM3D_K_KRYLOV, 2, [&] {
+    RC(timed(c, HELM3D_K_KRYLOV, 1, [&] {
+        return launch_update(Vall, N, vsb, j + 1, d_h1, SH, w, N, B, 1, red, d_nrm, SH, c->stream, nullptr, &a, j);
+    }));
+    RC(timed(c, HELM3D_K_KRYLOV, 1, [&] {
         return launch_dots(Vall, N, vsb, j + 1, w, N, B, red, d_h2, SH, c->stream, false, a.flags);
     }));
-    RC(timed(c, HELM3D_K_KRYLOV, 2, [&] {
-        return launch_update(Vall, N, vsb, j + 1, d_h2, SH, w, N, B, 1, red, d_nrm, SH, c->stream, a.flags);
-    }));
-    return timed(c, HELM3D_K_KRYLOV, 1, [&] { return launch_givens(a, j, has_next, next, c->stream); });
+    return timed(c, HELM3D_K_KRYLOV, 1, [&] {
+        return launch_update(Vall, N, vsb, j + 1, d_h2, SH, w, N, B, 1, red, d_nrm, SH, c->stream, a.flags, &a, j,
+                             has_next, next);
+    });
 }
 
 // end of a cycle: y = R^{-1} g on the device, x += Z y (mode R: V y)
@@ -466,16 +456,11 @@ static int cycle_tail(helm3d_ctx *c, int m, int B, const ArnState &a) {
     const long ldV = (long)(m + 1) * N, ldZ = (long)m * N;
     const int M2 = m + 2, SH = scalars_per_rhs(m);
     double2 *d_y = c->d_h + 3 * M2;
-    if (lowsync(c)) {
-        // the open column of the last step (skipped when every right-hand
-        // side stopped inside the cycle)
-        RC(timed(c, HELM3D_K_KRYLOV, 2, [&] {
-            return launch_dots_tail(VecBatch{c->d_V, ldV}, N, ScaleBatch{c->d_vs, M2}, m, a.flags + 4, N, B,
-                                    reducer(c), c->d_h, SH, c->stream, a.flags + 5, a.frozen);
-        }));
-        RC(timed(c, HELM3D_K_KRYLOV, 1, [&] { return launch_lagged_final(a, c->stream); }));
-    }
-    RC(timed(c, HELM3D_K_KRYLOV, 1, [&] { return launch_backsub(a, c->stream); }));
+    // the open column of the last step (DCGS2; skipped when every right-hand
+    // side stopped inside the cycle) and y
+    RC(timed(c, HELM3D_K_KRYLOV, 1, [&] {
+        return launch_cycle_end(VecBatch{c->d_V, ldV}, N, a, lowsync(c), N, B, reducer(c), c->stream);
+    }));
     return timed(c, HELM3D_K_KRYLOV, 1, [&] {
         return c->opts.mode == HELM3D_MODE_N
                    ? launch_combine(zbasis(c, 0, ldZ), N, kNoScale, m, d_y, SH, VecBatch{c->d_Uw, N}, N, B,
@@ -620,7 +605,7 @@ int tune_solve(helm3d_ctx *c, int R, bool adjoint) {
         red.nblocks = reduce_blocks(v);
         return launch_dots2(VecBatch{c->d_V, ldV}, N, ScaleBatch{c->d_vs, m + 2}, j,
                             VecBatch{c->d_V + (size_t)(j + 1) * N, ldV}, N, R, red, c->d_h, scalars_per_rhs(m),
-                            c->stream, nullptr, nullptr);
+                            c->stream, nullptr);
     });
     c->red_blocks = reduce_blocks(rv);
     // the DCGS2 update pass at the same depth, in place on V_j and V_{j+1}
@@ -633,7 +618,7 @@ int tune_solve(helm3d_ctx *c, int R, bool adjoint) {
             red.update = v;
             return launch_update2(VecBatch{c->d_V, ldV}, N, j, c->d_h + 4 * M2, scalars_per_rhs(m), M2,
                                   VecBatch{c->d_V + (size_t)(j + 1) * N, ldV}, N, R, red, c->d_h + 2 * M2,
-                                  scalars_per_rhs(m), c->stream, nullptr, nullptr);
+                                  scalars_per_rhs(m), c->stream, nullptr);
         });
     }
     return HELM3D_OK;
@@ -973,9 +958,9 @@ int FgmresRun::run_host_cycle() {
         // enough"): h1 = V^H w with ||w||^2 from the same pass, w -= V h1
         // with ||w||^2 after; a second pass runs when the norm of some
         // right-hand side dropped below 1/sqrt(2) of its value.
-        RC(timed(c, HELM3D_K_KRYLOV, 2,
+        RC(timed(c, HELM3D_K_KRYLOV, 1,
                  [&] { return launch_dots(Vall, N, vsb, j + 1, w, N, B, red, d_h1, SH, c->stream, true); }));
-        RC(timed(c, HELM3D_K_KRYLOV, 2, [&] {
+        RC(timed(c, HELM3D_K_KRYLOV, 1, [&] {
             return launch_update(Vall, N, vsb, j + 1, d_h1, SH, w, N, B, 1, red, d_nrm, SH, c->stream);
         }));
         RC(fetch_scalars(B, "Arnoldi coefficients"));
@@ -991,9 +976,9 @@ int FgmresRun::run_host_cycle() {
             for (int i = 0; i <= j; i++) r.H[(size_t)i * m + j] = zc(h[i].x, h[i].y);
         }
         if (again) {
-            RC(timed(c, HELM3D_K_KRYLOV, 2,
+            RC(timed(c, HELM3D_K_KRYLOV, 1,
                      [&] { return launch_dots(Vall, N, vsb, j + 1, w, N, B, red, d_h2, SH, c->stream); }));
-            RC(timed(c, HELM3D_K_KRYLOV, 2, [&] {
+            RC(timed(c, HELM3D_K_KRYLOV, 1, [&] {
                 return launch_update(Vall, N, vsb, j + 1, d_h2, SH, w, N, B, 1, red, d_nrm, SH, c->stream);
             }));
             RC(fetch_scalars(B, "Arnoldi second pass"));
@@ -1204,7 +1189,7 @@ int fgmres_group(helm3d_ctx *const *cs, int n, const double2 *const *f, double2 
 // dot <a, b> = sum conj(a) b on the device, returned to the host
 static int zdot(helm3d_ctx *c, const double2 *a, const double2 *b, zc *out) {
     const Reduce red = reducer(c);
-    RC(timed(c, HELM3D_K_KRYLOV, 2, [&] {
+    RC(timed(c, HELM3D_K_KRYLOV, 1, [&] {
         return launch_dots(one(a), c->N, kNoScale, 1, one(b), c->N, 1, red, c->d_h, 0, c->stream);
     }));
     double2 v;
