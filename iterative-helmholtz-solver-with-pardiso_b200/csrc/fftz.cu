@@ -9,7 +9,9 @@
 // with radix r and span p maps task i (k = i mod p) to
 //     u_q = x[i + q*(n/r)] * w_{p r}^{q k},   U = DFT_r(u),
 //     y[(i - k) r + k + q p] = U_q.
-// Radices 2..8 are unrolled; any other prime factor uses a generic loop.
+// Radices 2..8 are unrolled; any other prime factor uses a generic pass, and
+// comes first, where no twiddles are needed (58 = 29 x 2, complex128: 49 us with
+// one thread per butterfly).
 #include <cuda_runtime.h>
 
 #include "cplx.cuh"
@@ -71,21 +73,48 @@ __device__ __forceinline__ void radix_task(const cplx<R> *__restrict__ src, cplx
     for (int q = 0; q < RR; q++) dst[(j + q * p) * TW + col] = U[q];
 }
 
+// A pass of any prime radix r: kGenQ outputs of one butterfly at a time per
+// thread (the m butterflies of such a pass are too few to occupy the block one
+// thread each), every input read once for them.
+constexpr int kGenQ = 4;
 template <typename R, bool INV, int TW>
-__device__ void radix_task_generic(const cplx<R> *__restrict__ src, cplx<R> *__restrict__ dst,
-                                   const cplx<R> *__restrict__ tw, int twoff, int dftoff, int r, int i, int m,
-                                   int p, int col) {
-    const int k = i % p;
-    const int j = (i - k) * r + k;
-    for (int q = 0; q < r; q++) {
-        cplx<R> acc = mkc<R>(0, 0);
+__device__ void radix_pass_generic(const cplx<R> *__restrict__ src, cplx<R> *__restrict__ dst,
+                                   const cplx<R> *__restrict__ tw, int twoff, int dftoff, int r, int m, int p,
+                                   int col, int grp, int ngrp) {
+    const int nq = (r + kGenQ - 1) / kGenQ;
+    for (int e = grp; e < m * nq; e += ngrp) {
+        const int i = e / nq, q0 = (e - i * nq) * kGenQ;
+        const int k = i % p;
+        const int j = (i - k) * r + k;
+        cplx<R> acc[kGenQ];
+        int idx[kGenQ], qs[kGenQ];   // (q t) mod r; past the last output: any q, not stored
+#pragma unroll
+        for (int u = 0; u < kGenQ; u++) {
+            acc[u] = mkc<R>(0, 0);
+            idx[u] = 0;
+            qs[u] = q0 + u < r ? q0 + u : 0;
+        }
         for (int t = 0; t < r; t++) {
             cplx<R> ut = src[(i + t * m) * TW + col];
             if (p > 1 && t > 0) ut = cmul(ut, tw_load<R, INV>(tw, twoff + k * r + t));
-            acc = cfma(ut, tw_load<R, INV>(tw, dftoff + (q * t) % r), acc);
+#pragma unroll
+            for (int u = 0; u < kGenQ; u++) {
+                acc[u] = cfma(ut, tw_load<R, INV>(tw, dftoff + idx[u]), acc[u]);
+                idx[u] += qs[u];
+                if (idx[u] >= r) idx[u] -= r;
+            }
         }
-        dst[(j + q * p) * TW + col] = acc;
+#pragma unroll
+        for (int u = 0; u < kGenQ; u++)
+            if (q0 + u < r) dst[(j + (q0 + u) * p) * TW + col] = acc[u];
     }
+}
+
+template <typename R, int RR, bool INV, int TW>
+__device__ __forceinline__ void radix_pass(const cplx<R> *__restrict__ src, cplx<R> *__restrict__ dst,
+                                           const cplx<R> *__restrict__ tw, int to, int dof, int m, int p, int col,
+                                           int grp, int ngrp) {
+    for (int i = grp; i < m; i += ngrp) radix_task<R, RR, INV, TW>(src, dst, tw, to, dof, i, m, p, col);
 }
 
 template <typename R, bool INV, int TW>
@@ -95,16 +124,14 @@ __device__ cplx<R> *fft_passes(cplx<R> *A, cplx<R> *B, const FftK &fp, const cpl
     for (int s = 0; s < fp.npass; s++) {
         const int r = fp.radix[s], p = fp.span[s], m = fp.n / r;
         const int to = fp.twoff[s], dof = fp.dftoff[s];
-        for (int i = grp; i < m; i += ngrp) {
-            switch (r) {
-                case 2: radix_task<R, 2, INV, TW>(src, dst, tw, to, dof, i, m, p, col); break;
-                case 3: radix_task<R, 3, INV, TW>(src, dst, tw, to, dof, i, m, p, col); break;
-                case 4: radix_task<R, 4, INV, TW>(src, dst, tw, to, dof, i, m, p, col); break;
-                case 5: radix_task<R, 5, INV, TW>(src, dst, tw, to, dof, i, m, p, col); break;
-                case 7: radix_task<R, 7, INV, TW>(src, dst, tw, to, dof, i, m, p, col); break;
-                case 8: radix_task<R, 8, INV, TW>(src, dst, tw, to, dof, i, m, p, col); break;
-                default: radix_task_generic<R, INV, TW>(src, dst, tw, to, dof, r, i, m, p, col); break;
-            }
+        switch (r) {
+            case 2: radix_pass<R, 2, INV, TW>(src, dst, tw, to, dof, m, p, col, grp, ngrp); break;
+            case 3: radix_pass<R, 3, INV, TW>(src, dst, tw, to, dof, m, p, col, grp, ngrp); break;
+            case 4: radix_pass<R, 4, INV, TW>(src, dst, tw, to, dof, m, p, col, grp, ngrp); break;
+            case 5: radix_pass<R, 5, INV, TW>(src, dst, tw, to, dof, m, p, col, grp, ngrp); break;
+            case 7: radix_pass<R, 7, INV, TW>(src, dst, tw, to, dof, m, p, col, grp, ngrp); break;
+            case 8: radix_pass<R, 8, INV, TW>(src, dst, tw, to, dof, m, p, col, grp, ngrp); break;
+            default: radix_pass_generic<R, INV, TW>(src, dst, tw, to, dof, r, m, p, col, grp, ngrp); break;
         }
         __syncthreads();
         cplx<R> *t = src;
@@ -115,6 +142,7 @@ __device__ cplx<R> *fft_passes(cplx<R> *A, cplx<R> *B, const FftK &fp, const cpl
 }
 
 constexpr int kFftThreads = 256;
+constexpr int kFftRows = 4;   // rows a thread loads at a time
 
 // plane index of (row k, column w = i + nx*j) for right-hand side r
 __device__ __forceinline__ long plane_index(const PlaneLayout &L, int r, int k, long w) {
@@ -136,14 +164,24 @@ __global__ void __launch_bounds__(kFftThreads) fftz_forward_kernel(FftK fp, VecB
     const double s = scale * (sc.p ? sc.p[r * sc.stride] : 1.0);
     const long w = (long)blockIdx.x * TW + col;
     const bool valid = w < plane;
-    for (int row = grp; row < fp.n; row += ngrp) {
-        double2 v = valid ? xr[(long)row * plane + w] : make_double2(0.0, 0.0);
-        A[row * TW + col] = cvt<cplx<R>, double2>(make_double2(v.x * s, v.y * s));
+    for (int row0 = grp; row0 < fp.n; row0 += kFftRows * ngrp) {   // kFftRows loads in flight
+        double2 v[kFftRows];
+#pragma unroll
+        for (int u = 0; u < kFftRows; u++) {
+            const int row = row0 + u * ngrp;
+            v[u] = valid && row < fp.n ? xr[(long)row * plane + w] : make_double2(0.0, 0.0);
+        }
+#pragma unroll
+        for (int u = 0; u < kFftRows; u++) {
+            const int row = row0 + u * ngrp;
+            if (row < fp.n) A[row * TW + col] = cvt<cplx<R>, double2>(make_double2(v[u].x * s, v[u].y * s));
+        }
     }
     __syncthreads();
     cplx<R> *res = fft_passes<R, false, TW>(A, B, fp, tw, col, grp, ngrp);
-    if (valid)
-        for (int row = grp; row < fp.n; row += ngrp) out[plane_index(L, r, row, w)] = res[row * TW + col];
+    if (!valid) return;
+    const long obase = plane_index(L, r, 0, w), ostep = L.plane * L.R;
+    for (int row = grp; row < fp.n; row += ngrp) out[obase + row * ostep] = res[row * TW + col];
 }
 
 template <typename R, int TW>
@@ -160,8 +198,20 @@ __global__ void __launch_bounds__(kFftThreads) fftz_inverse_kernel(FftK fp, cons
     const long plane = L.plane;
     const long w = (long)blockIdx.x * TW + col;
     const bool valid = w < plane;
-    for (int row = grp; row < fp.n; row += ngrp)
-        A[row * TW + col] = valid ? in[plane_index(L, r, row, w)] : mkc<R>(0, 0);
+    const long ibase = valid ? plane_index(L, r, 0, w) : 0, istep = L.plane * L.R;
+    for (int row0 = grp; row0 < fp.n; row0 += kFftRows * ngrp) {
+        cplx<R> v[kFftRows];
+#pragma unroll
+        for (int u = 0; u < kFftRows; u++) {
+            const int row = row0 + u * ngrp;
+            v[u] = valid && row < fp.n ? in[ibase + row * istep] : mkc<R>(0, 0);
+        }
+#pragma unroll
+        for (int u = 0; u < kFftRows; u++) {
+            const int row = row0 + u * ngrp;
+            if (row < fp.n) A[row * TW + col] = v[u];
+        }
+    }
     __syncthreads();
     cplx<R> *res = fft_passes<R, true, TW>(A, B, fp, tw, col, grp, ngrp);
     if (!valid) return;
@@ -196,10 +246,13 @@ static FftK to_k(const FftPlan &p) {
     return k;
 }
 
-template <typename R> static int pick_tw(int n) {
-    // two buffers of n x TW elements must fit the opt-in shared memory
+// Columns per CTA: 32, or 16 (256-byte rows in complex128, still whole
+// sectors) where 32 would leave less than two CTAs per SM or do not fit the
+// shared memory (two buffers of n x TW elements).
+template <typename R> static int pick_tw(int n, const PlaneLayout &L) {
     const size_t cap = device_info().smem_optin;
-    if ((size_t)2 * n * 32 * sizeof(cplx<R>) <= cap) return 32;
+    const bool few = ((L.plane + 31) / 32) * L.R < 2L * device_info().sm_count;
+    if (!few && (size_t)2 * n * 32 * sizeof(cplx<R>) <= cap) return 32;
     if ((size_t)2 * n * 16 * sizeof(cplx<R>) <= cap) return 16;
     return 0;
 }
@@ -233,11 +286,11 @@ static int inv_impl(const void *planes, const PlaneLayout &L, const VecBatch &y,
 int launch_fft_forward(bool c64, const VecBatch &x, double scale, const ScaleBatch &sc, void *planes,
                        const PlaneLayout &L, const FftPlan &plan, const void *tw, cudaStream_t s) {
     if (c64) {
-        int tw_ = pick_tw<float>(plan.n);
+        int tw_ = pick_tw<float>(plan.n, L);
         if (tw_ == 32) return fwd_impl<float, 32>(x, scale, sc, planes, L, plan, tw, s);
         if (tw_ == 16) return fwd_impl<float, 16>(x, scale, sc, planes, L, plan, tw, s);
     } else {
-        int tw_ = pick_tw<double>(plan.n);
+        int tw_ = pick_tw<double>(plan.n, L);
         if (tw_ == 32) return fwd_impl<double, 32>(x, scale, sc, planes, L, plan, tw, s);
         if (tw_ == 16) return fwd_impl<double, 16>(x, scale, sc, planes, L, plan, tw, s);
     }
@@ -248,11 +301,11 @@ int launch_fft_inverse(bool c64, const void *planes, const PlaneLayout &L, const
                        const void *tw, int mode, const VecBatch &w, double scale, const ScaleBatch &sc,
                        const double2 *dl, cudaStream_t s) {
     if (c64) {
-        int tw_ = pick_tw<float>(plan.n);
+        int tw_ = pick_tw<float>(plan.n, L);
         if (tw_ == 32) return inv_impl<float, 32>(planes, L, y, plan, tw, mode, w, scale, sc, dl, s);
         if (tw_ == 16) return inv_impl<float, 16>(planes, L, y, plan, tw, mode, w, scale, sc, dl, s);
     } else {
-        int tw_ = pick_tw<double>(plan.n);
+        int tw_ = pick_tw<double>(plan.n, L);
         if (tw_ == 32) return inv_impl<double, 32>(planes, L, y, plan, tw, mode, w, scale, sc, dl, s);
         if (tw_ == 16) return inv_impl<double, 16>(planes, L, y, plan, tw, mode, w, scale, sc, dl, s);
     }

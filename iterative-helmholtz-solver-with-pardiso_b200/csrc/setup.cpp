@@ -215,13 +215,14 @@ void build_fft_plan(int n, FftPlan &plan, std::vector<zc> &tables) {
     plan = FftPlan();
     plan.n = n;
     int rem = n;
-    std::vector<int> rad;
+    std::vector<int> rad, gen;   // unrolled radices, other primes (first: their pass then has no twiddles)
     while (rem % 8 == 0) { rad.push_back(8); rem /= 8; }
     while (rem % 4 == 0) { rad.push_back(4); rem /= 4; }
     while (rem % 2 == 0) { rad.push_back(2); rem /= 2; }
     for (int p : {3, 5, 7}) while (rem % p == 0) { rad.push_back(p); rem /= p; }
     for (int p = 11; rem > 1; p += 2)
-        while (rem % p == 0) { rad.push_back(p); rem /= p; }
+        while (rem % p == 0) { gen.push_back(p); rem /= p; }
+    rad.insert(rad.begin(), gen.rbegin(), gen.rend());
     if (rad.empty()) rad.push_back(1);
     plan.npass = (int)rad.size();
     tables.clear();
