@@ -58,24 +58,42 @@ struct VecArg {
     }
 };
 
+// the misfit gradient's wavefields given back (synchronizes the stream)
+void release_grad(helm3d_ctx *c) {
+    if (!c->d_grad) return;
+    cudaStreamSynchronize(c->stream);
+    cudaFree(c->d_grad);
+    c->bytes -= c->grad_bytes;
+    c->d_grad = nullptr;
+    c->grad_bytes = 0;
+}
+
 // Right-hand sides per lockstep batch: at most kMaxBatch, and as many as the
 // Krylov bases (V, Z), packed iterates, planes, staging and `extra` further
 // vectors of each fit in 85% of the free device memory (plus what the
-// context's Krylov workspace already holds).
+// context's Krylov workspace and, for the gradient's extra vectors, its
+// wavefields already hold).  A kept wavefield buffer that would make a solve's
+// batch smaller is given back.
 int batch_size(helm3d_ctx *c, int nrhs, bool staged, int extra = 0) {
     const int m = std::max(1, c->opts.restart);
     const size_t vb = sizeof(double2) * (size_t)c->N;
     const size_t per =
         vb * ((size_t)(m + 1) + (c->opts.mode == HELM3D_MODE_N ? m : 0) + 2 + (staged ? 2 : 0) + extra) +
         (c->c64 ? 8 : 16) * (size_t)c->N;
-    size_t fr = 0, tot = 0;
-    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
-        cudaGetLastError();
-        return 1;
+    for (;;) {
+        size_t fr = 0, tot = 0;
+        if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
+            cudaGetLastError();
+            return 1;
+        }
+        const size_t avail = (size_t)(0.85 * (double)(fr + c->kry_bytes + (extra ? c->grad_bytes : 0)));
+        const int R = (int)std::min<size_t>(avail / std::max<size_t>(per, 1), (size_t)kMaxBatch);
+        if (R < std::min(nrhs, kMaxBatch) && !extra && c->d_grad) {
+            release_grad(c);
+            continue;
+        }
+        return std::max(1, std::min(R, nrhs));
     }
-    const size_t avail = (size_t)(0.85 * (double)(fr + c->kry_bytes));
-    int R = (int)std::min<size_t>(avail / std::max<size_t>(per, 1), (size_t)kMaxBatch);
-    return std::max(1, std::min(R, nrhs));
 }
 
 int validate(const helm3d_grid *g, const helm3d_opts *o) {
@@ -98,14 +116,16 @@ int validate(const helm3d_grid *g, const helm3d_opts *o) {
 
 // Start of a call that runs the operator or the preconditioner: refused
 // after a failed set-up or factor of this context (that error again), else
-// the device status word is cleared, so that a bounded wait that expired or
+// the device status word is cleared (unless it was last read as zero), so that a bounded wait that expired or
 // an index check that failed in an earlier call is not reported again (the
 // factor's own bits were reported when it ran).
 int h3d::begin_call(helm3d_ctx *c) {
     if (c->factor_rc)
         return set_error(c, c->factor_rc,
                          std::string("the context's last set-up or factor failed: ") + helm3d_status_string(c->factor_rc));
-    return cuda_check(c, cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream), "status reset");
+    const bool clear = c->status_clear;
+    c->status_clear = false;   // until check_status has read it after this call's kernels
+    return clear ? HELM3D_OK : cuda_check(c, cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream), "status reset");
 }
 
 extern "C" {
@@ -477,6 +497,8 @@ struct DevBuf {
 static int apply_common(helm3d_ctx *c, const double *x, double *y, int which) {
     if (!c || !x || !y) return HELM3D_ERR_ARG;
     cudaSetDevice(c->device);
+    // mode N's operator is one kernel that reports nothing in the status word
+    const bool plain = which <= 1 && c->opts.mode == HELM3D_MODE_N;
     if (int rc = begin_call(c)) return rc;
     VecArg xa(c, x, c->N, true, &c->d_f, &c->f_cap);
     if (xa.rc) return xa.rc;
@@ -492,7 +514,10 @@ static int apply_common(helm3d_ctx *c, const double *x, double *y, int which) {
     if (rc) return rc;
     rc = ya.copy_out(y, c->N);
     if (rc) return rc;
-    return check_status(c);
+    if (!plain) return check_status(c);
+    rc = cuda_check(c, cudaStreamSynchronize(c->stream), "operator");
+    c->status_clear = rc == HELM3D_OK;
+    return rc;
 }
 
 int helm3d_apply_op(helm3d_ctx *c, const double *x, double *y) { return apply_common(c, x, y, 0); }
@@ -541,7 +566,7 @@ int helm3d_misfit_grad(helm3d_ctx *c, const double *f, int nsrc, const long long
     int rc;
     // receivers: checked on the host, used from the device
     std::vector<long long> hrecv((size_t)nrecv);
-    DevBuf d_recv, d_data, d_grad, d_u, d_lam, d_adj, d_res;
+    DevBuf d_recv, d_data, d_grad, d_res;
     if (nrecv > 0) {
         if ((rc = cuda_check(c, cudaMemcpy(hrecv.data(), recv, sizeof(long long) * nrecv, cudaMemcpyDefault),
                              "receivers")))
@@ -571,11 +596,16 @@ int helm3d_misfit_grad(helm3d_ctx *c, const double *f, int nsrc, const long long
     const bool fstaged = !is_device_ptr(f);
     const int B = batch_size(c, nsrc, fstaged, 3);
     const size_t vb = sizeof(double2) * (size_t)N;
-    if ((rc = d_u.alloc(c, vb * B, "wavefields")) || (rc = d_lam.alloc(c, vb * B, "adjoint wavefields")) ||
-        (rc = d_adj.alloc(c, vb * B, "adjoint sources")) ||
-        (nrecv > 0 && (rc = d_res.alloc(c, sizeof(double2) * (size_t)B * nrecv, "receiver residuals"))))
-        return rc;
-    double2 *U = (double2 *)d_u.p, *Lam = (double2 *)d_lam.p, *Adj = (double2 *)d_adj.p, *Res = (double2 *)d_res.p;
+    // the wavefields are kept by the context (allocating and freeing them
+    // took longer than a small gradient's kernels)
+    if (c->grad_bytes < 3 * vb * B) {
+        release_grad(c);
+        if ((rc = cuda_check(c, cudaMalloc(&c->d_grad, 3 * vb * B), "wavefields"))) return rc;
+        c->grad_bytes = 3 * vb * B;
+        c->bytes += c->grad_bytes;
+    }
+    if (nrecv > 0 && (rc = d_res.alloc(c, sizeof(double2) * (size_t)B * nrecv, "receiver residuals"))) return rc;
+    double2 *U = (double2 *)c->d_grad, *Lam = U + (size_t)B * N, *Adj = Lam + (size_t)B * N, *Res = (double2 *)d_res.p;
     std::vector<double2> hres((size_t)B * std::max(nrecv, 0));
     const double w2 = c->grid.omega * c->grid.omega;
     double J = 0.0;
@@ -637,6 +667,8 @@ int helm3d_destroy(helm3d_ctx *c) {
     for (float *p : c->d_ztc)
         if (p) cudaFree(p);
     for (auto &g : c->graphs) cudaGraphExecDestroy(g.exec);
+    for (auto &g : c->groups) cudaGraphExecDestroy(g.exec);
+    if (c->d_grad) cudaFree(c->d_grad);
     if (c->d_arn) cudaFree(c->d_arn);
     for (auto &e : c->prof_ev) {
         cudaEventDestroy(e.a);

@@ -256,6 +256,15 @@ int launch_update2(const VecBatch &V, long ldv, int j, const double2 *coef, long
 // flags[2] = max k.
 int launch_cycle_end(const VecBatch &V, long ldv, const ArnState &arn, bool tail, long N, int R, const Reduce &red,
                      cudaStream_t s);
+// The start of a cycle for B right-hand sides: nf, tol, it, max_iter, g[0] =
+// beta, the scale of V_0, nothing frozen, zero flags.
+struct CycleInit {
+    double nf[kMaxBatch], beta[kMaxBatch];
+    int it[kMaxBatch];
+    double tol;
+    int max_iter;
+};
+int launch_cycle_init(const ArnState &a, const CycleInit &ci, cudaStream_t s);
 // out[r * sOut].x = ||x_r||^2 and, with box, out[r * sOut + 1].x over the box
 // [x0,x1) x [y0,y1) x [z0,z1)
 int launch_norm2(const VecBatch &x, int R, int nx, int ny, int nz, const int *box, const Reduce &red, double2 *out,
@@ -410,6 +419,7 @@ struct helm3d_ctx {
     void *d_planes = nullptr;      // spectral planes, P precision (planes_R right-hand sides)
     int planes_R = 0;
     int *d_status = nullptr;
+    bool status_clear = false;     // the device word was last read as zero and no kernel has run since
     int factor_rc = HELM3D_OK;   // status of the last set-up and factor (set_medium)
     // Krylov workspace for r_alloc right-hand sides of restart length m_alloc
     int m_alloc = 0, r_alloc = 0;
@@ -425,6 +435,15 @@ struct helm3d_ctx {
         long long kernels_per_step, tail_kernels;
     };
     std::vector<CycleGraph> graphs;
+    unsigned long long epoch = 0;               // a number of its own whenever captured launches go stale
+    // group cycles led by this context (helm3d_solve_group), a few, the oldest replaced
+    struct GroupGraph {
+        std::vector<unsigned long long> epochs; // of the contexts in the cycle
+        std::vector<int> key;                   // batch per context (0: not in the cycle)
+        cudaGraphExec_t exec;
+        std::vector<long long> per_step, tail;
+    };
+    std::vector<GroupGraph> groups;
     bool use_graphs = true;
     bool gs_lowsync = true;                     // mode N: DCGS2 (HELM3D_GS=cgs2: classical CGS2)
     // autotuned launch variants: the factor's, and the sweep's (forward,
@@ -444,6 +463,8 @@ struct helm3d_ctx {
     long red_stride = 0;           // partials of one right-hand side
     double2 *d_f = nullptr, *d_u = nullptr, *d_r = nullptr, *d_t = nullptr, *d_t2 = nullptr;
     double2 *d_bic = nullptr;      // BiCGStab vectors
+    void *d_grad = nullptr;        // misfit gradient: wavefields, adjoint wavefields and sources
+    size_t grad_bytes = 0;
     size_t bytes = 0;
 
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -506,5 +527,8 @@ int cuda_check(helm3d_ctx *c, cudaError_t e, const char *what);
 int check_status(helm3d_ctx *c);
 // Start of a call that runs kernels on the context (see capi.cpp).
 int begin_call(helm3d_ctx *c);
+// The captured launches of the context (its cycle graphs, and any group cycle
+// that holds it) are stale: its workspace, planes or skipped modes moved.
+void drop_graphs(helm3d_ctx *c);
 void build_fft_plan(int n, FftPlan &plan, std::vector<zc> &tables);
 }  // namespace h3d

@@ -416,6 +416,19 @@ __global__ void __launch_bounds__(kRedThreads) update2_kernel(UpdateK a) {
     update_end<false>(a, r, pass, nrm, sc);
 }
 
+__global__ void cycle_init_kernel(ArnState a, CycleInit ci) {
+    const int p = threadIdx.x;
+    if (p < kArnFlags) a.flags[p] = 0;
+    if (p >= a.B) return;
+    a.nf[p] = ci.nf[p];
+    a.tol[p] = ci.tol;
+    a.it[p] = ci.it[p];
+    a.max_iter[p] = ci.max_iter;
+    a.frozen[p] = a.k[p] = 0;
+    a.g[(long)p * (a.m + 1)] = make_double2(ci.beta[p], 0.0);
+    a.vs[(long)p * a.M2] = 1.0 / ci.beta[p];
+}
+
 // x += sum_i y[i] zs[i] Z_i  (i < *nzv_dev when given, else nzv); Z complex128 or complex64
 template <typename TZ>
 __global__ void __launch_bounds__(kRedThreads) combine_kernel(const TZ *__restrict__ Z, long ldz, long sZ,
@@ -690,6 +703,12 @@ int launch_combine(const VecBatch &Z, long ldz, const ScaleBatch &zs, int nzv, c
     else
         combine_kernel<double2><<<grid, kRedThreads, sm, s>>>(Z.p, ldz, Z.stride, zs.p, zs.stride, nzv, y, sY, x.p,
                                                               x.stride, N, nzv_dev);
+    return ok() ? HELM3D_OK : HELM3D_ERR_CUDA;
+}
+
+int launch_cycle_init(const ArnState &a, const CycleInit &ci, cudaStream_t s) {
+    static_assert(kMaxBatch <= 32 && kArnFlags <= 32, "one warp");
+    cycle_init_kernel<<<1, 32, 0, s>>>(a, ci);
     return ok() ? HELM3D_OK : HELM3D_ERR_CUDA;
 }
 

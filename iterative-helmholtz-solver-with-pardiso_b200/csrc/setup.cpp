@@ -405,6 +405,7 @@ int ctx_setup_grid(helm3d_ctx *c) {
     if ((rc = dalloc(c, &c->d_planes, esz * c->N + 256, "planes"))) return rc;
     c->planes_R = 1;
     if ((rc = dalloc(c, (void **)&c->d_status, 64, "status"))) return rc;
+    drop_graphs(c);   // the context's first epoch
     c->ldg = (nx + 3) & ~3;
     c->Gt_bytes = esz * (size_t)nz * ny * nx * c->ldg;
     if ((rc = dalloc(c, &c->d_Gt, c->Gt_bytes, "block LU factor"))) return rc;
@@ -424,6 +425,7 @@ int ctx_setup_medium(helm3d_ctx *c, const double *s2, bool s2_on_device) {
     const double w2 = g.omega * g.omega;
     int rc = cuda_check(c, cudaMemsetAsync(c->d_status, 0, 64, c->stream), "status reset");
     if (rc) return rc;
+    c->status_clear = false;
     if (o.mode == HELM3D_MODE_N) {
         rc = cuda_check(c, cudaMemcpyAsync(c->d_s2, s2, sizeof(double) * c->N,
                                            s2_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c->stream),
@@ -510,6 +512,7 @@ static int setup_kz_skip(helm3d_ctx *c) {
     c->nskip = 0;
     c->kzslot_h.assign(nz, -1);
     if (!(o.kz_skip_ratio > 0)) return HELM3D_OK;
+    drop_graphs(c);   // captured sweeps hold the last medium's skipped modes
     int rc;
     double k2 = 0.0;
     if (o.s2_l0 > 0) {

@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -99,9 +100,11 @@ static ArnState arn_state(helm3d_ctx *c, int m, int B) {
     return a;
 }
 
-static void drop_graphs(helm3d_ctx *c) {
+void drop_graphs(helm3d_ctx *c) {
+    static std::atomic<unsigned long long> next{1};
     for (auto &g : c->graphs) cudaGraphExecDestroy(g.exec);
     c->graphs.clear();
+    c->epoch = next++;   // of this context at this time only: no group cycle captured before matches
 }
 
 static void free_krylov(helm3d_ctx *c) {
@@ -232,6 +235,7 @@ static int prec_to_planes(helm3d_ctx *c, const VecBatch &x, double xscale, const
                           bool adjoint) {
     RC(check_batch(c, R));
     RC(ensure_planes(c, R));
+    c->status_clear = false;
     const PlaneLayout L = layout(c, R);
     RC(timed(c, HELM3D_K_FFT_FWD, 1, [&] {
         if (c->ztc)
@@ -363,9 +367,14 @@ static int norms(helm3d_ctx *c, const VecBatch &x, int R, bool phys, double2 *ou
 }
 
 int check_status(helm3d_ctx *c) {
-    int st = 0;
-    RC(cuda_check(c, cudaMemcpyAsync(&st, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "status"));
+    // into pinned memory where a solve has left some (pinning costs a new
+    // context more than the pageable copy costs an apply)
+    int pageable = 0;
+    int *st_h = c->h_scal ? reinterpret_cast<int *>(c->h_scal) : &pageable;
+    RC(cuda_check(c, cudaMemcpyAsync(st_h, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "status"));
     RC(cuda_check(c, cudaStreamSynchronize(c->stream), "status sync"));
+    const int st = *st_h;
+    c->status_clear = st == 0;
     if (st & 6) return set_error(c, HELM3D_ERR_CUDA, "a bounded wait expired in a kernel");
     if (st & 8) return set_error(c, HELM3D_ERR_CUDA, "an index check failed in a kernel");
     return HELM3D_OK;
@@ -450,8 +459,10 @@ static int arnoldi_step(helm3d_ctx *c, int m, int B, int j, bool adjoint, const 
     });
 }
 
-// end of a cycle: y = R^{-1} g on the device, x += Z y (mode R: V y)
-static int cycle_tail(helm3d_ctx *c, int m, int B, const ArnState &a) {
+// end of a cycle: y = R^{-1} g on the device, x += Z y (mode R: V y), the true
+// residual f - A x into V_0 and its norms, so that the host reads all it needs
+// for the next cycle at once
+static int cycle_tail(helm3d_ctx *c, int m, int B, bool adjoint, const ArnState &a) {
     const long N = c->N;
     const long ldV = (long)(m + 1) * N, ldZ = (long)m * N;
     const int M2 = m + 2, SH = scalars_per_rhs(m);
@@ -461,13 +472,16 @@ static int cycle_tail(helm3d_ctx *c, int m, int B, const ArnState &a) {
     RC(timed(c, HELM3D_K_KRYLOV, 1, [&] {
         return launch_cycle_end(VecBatch{c->d_V, ldV}, N, a, lowsync(c), N, B, reducer(c), c->stream);
     }));
-    return timed(c, HELM3D_K_KRYLOV, 1, [&] {
+    RC(timed(c, HELM3D_K_KRYLOV, 1, [&] {
         return c->opts.mode == HELM3D_MODE_N
                    ? launch_combine(zbasis(c, 0, ldZ), N, kNoScale, m, d_y, SH, VecBatch{c->d_Uw, N}, N, B,
                                     c->stream, a.flags + 2)
                    : launch_combine(VecBatch{c->d_V, ldV}, N, ScaleBatch{c->d_vs, M2}, m, d_y, SH,
                                     VecBatch{c->d_Uw, N}, N, B, c->stream, a.flags + 2);
-    });
+    }));
+    const VecBatch V0{c->d_V, ldV};
+    RC(residual(c, VecBatch{c->d_Fw, N}, VecBatch{c->d_Uw, N}, V0, B, adjoint));
+    return norms(c, V0, B, true, c->d_h + 2 * M2, SH);
 }
 
 // Adds the restart cycle of context c (a batch of B) to graph G as one more
@@ -519,7 +533,7 @@ static bool add_cycle(cudaGraph_t G, helm3d_ctx *c, int m, int B, bool adjoint, 
         ok = cudaStreamBeginCaptureToGraph(cap, G, &prev, nullptr, 1, cudaStreamCaptureModeRelaxed) == cudaSuccess;
         if (ok) {
             const long long l0 = c->launches;
-            const int rc = cycle_tail(c, m, B, a);
+            const int rc = cycle_tail(c, m, B, adjoint, a);
             cudaGraph_t out = nullptr;
             ok = cudaStreamEndCapture(cap, &out) == cudaSuccess && rc == HELM3D_OK;
             tail = c->launches - l0;
@@ -637,6 +651,7 @@ struct Rhs {
     bool frozen = false;      // converged inside the current cycle: no more columns
     int k = 0;                // columns of the current cycle
     double beta = 0;
+    double b2 = 0, p2 = 0;    // ||r||^2 of the current residual, whole grid and physical domain
     std::vector<zc> H, cs, sn, gv;
 };
 }  // namespace
@@ -662,12 +677,9 @@ struct FgmresRun {
     std::vector<Rhs> S;
     std::vector<int> act;        // packed position p -> right-hand side
     bool x_zero = true;
+    bool have_res = false;       // V_0 holds the residual of the active batch and its norms are in the Rhs (b2, p2)
     int B = 0;                   // batch of the current cycle
-    std::vector<double> vs0;
     std::vector<double2> ybuf;
-    std::vector<int> iv;         // device cycle state of the current cycle (host side)
-    std::vector<double> dv, est;
-    std::vector<double2> g0;
 
     FgmresRun(helm3d_ctx *c_, const double2 *f_, double2 *u_, int R_, bool adj, helm3d_stats *st_)
         : c(c_), f(f_), u(u_), R(R_), adjoint(adj), st(st_) {}
@@ -708,6 +720,7 @@ struct FgmresRun {
     }
 
     int begin() {
+        c->status_clear = false;   // until check_status (an error may return before it)
         const helm3d_opts &o = c->opts;
         flexible = (o.mode == HELM3D_MODE_N);
         if (adjoint && !flexible) return set_error(c, HELM3D_ERR_ARG, "adjoint solve is mode N only");
@@ -725,7 +738,7 @@ struct FgmresRun {
         // the pinned mirror lives in the context: pinning and unpinning host
         // memory are driver calls (cudaFreeHost also waits for the device),
         // kept out of every solve after the first of a size
-        const size_t need = (size_t)SH * R;
+        const size_t need = (size_t)SH * R + (arn_bytes(m, c->r_alloc) + sizeof(double2) - 1) / sizeof(double2);
         if (c->h_scal_cap < need) {
             if (c->h_scal) cudaFreeHost(c->h_scal);
             c->h_scal = nullptr;
@@ -742,14 +755,17 @@ struct FgmresRun {
         RC(cuda_check(c, cudaMemcpyAsync(c->d_Fw, f, vb * R, cudaMemcpyDeviceToDevice, c->stream), "f copy"));
         RC(cuda_check(c, cudaMemsetAsync(c->d_Uw, 0, vb * R, c->stream), "x0"));
         RC(cuda_check(c, cudaMemsetAsync(u, 0, vb * R, c->stream), "u0"));
-        RC(norms(c, VecBatch{c->d_Fw, N}, R, false, c->d_h + 2 * M2, SH));
+        RC(norms(c, VecBatch{c->d_Fw, N}, R, true, c->d_h + 2 * M2, SH));
         RC(fetch_scalars(R, "norms of f"));
         S.assign(R, Rhs());
         act.clear();
         for (int r = 0; r < R; r++) {
             Rhs &q = S[r];
             q.orig = r;
-            q.nf = std::sqrt(hbuf[(size_t)r * SH + 2 * M2].x);
+            // x0 = 0: the first residual is f
+            q.b2 = hbuf[(size_t)r * SH + 2 * M2].x;
+            q.p2 = hbuf[(size_t)r * SH + 2 * M2 + 1].x;
+            q.nf = std::sqrt(q.b2);
             if (!std::isfinite(q.nf)) return set_error(c, HELM3D_ERR_NONFINITE, "right-hand side has NaN/Inf");
             q.H.assign((size_t)(m + 1) * m, zc(0, 0));
             q.cs.assign(m, zc(0, 0));
@@ -765,7 +781,7 @@ struct FgmresRun {
             }
         RC(retire(false));
         x_zero = true;
-        vs0.assign(R, 0.0);
+        have_res = false;
         ybuf.assign((size_t)M2 * R, make_double2(0, 0));
         return HELM3D_OK;
     }
@@ -783,15 +799,17 @@ struct FgmresRun {
             RC(cuda_check(c, cudaMemcpy2DAsync(V, sizeof(double2) * ldV, c->d_Fw, vb, vb, A,
                                                cudaMemcpyDeviceToDevice, c->stream),
                           "r0"));
-        } else {
+        } else if (!have_res) {
             RC(residual(c, VecBatch{c->d_Fw, N}, VecBatch{c->d_Uw, N}, V0, A, adjoint));
+            RC(norms(c, V0, A, true, c->d_h + 2 * M2, SH));
+            RC(fetch_scalars(A, "residual norms"));
+            take_norms(A);
         }
-        RC(norms(c, V0, A, true, c->d_h + 2 * M2, SH));
-        RC(fetch_scalars(A, "residual norms"));
+        have_res = false;
         bool any_done = false;
         for (int p = 0; p < A; p++) {
             Rhs &r = S[act[p]];
-            const double b2 = hbuf[(size_t)p * SH + 2 * M2].x, p2 = hbuf[(size_t)p * SH + 2 * M2 + 1].x;
+            const double b2 = r.b2, p2 = r.p2;
             r.beta = std::sqrt(b2);
             if (!std::isfinite(r.beta)) return set_error(c, HELM3D_ERR_NONFINITE, "residual is NaN/Inf");
             r.relres = r.beta / r.nf;
@@ -807,43 +825,33 @@ struct FgmresRun {
         B = (int)act.size();
         for (int p = 0; p < B; p++) {
             Rhs &r = S[act[p]];
-            vs0[p] = 1.0 / r.beta;
             std::fill(r.H.begin(), r.H.end(), zc(0, 0));
             std::fill(r.gv.begin(), r.gv.end(), zc(0, 0));
             r.gv[0] = r.beta;
             r.frozen = false;
             r.k = 0;
         }
-        return cuda_check(c, cudaMemcpy2DAsync(c->d_vs, sizeof(double) * M2, vs0.data(), sizeof(double),
-                                               sizeof(double), B, cudaMemcpyHostToDevice, c->stream),
-                          "vs0");
-    }
-
-    // the device cycle state of the batch in (before the graph or the steps)
-    int upload_state() {
-        const helm3d_opts &o = c->opts;
-        const ArnState a = arn_state(c, m, B);
-        const int Ra = c->r_alloc;
-        dv.assign((size_t)2 * Ra, 0.0);
-        iv.assign((size_t)4 * Ra + kArnFlags, 0);
-        g0.assign((size_t)B, make_double2(0, 0));
+        // the device state of the cycle (and V_0's scales)
+        CycleInit ci = {};
+        ci.tol = o.tol;
+        ci.max_iter = o.max_iter;
         for (int p = 0; p < B; p++) {
             const Rhs &r = S[act[p]];
-            dv[p] = r.nf;
-            dv[Ra + p] = o.tol;
-            iv[2 * Ra + p] = r.it;
-            iv[3 * Ra + p] = o.max_iter;
-            g0[p] = make_double2(r.beta, 0.0);
+            ci.nf[p] = r.nf;
+            ci.beta[p] = r.beta;
+            ci.it[p] = r.it;
         }
-        RC(cuda_check(c, cudaMemcpyAsync(a.nf, dv.data(), sizeof(double) * dv.size(), cudaMemcpyHostToDevice,
-                                         c->stream),
-                      "cycle state"));
-        RC(cuda_check(c, cudaMemcpyAsync(a.frozen, iv.data(), sizeof(int) * iv.size(), cudaMemcpyHostToDevice,
-                                         c->stream),
-                      "cycle state"));
-        return cuda_check(c, cudaMemcpy2DAsync(a.g, sizeof(double2) * (m + 1), g0.data(), sizeof(double2),
-                                               sizeof(double2), B, cudaMemcpyHostToDevice, c->stream),
-                          "cycle state");
+        const ArnState a = arn_state(c, m, B);
+        return timed(c, HELM3D_K_KRYLOV, 1, [&] { return launch_cycle_init(a, ci, c->stream); });
+    }
+
+    // the residual norms of the first A active right-hand sides, from hbuf
+    void take_norms(int A) {
+        for (int p = 0; p < A; p++) {
+            Rhs &r = S[act[p]];
+            r.b2 = hbuf[(size_t)p * SH + 2 * M2].x;
+            r.p2 = hbuf[(size_t)p * SH + 2 * M2 + 1].x;
+        }
     }
 
     // a device cycle without a graph: the steps one by one, the host checking
@@ -859,23 +867,25 @@ struct FgmresRun {
             if (c->opts.verbose) fprintf(stderr, "helm3d: step %d, %s\n", j + 1, active ? "active" : "done");
             if (!active) break;
         }
-        return cycle_tail(c, m, B, a);
+        return cycle_tail(c, m, B, adjoint, a);
     }
 
     // the device cycle state out; per_step / tail: kernels of a graph launch
     // (counted here), or -1 when the steps were launched (already counted)
     int cycle_end_device(long long per_step, long long tail) {
+        // est, nf, tol, beta and the integers are one block (arn_state)
         const ArnState a = arn_state(c, m, B);
         const int Ra = c->r_alloc;
-        est.assign((size_t)Ra * m, 0.0);
-        RC(cuda_check(c, cudaMemcpyAsync(iv.data(), a.frozen, sizeof(int) * iv.size(), cudaMemcpyDeviceToHost,
-                                         c->stream),
-                      "cycle result"));
-        RC(cuda_check(c, cudaMemcpyAsync(est.data(), a.est, sizeof(double) * est.size(), cudaMemcpyDeviceToHost,
-                                         c->stream),
-                      "cycle result"));
-        RC(cuda_check(c, cudaStreamSynchronize(c->stream), "cycle"));
-        const int *flags = iv.data() + 4 * Ra;
+        const size_t scal = sizeof(double2) * (size_t)SH * B;
+        const size_t dbl = (size_t)Ra * (m + 3), arn = sizeof(double) * dbl + sizeof(int) * ((size_t)4 * Ra + kArnFlags);
+        char *hs = reinterpret_cast<char *>(hbuf) + scal;
+        RC(cuda_check(c, cudaMemcpyAsync(hs, a.est, arn, cudaMemcpyDeviceToHost, c->stream), "cycle result"));
+        RC(fetch_scalars(B, "cycle"));
+        take_norms(B);
+        have_res = true;
+        const double *est = reinterpret_cast<const double *>(hs);
+        const int *iv = reinterpret_cast<const int *>(est + dbl);
+        const int *flags = iv + 4 * Ra;
         if (flags[3]) return set_error(c, HELM3D_ERR_NONFINITE, "Arnoldi norm is NaN/Inf");
         const int kmax = flags[2];
         c->reorth += flags[1];
@@ -1057,11 +1067,9 @@ int fgmres(helm3d_ctx *c, const double2 *f, double2 *u, int R, bool adjoint, hel
         if (run.B == 0) break;
         const int gi = run.graphs_usable() ? cycle_graph(c, run.m, run.B, adjoint) : -1;
         if (gi >= 0) {
-            RC(run.upload_state());
             RC(cuda_check(c, cudaGraphLaunch(c->graphs[gi].exec, c->stream), "cycle graph"));
             RC(run.cycle_end_device(c->graphs[gi].kernels_per_step, c->graphs[gi].tail_kernels));
         } else if (lowsync(c)) {
-            RC(run.upload_state());
             RC(run.run_steps());
             RC(run.cycle_end_device(-1, 0));
         } else {
@@ -1076,11 +1084,6 @@ int fgmres(helm3d_ctx *c, const double2 *f, double2 *u, int R, bool adjoint, hel
 // as independent chains of one graph, so that the kernels of grids of
 // different sizes run side by side on the GPU.
 namespace {
-struct GroupGraph {
-    std::vector<int> key;                  // batch per context (0: not in the cycle)
-    cudaGraphExec_t exec = nullptr;
-    std::vector<long long> per_step, tail;
-};
 struct StreamGuard {
     std::vector<helm3d_ctx *> cs;
     std::vector<cudaStream_t> saved;
@@ -1106,14 +1109,12 @@ int fgmres_group(helm3d_ctx *const *cs, int n, const double2 *const *f, double2 
         runs.emplace_back(new FgmresRun(cs[i], f[i], u[i], R[i], false, st[i]));
         RC(runs.back()->begin());
     }
-    std::vector<GroupGraph> graphs;
-    struct Cleanup {
-        std::vector<GroupGraph> *g;
-        ~Cleanup() {
-            for (auto &x : *g)
-                if (x.exec) cudaGraphExecDestroy(x.exec);
-        }
-    } cleanup{&graphs};
+    // the leader keeps a few group cycles across calls (building one takes
+    // longer than a small group's cycle runs); one matches while every context
+    // in it has the epoch it was captured at
+    constexpr size_t kKeep = 4;
+    std::vector<helm3d_ctx::GroupGraph> &graphs = cs[0]->groups;
+    std::vector<unsigned long long> epochs(n);
     bool use_group = true;
     for (int i = 0; i < n; i++) use_group = use_group && runs[i]->graphs_usable();
     for (;;) {
@@ -1128,20 +1129,31 @@ int fgmres_group(helm3d_ctx *const *cs, int n, const double2 *const *f, double2 
         if (!any) break;
         int gi = -1;
         if (use_group) {
+            for (int i = 0; i < n; i++) {
+                // what a capture would move, moved before the epochs are compared
+                if (key[i] > 0) RC(ensure_planes(cs[i], key[i]));
+                epochs[i] = key[i] > 0 ? cs[i]->epoch : 0;
+            }
             for (size_t q = 0; q < graphs.size(); q++)
-                if (graphs[q].key == key) gi = (int)q;
+                if (graphs[q].key == key && graphs[q].epochs == epochs) gi = (int)q;
             if (gi < 0) {
-                GroupGraph g;
+                helm3d_ctx::GroupGraph g;
                 g.key = key;
+                g.epochs = epochs;
                 g.per_step.assign(n, 0);
                 g.tail.assign(n, 0);
                 cudaGraph_t G = nullptr;
                 bool ok = cudaGraphCreate(&G, 0) == cudaSuccess;
                 for (int i = 0; ok && i < n; i++)
                     if (key[i] > 0) ok = add_cycle(G, cs[i], runs[i]->m, key[i], false, g.per_step[i], g.tail[i]);
+                g.exec = nullptr;
                 if (ok) ok = cudaGraphInstantiate(&g.exec, G, 0) == cudaSuccess;
                 if (G) cudaGraphDestroy(G);
                 if (ok) {
+                    if (graphs.size() >= kKeep) {
+                        cudaGraphExecDestroy(graphs.front().exec);
+                        graphs.erase(graphs.begin());
+                    }
                     graphs.push_back(g);
                     gi = (int)graphs.size() - 1;
                 } else {
@@ -1151,8 +1163,6 @@ int fgmres_group(helm3d_ctx *const *cs, int n, const double2 *const *f, double2 
             }
         }
         if (gi >= 0) {
-            for (int i = 0; i < n; i++)
-                if (key[i] > 0) RC(runs[i]->upload_state());
             RC(cuda_check(cs[0], cudaGraphLaunch(graphs[gi].exec, gs), "group cycle graph"));
             for (int i = 0; i < n; i++)
                 if (key[i] > 0) RC(runs[i]->cycle_end_device(graphs[gi].per_step[i], graphs[gi].tail[i]));
@@ -1164,12 +1174,10 @@ int fgmres_group(helm3d_ctx *const *cs, int n, const double2 *const *f, double2 
             helm3d_ctx *c = cs[i];
             const int g1 = run.graphs_usable() ? cycle_graph(c, run.m, run.B, false) : -1;
             if (g1 >= 0) {
-                RC(run.upload_state());
-                RC(cuda_check(c, cudaGraphLaunch(c->graphs[g1].exec, c->stream), "cycle graph"));
+                    RC(cuda_check(c, cudaGraphLaunch(c->graphs[g1].exec, c->stream), "cycle graph"));
                 RC(run.cycle_end_device(c->graphs[g1].kernels_per_step, c->graphs[g1].tail_kernels));
             } else if (lowsync(c)) {
-                RC(run.upload_state());
-                RC(run.run_steps());
+                    RC(run.run_steps());
                 RC(run.cycle_end_device(-1, 0));
             } else {
                 RC(run.run_host_cycle());
