@@ -182,11 +182,11 @@ struct StencilArgs {
     VecBatch y;
     VecBatch f;               // if f.p: y = f - A x
     int R;
-    int zchunk = 16;          // z points per thread (autotuned: 8, 16, 32, 64)
-    int src_fast = 0;         // grid z order: 0 = z chunks within a source, 1 = sources within a z chunk
-    int smem = 0;             // 1: x/y neighbours from the plane's tile staged in shared memory
+    int zblock = 2;           // z points per thread (1, 2; 4, 6, 8, 12: blocks in shared memory)
+    int src_fast = 0;         // grid z order: 0 = z blocks within a source, 1 = sources within a z block
 };
 int launch_stencil(const StencilArgs &a, bool adjoint, cudaStream_t s);
+int stencil_default(int nx, int ny, int nz, int R);   // zblock of an untuned launch
 
 // ------------------------------------------------------ Krylov kernels
 // All vectors complex128 of length N; a basis V_r of nv vectors (leading
@@ -339,14 +339,13 @@ bool tune_enabled();
 uint32_t wait_limit_polls(uint32_t dflt);
 // HELM3D_FORCE_<family> as an integer, or -1 when unset
 int tune_forced(const char *family);
-// z chunk 16, 8, 32, 64; source-major (0-3) or source-minor (4-7) grid;
-// 8-11: the shared-memory staged kernel, source-minor, z chunk 16, 32, 64, 8
+// z points per thread 8, 1, 2, 4, 6, 12 (1, 2: the register kernel, else blocks in
+// shared memory); source-major (0-5) or source-minor (6-11) grid
 constexpr int kStencilVariants = 12;
 constexpr int kReduceVariants = 3;    // reduction blocks 2, 1, 4 per SM
 constexpr int kUpdateVariants = 2;    // DCGS2 update pass: basis loads one by one, 8 batched
-int stencil_zchunk(int v);
+int stencil_zblock(int v);
 int stencil_src_fast(int v);
-int stencil_smem(int v);
 int reduce_blocks(int v);
 
 }  // namespace h3d
@@ -452,7 +451,7 @@ struct helm3d_ctx {
     int tv_factor = 0;
     int tv_sweep[2] = {0, 0};
     int tv_sweep_R[2] = {0, 0};                 // the batch tv_sweep was chosen for (0: none yet, sweep_default)
-    int tv_stencil = 0;
+    int tv_stencil = -1;                        // -1: not tuned, stencil_default
     int tv_update = 0;
     size_t f_cap = 0, u_cap = 0;                // staging capacities (vectors) of d_f, d_u
     double *d_vs = nullptr;

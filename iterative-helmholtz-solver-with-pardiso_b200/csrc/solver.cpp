@@ -295,9 +295,8 @@ static StencilArgs stencil_args(helm3d_ctx *c, const VecBatch &x, double xscale,
     a.y = y;
     a.f = f;
     a.R = R;
-    a.zchunk = stencil_zchunk(c->tv_stencil);
+    a.zblock = c->tv_stencil >= 0 ? stencil_zblock(c->tv_stencil) : stencil_default(a.nx, a.ny, a.nz, R);
     a.src_fast = stencil_src_fast(c->tv_stencil);
-    a.smem = stencil_smem(c->tv_stencil);
     return a;
 }
 
@@ -575,7 +574,7 @@ int tune_solve(helm3d_ctx *c, int R, bool adjoint) {
                             std::getenv("HELM3D_FORCE_REDUCE") || std::getenv("HELM3D_FORCE_UPDATE");
     if (!tune_enabled() && !any_forced) {
         c->tv_sweep_R[0] = c->tv_sweep_R[1] = 0;   // sweep_default
-        c->tv_stencil = 0;
+        c->tv_stencil = -1;
         c->tv_update = 0;
         c->red_blocks = reduce_blocks(0);
         return HELM3D_OK;
@@ -600,14 +599,13 @@ int tune_solve(helm3d_ctx *c, int R, bool adjoint) {
     if (c->opts.mode == HELM3D_MODE_N) {
         // the stencil from Z_0 (its FGMRES input: complex64 when the
         // context keeps Z so) into V_1 of every right-hand side
-        std::snprintf(shape, sizeof(shape), "%d|%d|%d|%d|%d", g.nx, g.ny, g.nz, R, c->z64 ? 64 : 128);
+        std::snprintf(shape, sizeof(shape), "t2|%d|%d|%d|%d|%d", g.nx, g.ny, g.nz, R, c->z64 ? 64 : 128);
         StencilArgs a0 = stencil_args(c, zbasis(c, 0, (long)m * N), 1.0, kNoScale, VecBatch{c->d_V + N, ldV},
                                       VecBatch{nullptr, 0}, R);
         c->tv_stencil = tune_pick(c, "STENCIL", shape, kStencilVariants, [&](int v) {
             StencilArgs t = a0;
-            t.zchunk = stencil_zchunk(v);
+            t.zblock = stencil_zblock(v);
             t.src_fast = stencil_src_fast(v);
-            t.smem = stencil_smem(v);
             return launch_stencil(t, adjoint, c->stream);
         });
     }

@@ -1,6 +1,6 @@
 // tune.cpp -- the autotuner: for every kernel family with several launch
 // shapes (the factor's cluster and warp layout, the sweep's bulk-copy stage
-// and ring sizes, the stencil's z chunk and grid order, the number of
+// and ring sizes, the stencil's z points per thread and grid order, the number of
 // reduction blocks of the Gram-Schmidt passes, the update pass's load
 // batching), the shape that runs fastest on this device for a
 // given problem shape.  Each candidate is launched once to warm up and then
@@ -8,7 +8,7 @@
 // counts); the choice is kept for the process under a key of the family and
 // the sizes it depends on and, with HELM3D_TUNE_CACHE=<file>, read from and
 // appended to that file so that later processes skip the timing.
-//   HELM3D_TUNE=0             no timing: the default shape (variant 0) of every family
+//   HELM3D_TUNE=0             no timing: the default shape of every family (variant 0, or a rule on the sizes)
 //   HELM3D_FORCE_<FAMILY>=v   force variant v (FACTOR, SWEEP, STENCIL, REDUCE, UPDATE)
 #include <cuda_runtime.h>
 
@@ -139,16 +139,12 @@ int tune_pick(helm3d_ctx *c, const char *family, const std::string &shape, int n
     return best;
 }
 
-int stencil_zchunk(int v) {
-    static const int kZ[4] = {16, 8, 32, 64};
-    static const int kZs[4] = {16, 32, 64, 8};
-    if (v >= 8 && v < kStencilVariants) return kZs[v - 8];
-    return kZ[(v >= 0 && v < kStencilVariants) ? v % 4 : 0];
+int stencil_zblock(int v) {
+    static const int kZ[6] = {8, 1, 2, 4, 6, 12};
+    return kZ[(v >= 0 && v < kStencilVariants) ? v % 6 : 0];
 }
 
-int stencil_src_fast(int v) { return (v >= 4 && v < kStencilVariants) ? 1 : 0; }
-
-int stencil_smem(int v) { return (v >= 8 && v < kStencilVariants) ? 1 : 0; }
+int stencil_src_fast(int v) { return (v >= 6 && v < kStencilVariants) ? 1 : 0; }
 
 int reduce_blocks(int v) {
     static const int kPerSm[kReduceVariants] = {2, 1, 4};
