@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(kFtThreads, 1) factor_tc_kernel(FactorTcK a) {
                 // is linear in the row.  The next step's warp reduction is
                 // issued right after the update of the next pivot column.
                 float2 psc = make_float2(1.f, 0.f);
-                bool pivp = false;
+                bool pivp = false, bad = false;
                 uint32_t key = 0;
                 {
                     const float av = fabsf(P[0].x) + fabsf(P[0].y);
@@ -256,12 +256,15 @@ __global__ void __launch_bounds__(kFtThreads, 1) factor_tc_kernel(FactorTcK a) {
 #pragma unroll 1
                 for (int kk = 0; kk < bl; kk++) {
                     const int k = k0 + kk, buf = k & 1;
-                    if (lane == 0) sm.ckey[buf * 4 + warp] = kw;
-                    if (kw != 0u && key == kw) {
+                    st_shared_u32_if(lane == 0, smem_u32(&sm.ckey[buf * 4 + warp]), kw);
+                    {
                         // the winning row in register order: w[0] the pivot, w[1 + e] = prow[e]
-                        float4 *w = reinterpret_cast<float4 *>(sm.wrow + (buf * 4 + warp) * kFtB);
+                        const bool win = kw != 0u && key == kw;
+                        const uint32_t w = smem_u32(sm.wrow + (buf * 4 + warp) * kFtB);
 #pragma unroll
-                        for (int e = 0; e < kFtB / 2; e++) w[e] = make_float4(P[2 * e].x, P[2 * e].y, P[2 * e + 1].x, P[2 * e + 1].y);
+                        for (int e = 0; e < kFtB / 2; e++)
+                            st_shared_v4_if(win, w + 16u * (uint32_t)e,
+                                            make_float4(P[2 * e].x, P[2 * e].y, P[2 * e + 1].x, P[2 * e + 1].y));
                     }
                     ft_row_barrier();
                     const uint4 kv = *reinterpret_cast<const uint4 *>(sm.ckey + buf * 4);
@@ -290,23 +293,21 @@ __global__ void __launch_bounds__(kFtThreads, 1) factor_tc_kernel(FactorTcK a) {
                         else prow[2 * e - 1] = make_float2(q4.x, q4.y);
                         prow[2 * e] = make_float2(q4.z, q4.w);
                     }
-                    float2 pinv = make_float2(0.f, 0.f);
-                    if (r < 0 || (pv.x == 0.f && pv.y == 0.f)) {
-                        // no finite candidate, or an exactly zero pivot: flagged, the block is invalid
-                        if (t == 0) atomicOr(a.status, 1);
-                    } else {
-                        pinv = pivot_inv(pv);
-                    }
+                    // no finite candidate, or an exactly zero pivot: flagged (after
+                    // the panel), the block is invalid
+                    const bool none = r < 0 || (pv.x == 0.f && pv.y == 0.f);
+                    bad |= none;
+                    const float2 pi = pivot_inv(pv);
+                    const float2 pinv = make_float2(none ? 0.f : pi.x, none ? 0.f : pi.y);
                     // row -= (c / pv) * pivot row, column k becomes -c / pv
                     const bool ip = t == r;
                     float2 sfac = cmul(P[0], pinv);
-                    if (ip) {
-                        sfac = make_float2(0.f, 0.f);
-                        psc = pinv;
-                        used = pivp = true;
-                        my_step = k;
-                        sm.perm[k] = t;
-                    }
+                    sfac = make_float2(ip ? 0.f : sfac.x, ip ? 0.f : sfac.y);
+                    psc = make_float2(ip ? pinv.x : psc.x, ip ? pinv.y : psc.y);
+                    used |= ip;
+                    pivp |= ip;
+                    my_step = ip ? k : my_step;
+                    st_shared_u32_if(ip, smem_u32(&sm.perm[k]), (uint32_t)t);
                     P[0] = cfms(sfac, prow[0], P[1]);
                     key = 0;
                     {
@@ -318,6 +319,7 @@ __global__ void __launch_bounds__(kFtThreads, 1) factor_tc_kernel(FactorTcK a) {
                     for (int e = 1; e < kFtB - 1; e++) P[e] = cfms(sfac, prow[e], P[e + 1]);
                     P[kFtB - 1] = ip ? make_float2(1.f, 0.f) : make_float2(-sfac.x, -sfac.y);
                 }
+                if (bad && t == 0) atomicOr(a.status, 1);
                 // the panel's pivot row scaled by its 1 / pv
                 if (pivp) {
 #pragma unroll

@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                 // the next step's warp reduction right after the update of
                 // the next pivot column, before the other columns.
                 float2 sc0 = make_float2(1.f, 0.f), sc1 = sc0;
-                bool piv0 = false, piv1 = false;
+                bool piv0 = false, piv1 = false, bad = false;
                 uint32_t key0 = f2_key(P0[0], !used0, t);
                 uint32_t key1 = f2_key(P1[0], has1 && !used1, g1);
                 uint32_t key = key0 > key1 ? key0 : key1;
@@ -390,19 +390,17 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
 #pragma unroll 1
                 for (int kk = 0; kk < bl; kk++) {
                     const int k = k0 + kk, buf = k & 1;
-                    if (lane == 0) sm.wkey[buf * kF2RowWarps + warp] = kw;
-                    if (kw != 0u && key == kw) {
+                    st_shared_u32_if(lane == 0, smem_u32(&sm.wkey[buf * kF2RowWarps + warp]), kw);
+                    {
                         // the winning row in register order: w[0] the pivot, w[1 + e] = prow[e]
-                        float4 *w = reinterpret_cast<float4 *>(sm.wrow + (size_t)(buf * kF2RowWarps + warp) * kF2B);
-                        if (key0 == kw) {
+                        const bool win = kw != 0u && key == kw, first = key0 == kw;
+                        const uint32_t w = smem_u32(sm.wrow + (size_t)(buf * kF2RowWarps + warp) * kF2B);
 #pragma unroll
-                            for (int e = 0; e < kF2B / 2; e++)
-                                w[e] = make_float4(P0[2 * e].x, P0[2 * e].y, P0[2 * e + 1].x, P0[2 * e + 1].y);
-                        } else {
-#pragma unroll
-                            for (int e = 0; e < kF2B / 2; e++)
-                                w[e] = make_float4(P1[2 * e].x, P1[2 * e].y, P1[2 * e + 1].x, P1[2 * e + 1].y);
-                        }
+                        for (int e = 0; e < kF2B / 2; e++)
+                            st_shared_v4_if(win, w + 16u * (uint32_t)e,
+                                            make_float4(first ? P0[2 * e].x : P1[2 * e].x, first ? P0[2 * e].y : P1[2 * e].y,
+                                                        first ? P0[2 * e + 1].x : P1[2 * e + 1].x,
+                                                        first ? P0[2 * e + 1].y : P1[2 * e + 1].y));
                     }
                     f2_row_barrier();
                     const uint4 kv = *reinterpret_cast<const uint4 *>(sm.wkey + buf * kF2RowWarps);
@@ -431,29 +429,25 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                         else prow[2 * e - 1] = make_float2(q4.x, q4.y);
                         prow[2 * e] = make_float2(q4.z, q4.w);
                     }
-                    float2 pinv = make_float2(0.f, 0.f);
-                    if (r < 0 || (pv.x == 0.f && pv.y == 0.f)) {
-                        // no finite candidate, or an exactly zero pivot: flagged, the block is invalid
-                        if (t == 0 && rank == 0) atomicOr(a.status, 1);
-                    } else {
-                        pinv = pivot_inv(pv);
-                    }
-                    if (t == 0) sm.perm[k] = r >= 0 ? r : 0;
+                    // no finite candidate, or an exactly zero pivot: flagged (after
+                    // the panel), the block is invalid
+                    const bool none = r < 0 || (pv.x == 0.f && pv.y == 0.f);
+                    bad |= none;
+                    const float2 pi = pivot_inv(pv);
+                    const float2 pinv = make_float2(none ? 0.f : pi.x, none ? 0.f : pi.y);
+                    st_shared_u32_if(t == 0, smem_u32(&sm.perm[k]), (uint32_t)(r >= 0 ? r : 0));
                     // row -= (c / pv) * pivot row, column k becomes -c / pv
                     const bool ip0 = t == r, ip1 = g1 == r;
                     float2 s0 = cmul(P0[0], pinv), s1 = cmul(P1[0], pinv);
-                    if (ip0) {
-                        s0 = make_float2(0.f, 0.f);
-                        sc0 = pinv;
-                        used0 = piv0 = true;
-                        sm.stepof[t] = k;
-                    }
-                    if (ip1) {
-                        s1 = make_float2(0.f, 0.f);
-                        sc1 = pinv;
-                        used1 = piv1 = true;
-                        sm.stepof[g1] = k;
-                    }
+                    s0 = make_float2(ip0 ? 0.f : s0.x, ip0 ? 0.f : s0.y);
+                    s1 = make_float2(ip1 ? 0.f : s1.x, ip1 ? 0.f : s1.y);
+                    sc0 = make_float2(ip0 ? pinv.x : sc0.x, ip0 ? pinv.y : sc0.y);
+                    sc1 = make_float2(ip1 ? pinv.x : sc1.x, ip1 ? pinv.y : sc1.y);
+                    used0 |= ip0;
+                    used1 |= ip1;
+                    piv0 |= ip0;
+                    piv1 |= ip1;
+                    st_shared_u32_if(ip0 || ip1, smem_u32(&sm.stepof[r >= 0 ? r : 0]), (uint32_t)k);
                     P0[0] = cfms(s0, prow[0], P0[1]);
                     P1[0] = cfms(s1, prow[0], P1[1]);
                     key0 = f2_key(P0[0], !used0, t);
@@ -468,6 +462,7 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                     P0[kF2B - 1] = ip0 ? make_float2(1.f, 0.f) : make_float2(-s0.x, -s0.y);
                     P1[kF2B - 1] = ip1 ? make_float2(1.f, 0.f) : make_float2(-s1.x, -s1.y);
                 }
+                if (bad && t == 0 && rank == 0) atomicOr(a.status, 1);
                 // the panel's pivot rows scaled by their 1 / pv
                 if (piv0) {
 #pragma unroll

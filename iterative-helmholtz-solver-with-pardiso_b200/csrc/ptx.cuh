@@ -193,6 +193,21 @@ __device__ __forceinline__ void mbar_arrive_warp_cluster(uint32_t cluster_addr) 
         "r"((uint32_t)(threadIdx.x & 31))
         : "memory");
 }
+// 16 bytes to shared memory where p, as a predicated store: a branch around a
+// few stores costs the warp its reconvergence
+__device__ __forceinline__ void st_shared_v4_if(bool p, uint32_t addr, float4 v) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t"
+        "@q st.shared.v4.f32 [%1], {%2, %3, %4, %5};\n\t}" ::"r"((uint32_t)p),
+        "r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+        : "memory");
+}
+__device__ __forceinline__ void st_shared_u32_if(bool p, uint32_t addr, uint32_t v) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q st.shared.u32 [%1], %2;\n\t}" ::"r"((uint32_t)p),
+                 "r"(addr), "r"(v)
+                 : "memory");
+}
+
 // this thread's warp in its (1-D) block, in a form the compiler knows to be warp-uniform
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 
