@@ -121,3 +121,9 @@ __device__ __forceinline__ float2 pivot_inv(float2 pv) {
     const float rd = s * r;
     return make_float2(ax * rd, -ay * rd);
 }
+// the same, (0, 0) for an exactly zero pivot
+__device__ __forceinline__ float2 pivot_inv0(float2 pv) {
+    const float2 p = pivot_inv(pv);
+    const bool z = pv.x == 0.f && pv.y == 0.f;
+    return make_float2(z ? 0.f : p.x, z ? 0.f : p.y);
+}

@@ -387,54 +387,46 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                 uint32_t key1 = f2_key(P1[0], has1 && !used1, g1);
                 uint32_t key = key0 > key1 ? key0 : key1;
                 uint32_t kw = __reduce_max_sync(0xffffffffu, key);
+                // every row's 1 / candidate, under the reduction's latency: the
+                // winner's goes out with its row, so that no reciprocal stands
+                // between the barrier and the next pivot column
+                float2 inv0 = pivot_inv0(P0[0]), inv1 = pivot_inv0(P1[0]);
 #pragma unroll 1
                 for (int kk = 0; kk < bl; kk++) {
                     const int k = k0 + kk, buf = k & 1;
                     st_shared_u32_if(lane == 0, smem_u32(&sm.wkey[buf * kF2RowWarps + warp]), kw);
                     {
-                        // the winning row in register order: w[0] the pivot, w[1 + e] = prow[e]
+                        // the winning row in register order, w[1 + e] = prow[e], with
+                        // 1 / pivot in the pivot's place
                         const bool win = kw != 0u && key == kw, first = key0 == kw;
                         const uint32_t w = smem_u32(sm.wrow + (size_t)(buf * kF2RowWarps + warp) * kF2B);
+                        const float2 h0 = make_float2(first ? inv0.x : inv1.x, first ? inv0.y : inv1.y);
 #pragma unroll
                         for (int e = 0; e < kF2B / 2; e++)
                             st_shared_v4_if(win, w + 16u * (uint32_t)e,
-                                            make_float4(first ? P0[2 * e].x : P1[2 * e].x, first ? P0[2 * e].y : P1[2 * e].y,
+                                            make_float4(e == 0 ? h0.x : first ? P0[2 * e].x : P1[2 * e].x,
+                                                        e == 0 ? h0.y : first ? P0[2 * e].y : P1[2 * e].y,
                                                         first ? P0[2 * e + 1].x : P1[2 * e + 1].x,
                                                         first ? P0[2 * e + 1].y : P1[2 * e + 1].y));
                     }
                     f2_row_barrier();
                     const uint4 kv = *reinterpret_cast<const uint4 *>(sm.wkey + buf * kF2RowWarps);
-                    uint32_t kmax = kv.x;
-                    int wsel = 0;
-                    if (kv.y > kmax) {
-                        kmax = kv.y;
-                        wsel = 1;
-                    }
-                    if (kv.z > kmax) {
-                        kmax = kv.z;
-                        wsel = 2;
-                    }
-                    if (kv.w > kmax) {
-                        kmax = kv.w;
-                        wsel = 3;
-                    }
+                    const uint32_t kmax = max(max(kv.x, kv.y), max(kv.z, kv.w));
                     const int r = kmax != 0u ? 255 - (int)(kmax & 0xFFu) : -1;
+                    const int wsel = (r & (kF2RowThreads - 1)) >> 5;   // the warp that holds row r
                     // the pivot row, rotated like the rows: prow[e] = column (kk + 1 + e) mod 16
                     const float4 *w = reinterpret_cast<const float4 *>(sm.wrow + (size_t)(buf * kF2RowWarps + wsel) * kF2B);
-                    float2 prow[kF2B], pv = make_float2(0.f, 0.f);
+                    float2 prow[kF2B], pinv = make_float2(0.f, 0.f);
 #pragma unroll
                     for (int e = 0; e < kF2B / 2; e++) {
                         const float4 q4 = w[e];
-                        if (e == 0) pv = make_float2(q4.x, q4.y);
+                        if (e == 0) pinv = make_float2(r < 0 ? 0.f : q4.x, r < 0 ? 0.f : q4.y);
                         else prow[2 * e - 1] = make_float2(q4.x, q4.y);
                         prow[2 * e] = make_float2(q4.z, q4.w);
                     }
                     // no finite candidate, or an exactly zero pivot: flagged (after
                     // the panel), the block is invalid
-                    const bool none = r < 0 || (pv.x == 0.f && pv.y == 0.f);
-                    bad |= none;
-                    const float2 pi = pivot_inv(pv);
-                    const float2 pinv = make_float2(none ? 0.f : pi.x, none ? 0.f : pi.y);
+                    bad |= pinv.x == 0.f && pinv.y == 0.f;
                     st_shared_u32_if(t == 0, smem_u32(&sm.perm[k]), (uint32_t)(r >= 0 ? r : 0));
                     // row -= (c / pv) * pivot row, column k becomes -c / pv
                     const bool ip0 = t == r, ip1 = g1 == r;
@@ -454,6 +446,8 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                     key1 = f2_key(P1[0], has1 && !used1, g1);
                     key = key0 > key1 ? key0 : key1;
                     kw = __reduce_max_sync(0xffffffffu, key);
+                    inv0 = pivot_inv0(P0[0]);
+                    inv1 = pivot_inv0(P1[0]);
 #pragma unroll
                     for (int e = 1; e < kF2B - 1; e++) {
                         P0[e] = cfms(s0, prow[e], P0[e + 1]);
