@@ -122,6 +122,7 @@ struct SweepArgs {
     const void *cmy, *cpy;
     void *planes;             // PlaneLayout with R right-hand sides
     int R;
+    int rstride = 0;          // right-hand sides of the planes, where they hold more than this launch's (0: R)
     const void *dxy;          // null: S^{-1}; else S^{-H} with the [2][ny][n] alpha_x alpha_y table
     int *status;              // device flag: bit 2 = a bounded wait expired
     int stage_kb = 32;        // bulk-copy stage of G^T rows (KB, about)
@@ -150,7 +151,7 @@ int launch_kzskip_apply(bool c64, const SweepArgs &a, cudaStream_t s);
 // the CUDA-core kernel (0-5), the tensor-core kernel on the packed factor
 // planned for two CTAs per SM (6, 7) or one (8, 9), ring depths 8 and 4
 constexpr int kSweepVariants = 10;
-int sweep_default(bool c64, int n);   // the variant of an untuned batch
+int sweep_default(bool c64, int n, int R);   // the variant of an untuned batch
 // power-of-two scale of every complex64 block G_j for the FP16 products
 int launch_gscale(const void *Gt, int n, int ny, int nz, int ldg, float *gscale, cudaStream_t s);
 void sweep_variant(int v, SweepArgs &a);

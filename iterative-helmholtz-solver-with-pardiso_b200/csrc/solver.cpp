@@ -218,7 +218,7 @@ static SweepArgs sweep_args(helm3d_ctx *c, int R, bool adjoint) {
     // lines fit one row block is faster on the CUDA cores
     const int adj = adjoint ? 1 : 0, forced = tune_forced("SWEEP");
     const bool tuned = c->tv_sweep_R[adj] > 0 && (R == c->tv_sweep_R[adj] || R >= 3 || s.n > 128);
-    sweep_variant(forced >= 0 ? forced : tuned ? c->tv_sweep[adj] : sweep_default(c->c64, s.n), s);
+    sweep_variant(forced >= 0 ? forced : tuned ? c->tv_sweep[adj] : sweep_default(c->c64, s.n, R), s);
     return s;
 }
 

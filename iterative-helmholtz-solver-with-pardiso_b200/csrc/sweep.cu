@@ -36,6 +36,7 @@ namespace h3d {
 
 template <typename R> struct SweepK {
     int n, ny, ldg, nrhs;
+    int rstride;         // right-hand sides of the planes, nrhs of which from planes on are this launch's
     const cplx<R> *Gt;
     const cplx<R> *cmy, *cpy;
     cplx<R> *planes;
@@ -152,7 +153,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) sweep_kernel(SweepK<R> a) {
     typedef cplx<R> Cx;
     constexpr int RW = 32 / G;  // rows of y per warp
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    const int n = a.n, ldg = a.ldg, Rn = a.nrhs;
+    const int n = a.n, ldg = a.ldg, Rn = a.nrhs, Rs = a.rstride;
     const int kz = blockIdx.x >> 1;
     if (a.kzslot && a.kzslot[kz] >= 0) return;   // a skipped mode (kz_skip_ratio), in both CTAs
     const uint32_t rank = blockIdx.x & 1u, peer = rank ^ 1u;   // the rank in the cluster of two
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) sweep_kernel(SweepK<R> a) {
     uint64_t *empty = full + a.nstage;
     uint64_t *never = empty + a.nstage;         // no thread arrives on it
     uint64_t *met = never + 1, *read = never + 2;   // the peer's consumer warps arrive on them
-    Cx *P = a.planes + (long)kz * a.ny * Rn * n;  // line j, rhs r, row i at ((j*Rn + r)*n + i)
+    Cx *P = a.planes + (long)kz * a.ny * Rs * n;  // line j, rhs r, row i at ((j*Rs + r)*n + i)
     const int cpl = (n + a.rows_per_stage - 1) / a.rows_per_stage;
 
     if (threadIdx.x == 0) {
@@ -195,7 +196,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) sweep_kernel(SweepK<R> a) {
         }
         const Cx *cin = hc.half ? a.cpy : a.cmy, *cout = hc.half ? a.cmy : a.cpy;
         const int steps = hc.steps();
-        auto load_f = [&](int line, int r) { return adj_in<R, ADJ>(a, line, i, P[((long)line * Rn + r) * n + i]); };
+        auto load_f = [&](int line, int r) { return adj_in<R, ADJ>(a, line, i, P[((long)line * Rs + r) * n + i]); };
         // the middle line's input from its right-hand side f, this half's y and the peer's
         auto meet = [&](Cx (&v)[RR], const Cx (&y)[RR], const Cx (&f)[RR]) {
             sweep_arrive_peer(met, peer);
@@ -207,7 +208,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) sweep_kernel(SweepK<R> a) {
 #pragma unroll
             for (int r = 0; r < RR; r++) {
                 o[r] = mkc<R>(0, 0);
-                if (fin && r < Rn && hc.peer_lines()) o[r] = P[((long)hc.peer_last() * Rn + r) * n + i];
+                if (fin && r < Rn && hc.peer_lines()) o[r] = P[((long)hc.peer_last() * Rs + r) * n + i];
             }
             const Cx cm = a.cmy[hc.mid], cp = a.cpy[hc.mid];
 #pragma unroll
@@ -237,8 +238,8 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) sweep_kernel(SweepK<R> a) {
         RingPos rp;
         // this thread's element of the plane's line (r = 0), and the step
         // from one line to the next in the half's order
-        Cx *Pl = P + (long)hc.line(0) * Rn * n + i;
-        const long lstep = hc.half ? -(long)Rn * n : (long)Rn * n;
+        Cx *Pl = P + (long)hc.line(0) * Rs * n + i;
+        const long lstep = hc.half ? -(long)Rs * n : (long)Rs * n;
         const int cstep = hc.half ? -1 : 1;
         const Cx *cptr = cin + hc.line(0);   // forward: cin of the line; backward: cout
         for (int t = 0; t < steps; t++) {
@@ -358,13 +359,260 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) sweep_kernel(SweepK<R> a) {
     cluster_sync_all();   // no CTA leaves while the peer may arrive on its barriers
 }
 
-template <typename R, int G, int RR, bool ADJ, int CW> static int sweep_impl(const SweepArgs &sa, cudaStream_t st) {
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t p;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(lo), "f"(hi));
+    return p;
+}
+__device__ __forceinline__ void unpack2(uint64_t p, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p));
+}
+// two FP32 fused multiply-adds in one instruction
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+// Complex64 batches of RR >= 4, bound by the FP32 pipe and shared memory: a
+// thread owns two adjacent rows (one 16-byte load of G) for all RR right-hand
+// sides, so that a load of v feeds two products (one row per thread reads 34
+// cycles of shared memory per 64 warp FMAs; this reads at most 36 per 128), two
+// right-hand sides at a time in one instruction (fma2).  Lane il + RL g owns
+// rows 2 il, 2 il + 1 of the warp's and adds up the rows m = g, g + G, ... of
+// G^T; the G partial sums of a row meet by halving, which leaves each group g
+// the right-hand sides from g RR / G on to finish.  Everything else as in
+// sweep_kernel.  Sixteen sources, one row per thread -> this kernel: 32^3 84 ->
+// 50 us, 64^3 291 -> 197, 96^3 1425 -> 1032, 128^3 2461 -> 2030, 200 x 128 x 60
+// 3080 -> 2880; eight: 64^3 141 -> 122, 96^3 765 -> 567, 128^3 1409 -> 1120.
+// elements between the rows of v: the G rows that a warp reads at once lie in
+// banks of their own
+constexpr int kBatchPad = 2;
+
+template <int G, int RR, bool ADJ, int CW>
+__global__ void __launch_bounds__((CW + 1) * 32, 1) sweep_batch_kernel(SweepK<float> a) {
+    typedef float2 Cx;
+    constexpr int RL = 32 / G;                       // lanes along the rows
+    constexpr int VS = RR + kBatchPad;                       // row stride of v
+    constexpr int FS = RR >= G ? RR / G : 1;         // right-hand sides a thread finishes
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const int n = a.n, ldg = a.ldg, Rn = a.nrhs, Rs = a.rstride;
+    const int kz = blockIdx.x >> 1;
+    if (a.kzslot && a.kzslot[kz] >= 0) return;   // a skipped mode (kz_skip_ratio), in both CTAs
+    const uint32_t rank = blockIdx.x & 1u, peer = rank ^ 1u;   // the rank in the cluster of two
+    const HalfChain hc(a.ny, (int)rank);
+    const int lane = threadIdx.x & 31, warp = warp_index();
+    Cx *ring = reinterpret_cast<Cx *>(smem_raw);
+    Cx *vbuf = reinterpret_cast<Cx *>(smem_raw + (size_t)a.nstage * a.stage_bytes);  // [2][n][RR]
+    uint64_t *full = reinterpret_cast<uint64_t *>(vbuf + 2 * (size_t)n * VS);
+    uint64_t *empty = full + a.nstage;
+    uint64_t *never = empty + a.nstage;         // no thread arrives on it
+    uint64_t *met = never + 1, *read = never + 2;   // the peer's consumer warps arrive on them
+    Cx *P = a.planes + (long)kz * a.ny * Rs * n;  // line j, rhs r, row i at ((j*Rs + r)*n + i)
+    const int cpl = (n + a.rows_per_stage - 1) / a.rows_per_stage;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < a.nstage; s++) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], CW);
+        }
+        mbar_init(never, 1);
+        mbar_init(met, CW);
+        mbar_init(read, CW);
+        fence_mbar_init_cluster();
+    }
+    __syncthreads();
+    cluster_arrive();   // the peer's barriers exist before the first remote arrive (waited below)
+
+    if (warp == CW) {
+        cluster_wait();
+        if (lane == 0) sweep_produce(a, hc, kz, ring, full, empty, cpl);
+        __syncwarp();
+    } else {
+        const int il = lane % RL, g = lane / RL;
+        const int i = (warp * RL + il) * 2;
+        const bool own = i < n;                      // (row i + 1 may be past n: ldg covers its loads)
+        const int r0s = g * RR / G;                  // the first right-hand side this thread finishes
+        const bool owner = own && (RR >= G || g % (G / RR) == 0);
+        bool dead = false;
+        if (a.expire_test && !mbar_wait_warp_cta(smem_u32(never), 0u, a.wait_limit)) {
+            dead = true;
+            if (lane == 0) atomicOr(a.status, 4);
+        }
+        const Cx *cin = hc.half ? a.cpy : a.cmy, *cout = hc.half ? a.cmy : a.cpy;
+        const int steps = hc.steps();
+        // element q of this thread's tile: row i + (q & 1), right-hand side r0s + (q >> 1)
+        auto in = [&](int q) { return owner && i + (q & 1) < n && r0s + (q >> 1) < Rn; };
+        auto at = [&](int line, int q) -> Cx & { return P[((long)line * Rs + r0s + (q >> 1)) * n + i + (q & 1)]; };
+        auto meet = [&](Cx (&v)[2 * FS], const Cx (&f)[2 * FS]) {   // v: this half's y on entry
+            sweep_arrive_peer(met, peer);
+            if (!dead && !mbar_wait_warp_cluster(smem_u32(met), 0u, a.wait_limit)) {
+                dead = true;
+                if (lane == 0) atomicOr(a.status, 4);
+            }
+            const Cx cm = a.cmy[hc.mid], cp = a.cpy[hc.mid];
+#pragma unroll
+            for (int q = 0; q < 2 * FS; q++) {
+                const Cx o = in(q) && hc.peer_lines() ? at(hc.peer_last(), q) : make_float2(0, 0);
+                v[q] = hc.half ? cfms(cp, v[q], cfms(cm, o, f[q])) : cfms(cp, o, cfms(cm, v[q], f[q]));
+            }
+            sweep_arrive_peer(read, peer);
+        };
+        // v of a row: (x, x, y, y) of each pair of right-hand sides
+        auto put = [&](Cx *vb, const Cx (&v)[2 * FS]) {
+            if (!owner) return;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                if (i + h >= n) continue;
+                float *row = reinterpret_cast<float *>(vb + (i + h) * VS);
+                if constexpr (FS == 1) {
+                    row[(r0s >> 1) * 4 + (r0s & 1)] = in(h) ? v[h].x : 0;
+                    row[(r0s >> 1) * 4 + (r0s & 1) + 2] = in(h) ? v[h].y : 0;
+                } else {
+#pragma unroll
+                    for (int f = 0; f < FS; f += 2) {
+                        const Cx v0 = v[2 * f + h], v1 = v[2 * f + 2 + h];
+                        const bool in0 = in(2 * f + h), in1 = in(2 * f + 2 + h);
+                        reinterpret_cast<float4 *>(row)[(r0s + f) >> 1] =
+                            make_float4(in0 ? v0.x : 0, in1 ? v1.x : 0, in0 ? v0.y : 0, in1 ? v1.y : 0);
+                    }
+                }
+            }
+        };
+        cluster_wait();
+        {   // the first line's input
+            Cx v[2 * FS], f[2 * FS];
+#pragma unroll
+            for (int q = 0; q < 2 * FS; q++) {
+                f[q] = in(q) ? adj_in<float, ADJ>(a, hc.line(0), i + (q & 1), at(hc.line(0), q)) : make_float2(0, 0);
+                v[q] = make_float2(0, 0);
+            }
+            if (hc.K == 0) {
+                meet(v, f);
+                put(vbuf, v);
+            } else {
+                put(vbuf, f);
+            }
+        }
+        consumer_barrier<CW>();
+        RingPos rp;
+        for (int t = 0; t < steps; t++) {
+            const int line = hc.step_line(t);
+            const bool fwd = t <= hc.K;
+            const Cx *v = vbuf + (t & 1) * n * VS;
+            Cx *vnext = vbuf + ((t + 1) & 1) * n * VS;
+            // prefetch: the next line's right-hand side (forward) or this line's y (backward)
+            Cx pre[2 * FS];
+#pragma unroll
+            for (int q = 0; q < 2 * FS; q++)
+                pre[q] = in(q) && t != hc.K ? at(t < hc.K ? hc.line(t + 1) : line, q) : make_float2(0, 0);
+            const Cx cc = t + 1 < hc.K ? cin[hc.line(t + 1)] : !fwd ? cout[line] : make_float2(0, 0);
+            uint64_t ax[2][RR / 2], ay[2][RR / 2];   // real and imaginary parts of right-hand sides 2 r, 2 r + 1
+#pragma unroll
+            for (int r = 0; r < RR / 2; r++) ax[0][r] = ax[1][r] = ay[0][r] = ay[1][r] = 0;
+            for (int ch = 0; ch < cpl; ch++) {
+                if (!dead && !mbar_wait_warp_cta(smem_u32(&full[rp.slot]), rp.phase, a.wait_limit)) {
+                    dead = true;
+                    if (lane == 0) atomicOr(a.status, 4);
+                }
+                const int r0 = ch * a.rows_per_stage;
+                const int rows = min(a.rows_per_stage, n - r0);
+                if (own) {
+                    const Cx *st = ring + (size_t)rp.slot * (a.stage_bytes / sizeof(Cx)) + g * ldg + i;
+                    const Cx *vm = v + (r0 + g) * VS;
+#pragma unroll 2
+                    for (int ml = g; ml < rows; ml += G, st += G * ldg, vm += G * VS) {
+                        const float4 gv = *reinterpret_cast<const float4 *>(st);
+                        const uint64_t gx0 = pack2(gv.x, gv.x), gy0 = pack2(gv.y, gv.y), hy0 = pack2(-gv.y, -gv.y);
+                        const uint64_t gx1 = pack2(gv.z, gv.z), gy1 = pack2(gv.w, gv.w), hy1 = pack2(-gv.w, -gv.w);
+#pragma unroll
+                        for (int r = 0; r < RR / 2; r++) {
+                            const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(vm + 2 * r);
+                            ax[0][r] = fma2(hy0, w.y, fma2(gx0, w.x, ax[0][r]));
+                            ay[0][r] = fma2(gy0, w.x, fma2(gx0, w.y, ay[0][r]));
+                            ax[1][r] = fma2(hy1, w.y, fma2(gx1, w.x, ax[1][r]));
+                            ay[1][r] = fma2(gy1, w.x, fma2(gx1, w.y, ay[1][r]));
+                        }
+                    }
+                }
+                mbar_arrive_warp(&empty[rp.slot]);
+                rp.next(a.nstage);
+            }
+            Cx acc[2][RR];
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+#pragma unroll
+                for (int r = 0; r < RR / 2; r++) {
+                    unpack2(ax[h][r], acc[h][2 * r].x, acc[h][2 * r + 1].x);
+                    unpack2(ay[h][r], acc[h][2 * r].y, acc[h][2 * r + 1].y);
+                }
+            // the G partial sums: the group bit of each step keeps its half of
+            // the right-hand sides (one left: plain sums)
+#pragma unroll
+            for (int s = G / 2, cnt = RR; s >= 1; s >>= 1) {
+                const bool hi = (g & s) != 0;
+                if (cnt > 1) {
+                    cnt >>= 1;
+#pragma unroll
+                    for (int r = 0; r < RR / 2; r++)
+                        if (r < cnt) {
+#pragma unroll
+                            for (int h = 0; h < 2; h++) {
+                                const Cx lo = acc[h][r], up = acc[h][r + cnt];
+                                const Cx send = hi ? lo : up;
+                                Cx keep = hi ? up : lo;
+                                keep.x += __shfl_xor_sync(0xffffffffu, send.x, RL * s);
+                                keep.y += __shfl_xor_sync(0xffffffffu, send.y, RL * s);
+                                acc[h][r] = keep;
+                            }
+                        }
+                } else {
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        acc[h][0].x += __shfl_xor_sync(0xffffffffu, acc[h][0].x, RL * s);
+                        acc[h][0].y += __shfl_xor_sync(0xffffffffu, acc[h][0].y, RL * s);
+                    }
+                }
+            }
+            // the peer has read this half's last y before it is overwritten
+            if (t == hc.K + 1 && !dead && !mbar_wait_warp_cluster(smem_u32(read), 0u, a.wait_limit)) {
+                dead = true;
+                if (lane == 0) atomicOr(a.status, 4);
+            }
+            if (ADJ && t < hc.K) {
+#pragma unroll
+                for (int q = 0; q < 2 * FS; q++)
+                    if (in(q)) pre[q] = adj_in<float, ADJ>(a, hc.line(t + 1), i + (q & 1), pre[q]);
+            }
+            Cx vn[2 * FS];
+#pragma unroll
+            for (int q = 0; q < 2 * FS; q++) {
+                const Cx sum = acc[q & 1][q >> 1];
+                const Cx out = fwd ? sum : cfms(cc, sum, pre[q]);   // y, x_mid, or x = y - cout G x_next
+                vn[q] = t + 1 < hc.K ? cfms(cc, out, pre[q]) : out;
+                if (in(q) && (t != hc.K || hc.half == 0))
+                    at(line, q) = t >= hc.K ? adj_out<float, ADJ>(a, line, i + (q & 1), out) : out;
+            }
+            if (t == hc.K - 1) meet(vn, pre);
+            put(vnext, vn);
+            consumer_barrier<CW>();
+        }
+        __syncwarp();
+    }
+    cluster_sync_all();   // no CTA leaves while the peer may arrive on its barriers
+}
+
+// A launch of kern: CW consumer warps, rows of v of vs elements; even > 0: the
+// stages of a line are the same multiple of that many rows.
+template <typename R, int CW>
+static int sweep_go(void (*kern)(SweepK<R>), int vs, int even, const SweepArgs &sa, cudaStream_t st) {
     typedef cplx<R> Cx;
     SweepK<R> k;
     k.n = sa.n;
     k.ny = sa.ny;
     k.ldg = sa.ldg;
     k.nrhs = sa.R;
+    k.rstride = sa.rstride ? sa.rstride : sa.R;
     k.Gt = (const Cx *)sa.Gt;
     k.cmy = (const Cx *)sa.cmy;
     k.cpy = (const Cx *)sa.cpy;
@@ -377,24 +625,43 @@ template <typename R, int G, int RR, bool ADJ, int CW> static int sweep_impl(con
         const char *e = std::getenv("HELM3D_TEST_EXPIRE_WAIT");
         k.expire_test = (e && *e && *e != '0') ? 1 : 0;
     }
-    const size_t vbytes = sizeof(Cx) * 2 * (size_t)sa.n * RR;
+    const size_t vbytes = sizeof(Cx) * 2 * (size_t)sa.n * vs;
     const size_t budget = device_info().smem_optin - vbytes - 1024;
-    // stages of about stage_kb, as many as fit the rest of shared memory
-    // (at most ring_kb)
+    // stages of about stage_kb (two at least fit), as many as fit the rest of
+    // shared memory (at most ring_kb)
     const size_t row_bytes = (size_t)sa.ldg * sizeof(Cx);
-    int rows = (int)(((size_t)sa.stage_kb * 1024) / row_bytes);
+    const size_t ring_max = (size_t)sa.ring_kb * 1024;
+    const size_t ring_cap = budget < ring_max ? budget : ring_max;
+    size_t stage = (size_t)sa.stage_kb * 1024;
+    if (stage > ring_cap / 2 - 128) stage = ring_cap / 2 - 128;
+    int rows = (int)(stage / row_bytes);
     if (rows < 1) rows = 1;
-    if (rows > sa.n) rows = sa.n;
+    if (even) {   // equal stages of a line, so that no group of lanes has more rows than another
+        rows = rows < even ? even : rows / even * even;
+        const int cpl = (sa.n + rows - 1) / rows, per = (sa.n + cpl - 1) / cpl;
+        rows = (per + even - 1) / even * even;
+    } else if (rows > sa.n) {
+        rows = sa.n;
+    }
     k.rows_per_stage = rows;
     k.stage_bytes = (uint32_t)(((size_t)rows * row_bytes + 127) & ~(size_t)127);
-    const size_t ring_max = (size_t)sa.ring_kb * 1024;
-    size_t ring_cap = budget < ring_max ? budget : ring_max;
     int nst = (int)(ring_cap / k.stage_bytes);
     if (nst > 32) nst = 32;
     if (nst < 2) return HELM3D_ERR_ARG;
     k.nstage = nst;
     const size_t smem = (size_t)nst * k.stage_bytes + vbytes + (2 * nst + 3) * sizeof(uint64_t);
-    return launch_pairs(sweep_kernel<R, G, RR, ADJ, CW>, sa.nz, (CW + 1) * 32, smem, k, st);
+    return launch_pairs(kern, sa.nz, (CW + 1) * 32, smem, k, st);
+}
+
+template <typename R, int G, int RR, bool ADJ, int CW> static int sweep_impl(const SweepArgs &sa, cudaStream_t st) {
+    return sweep_go<R, CW>(sweep_kernel<R, G, RR, ADJ, CW>, RR, 0, sa, st);
+}
+
+// complex64 batches: 64 / G rows per warp
+template <int G, bool ADJ, int CW> static int sweep_batch(const SweepArgs &sa, cudaStream_t st) {
+    if (sa.R <= 4) return sweep_go<float, CW>(sweep_batch_kernel<G, 4, ADJ, CW>, 4 + kBatchPad, G, sa, st);
+    if (sa.R <= 8) return sweep_go<float, CW>(sweep_batch_kernel<G, 8, ADJ, CW>, 8 + kBatchPad, G, sa, st);
+    return sweep_go<float, CW>(sweep_batch_kernel<G, 16, ADJ, CW>, 16 + kBatchPad, G, sa, st);
 }
 
 // The split of a line over the consumer warps: 32 / G rows per warp, CW warps.
@@ -403,12 +670,41 @@ template <typename R, int G, int RR, bool ADJ, int CW> static int sweep_impl(con
 template <typename R, bool ADJ, int G1, int CW1, int G2> static int sweep_rr(const SweepArgs &sa, cudaStream_t s) {
     if (sa.R <= 1) return sweep_impl<R, G1, 1, ADJ, CW1>(sa, s);
     if (sa.R <= 2) return sweep_impl<R, G1, 2, ADJ, CW1>(sa, s);
-    if (sa.R <= 4) return sweep_impl<R, G2, 4, ADJ, 8>(sa, s);
-    if (sa.R <= 8) return sweep_impl<R, G2, 8, ADJ, 8>(sa, s);
-    return sweep_impl<R, G2, 16, ADJ, 8>(sa, s);
+    if constexpr (sizeof(R) == 8 || G2 == 4)
+        if (sa.R <= 4) return sweep_impl<R, G2, 4, ADJ, 8>(sa, s);
+    if constexpr (sizeof(R) == 8) {
+        if (sa.R <= 8) return sweep_impl<R, G2, 8, ADJ, 8>(sa, s);
+        // sums of 16 right-hand sides do not fit the registers (spilled, 64^3:
+        // 957 us; two launches 2 x 269, although they read G twice)
+        SweepArgs h = sa;
+        h.rstride = sa.R;
+        h.R = 8;
+        const int rc = sweep_impl<R, G2, 8, ADJ, 8>(h, s);
+        if (rc) return rc;
+        h.R = sa.R - 8;
+        h.planes = (cplx<R> *)sa.planes + 8 * (long)sa.n;
+        return sweep_rr<R, ADJ, G1, CW1, G2>(h, s);
+    }
+    return HELM3D_ERR_ARG;   // (complex64 batches are sweep_batch's)
 }
 
 template <typename R, bool ADJ> static int sweep_n(const SweepArgs &sa, cudaStream_t s) {
+    if constexpr (sizeof(R) == 4) {
+        // (three or four sources of up to 64 rows: 88 us by sweep_kernel at 64^3,
+        // 93 by this.)  Warps of 8 or 16 rows by whichever leaves the four
+        // schedulers of an SM the same number: 96 rows as 12 warps of 8 rows,
+        // 16 sources, 1075 us, as 6 of 16 rows 1290; 160 rows (x 128 x 60) as
+        // 10 of 16 1980, as 5 of 32 2550; 200 rows as 13 2873, as 7 2922
+        if (sa.R > 4 || (sa.R > 2 && sa.n > 64)) {
+            if (sa.n <= 32) return sweep_batch<8, ADJ, 4>(sa, s);
+            if (sa.n <= 64) return sweep_batch<8, ADJ, 8>(sa, s);
+            if (sa.n <= 96) return sweep_batch<8, ADJ, 12>(sa, s);
+            if (sa.n <= 128) return sweep_batch<4, ADJ, 8>(sa, s);
+            if (sa.n <= 192) return sweep_batch<4, ADJ, 12>(sa, s);
+            if (sa.n <= 240) return sweep_batch<4, ADJ, 15>(sa, s);
+            return sweep_batch<2, ADJ, 8>(sa, s);
+        }
+    }
     if (sa.n <= 32) return sweep_rr<R, ADJ, 8, 8, 4>(sa, s);
     // complex64: 16 rows of a warp make 128 bytes, one shared-memory wavefront
     if (sa.n <= 64) return sweep_rr<R, ADJ, sizeof(R) == 4 ? 2 : 4, sizeof(R) == 4 ? 4 : 8, 4>(sa, s);
@@ -417,7 +713,7 @@ template <typename R, bool ADJ> static int sweep_n(const SweepArgs &sa, cudaStre
 }
 
 void sweep_variant(int v, SweepArgs &a) {
-    static const int kStage[kSweepVariants] = {32, 16, 64, 8, 32, 16, 0, 0, 0, 0};
+    static const int kStage[kSweepVariants] = {32, 16, 64, 96, 32, 16, 0, 0, 0, 0};
     static const int kRingKb[kSweepVariants] = {200, 200, 200, 200, 100, 100, 0, 0, 0, 0};
     static const int kTcOcc[kSweepVariants] = {0, 0, 0, 0, 0, 0, 2, 2, 1, 1};
     static const int kTcStages[kSweepVariants] = {0, 0, 0, 0, 0, 0, 8, 4, 4, 8};
@@ -432,10 +728,17 @@ void sweep_variant(int v, SweepArgs &a) {
 // the CUDA-core kernel, whose products are FP32 (the tensor cores' FP16 hi/lo
 // products add about a fifth to the complex64 preconditioner's error, 3.1e-6
 // -> 3.8e-6 at 96^3, which a solve corrects and a caller's single apply does
-// not), by stages of 64 KB where a line is longer than 32 KB (one source,
-// 112 x 112 x 64: 287 -> 225 us, 128^3: 745 -> 658; below, a line is one
-// stage either way).
-int sweep_default(bool c64, int n) { return (size_t)n * n * (c64 ? 8 : 16) > 32 * 1024 ? 2 : 0; }
+// not).  A stage's first products wait for its first loads, so stages are
+// large: complex64 by 96 KB where that holds a line or for several sources
+// (96^3 against 64 KB: one source 312 -> 295 us, 16 sources 1074 -> 1032), by
+// 64 KB for one or two of longer lines (128^3 with 96 KB 723 us, 64 KB 657)
+// and for complex128 (one source, 128^3: 1286 us by 32 KB, 1248).  Below
+// 32 KB a line is one stage either way.
+int sweep_default(bool c64, int n, int R) {
+    const size_t line = (size_t)n * n * (c64 ? 8 : 16);
+    if (line <= 32 * 1024) return 0;
+    return c64 && (R > 2 || line <= 96 * 1024) ? 3 : 2;
+}
 
 static int launch_sweep_kernels(bool c64, const SweepArgs &sa, cudaStream_t s);
 
