@@ -73,7 +73,7 @@ namespace h3d {
 
 constexpr int kF2RowWarps = 4;
 constexpr int kF2RowThreads = kF2RowWarps * 32;
-constexpr int kF2Threads = (kF2RowWarps + 1) * 32;
+constexpr int kF2Threads = 2 * kF2RowThreads;   // the row warps and as many helpers
 constexpr int kF2B = 16;                         // panel width
 constexpr int kF2MaxN = 224;                     // 2 ncol + 64 X columns <= 512
 constexpr int kF2Tab = 256;
@@ -90,13 +90,14 @@ struct F2K {
 
 struct F2Smem {
     float *Bhi, *Blo;   // [2 kF2MaxN rows][2 kF2B] canonical K-major each
-    float2 *Y;          // [kF2B][kF2Yld]: the panel's pivot rows
+    float2 *Y;          // [kF2B][kF2Yld]: the panel's pivot rows (the helpers')
+    float2 *Yn;         // [kF2B][kF2PFld]: their entries in the next panel's columns (the row warps')
     float2 *PF;         // [kF2MaxN][kF2PFld]: the panel's entries of every row
     float2 *wrow;       // [2][kF2RowWarps][kF2B]: each warp's candidate row, by step parity
     uint32_t *wkey;     // [2][kF2RowWarps]
     int *rho, *kap;     // [2][kF2Tab] each: the frame, double-buffered by line
     int *kapinv, *perm, *stepof;   // [kF2Tab]; stepof[g]: the step that pivoted row g
-    uint64_t *pan_bar, *y_bar, *b_ready, *next_ready, *rest_done, *fin;
+    uint64_t *pan_bar, *yn_bar, *bn_ready, *x_ready, *y_bar, *y_free, *next_ready, *rest_done, *fin;
     uint32_t *tslot;
 };
 
@@ -107,9 +108,9 @@ constexpr int kF2PFld = kF2B + 2;
 // row stride of Y: 226 complex, so that the B build's reads of four pivot
 // rows at the same column fall on distinct banks (16-byte aligned rows)
 constexpr int kF2Yld = kF2MaxN + 2;
-constexpr size_t kF2SmemBytes = 2 * kF2BBytes + sizeof(float2) * (kF2B * kF2Yld + kF2PFld * kF2MaxN) +
+constexpr size_t kF2SmemBytes = 2 * kF2BBytes + sizeof(float2) * (kF2B * kF2Yld + kF2B * kF2PFld + kF2PFld * kF2MaxN) +
                                 sizeof(float2) * 2 * kF2RowWarps * kF2B + sizeof(uint32_t) * 2 * kF2RowWarps +
-                                sizeof(int) * 7 * kF2Tab + 6 * sizeof(uint64_t) + 16 + 1024 + 16;
+                                sizeof(int) * 7 * kF2Tab + 9 * sizeof(uint64_t) + 16 + 1024 + 16;
 
 __device__ __forceinline__ F2Smem f2_carve(unsigned char *raw) {
     F2Smem s;
@@ -117,7 +118,8 @@ __device__ __forceinline__ F2Smem f2_carve(unsigned char *raw) {
     s.Bhi = reinterpret_cast<float *>(b);
     s.Blo = s.Bhi + 2 * kF2MaxN * 2 * kF2B;
     s.Y = reinterpret_cast<float2 *>(s.Blo + 2 * kF2MaxN * 2 * kF2B);
-    s.PF = s.Y + kF2B * kF2Yld;
+    s.Yn = s.Y + kF2B * kF2Yld;
+    s.PF = s.Yn + kF2B * kF2PFld;
     s.wrow = s.PF + kF2MaxN * kF2PFld;
     s.wkey = reinterpret_cast<uint32_t *>(s.wrow + 2 * kF2RowWarps * kF2B);
     s.rho = reinterpret_cast<int *>(s.wkey + 2 * kF2RowWarps);
@@ -128,18 +130,26 @@ __device__ __forceinline__ F2Smem f2_carve(unsigned char *raw) {
     uintptr_t m = reinterpret_cast<uintptr_t>(s.stepof + kF2Tab);
     m = (m + 15) & ~uintptr_t(15);
     s.pan_bar = reinterpret_cast<uint64_t *>(m);
-    s.y_bar = s.pan_bar + 1;
-    s.b_ready = s.pan_bar + 2;
-    s.next_ready = s.pan_bar + 3;
-    s.rest_done = s.pan_bar + 4;
-    s.fin = s.pan_bar + 5;
-    s.tslot = reinterpret_cast<uint32_t *>(s.pan_bar + 6);
+    s.yn_bar = s.pan_bar + 1;
+    s.bn_ready = s.pan_bar + 2;
+    s.x_ready = s.pan_bar + 3;
+    s.y_bar = s.pan_bar + 4;
+    s.y_free = s.pan_bar + 5;
+    s.next_ready = s.pan_bar + 6;
+    s.rest_done = s.pan_bar + 7;
+    s.fin = s.pan_bar + 8;
+    s.tslot = reinterpret_cast<uint32_t *>(s.pan_bar + 9);
     return s;
 }
 
 __device__ __forceinline__ void f2_row_barrier() {
     asm volatile("bar.sync 1, %0;" ::"n"(kF2RowThreads) : "memory");
 }
+
+__device__ __forceinline__ void f2_helper_barrier() {
+    asm volatile("bar.sync 2, %0;" ::"n"(kF2Threads - kF2RowThreads) : "memory");
+}
+__device__ __forceinline__ void f2_all_barrier() { asm volatile("bar.sync 3, %0;" ::"n"(kF2Threads) : "memory"); }
 
 __device__ __forceinline__ void st_cluster_v4f32(uint32_t addr, float4 v) {
     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z),
@@ -169,6 +179,64 @@ __device__ __forceinline__ uint32_t f2_key(float2 v, bool cand, int g) {
     const float av = fabsf(v.x) + fabsf(v.y);
     if (!(av == av)) return 0u;
     return (__float_as_uint(av) & 0xFFFFFF00u) | (uint32_t)(255 - g);
+}
+
+// Unit v of the real form of Y (rows 2j + c, K = 2kk + c'), hi and lo, from the
+// pivot rows' entries y0, y1 in column j = (v >> 5) * 4 + (v & 3), K quad
+// kq = (v >> 2) & 7: the 16-byte units of rows 2j, (Re y, -Im y), and 2j + 1,
+// (Im y, Re y), adjacent in address order (row & 7, K quad, 8-row group); the
+// TF32 split is odd in its argument, so one split serves both rows.
+__device__ __forceinline__ void f2_put_b(const F2Smem &sm, int v, float2 y0, float2 y1) {
+    float4 h, l;   // split of (Re y0, Im y0, Re y1, Im y1)
+    tf32_split_fast(y0.x, h.x, l.x);
+    tf32_split_fast(y0.y, h.y, l.y);
+    tf32_split_fast(y1.x, h.z, l.z);
+    tf32_split_fast(y1.y, h.w, l.w);
+    const int u0 = (v >> 5) * 64 + ((v >> 2) & 7) * 8 + 2 * (v & 3);
+    float4 *bh = reinterpret_cast<float4 *>(sm.Bhi) + u0;
+    float4 *bl = reinterpret_cast<float4 *>(sm.Blo) + u0;
+    bh[0] = make_float4(h.x, -h.y, h.z, -h.w);
+    bh[1] = make_float4(h.y, h.x, h.w, h.z);
+    bl[0] = make_float4(l.x, -l.y, l.z, -l.w);
+    bl[1] = make_float4(l.y, l.x, l.w, l.z);
+}
+
+// G_line^T to global memory in the frame (kap, i = rho of the thread's row),
+// and, with more, the next line's S in place: the 16-column chunks c = which,
+// which + 2, ... of this thread's TMEM lane.
+__device__ __forceinline__ void f2_line_out(const F2K &a, const F2Smem &sm, uint32_t trow, bool valid, int i,
+                                            const int *kap, float2 *gout, int ncol, int which, bool more, int nl,
+                                            float2 cc, float2 kzv) {
+    const int n = a.n;
+    F2Drow d = {};
+    int qd = -1, qs = -1, qp = -1;
+    if (more && valid) {
+        d = f2_drow(a, nl, i, kzv);
+        qd = sm.kapinv[i];
+        qs = i > 0 ? sm.kapinv[i - 1] : -1;
+        qp = i + 1 < n ? sm.kapinv[i + 1] : -1;
+    }
+#pragma unroll 1
+    for (int c = which; c < ncol / 16; c += 2) {
+        float f[32];
+        tmem_ld32_nowait(trow + (uint32_t)(32 * c), f);
+        int kq[16];
+#pragma unroll
+        for (int e = 0; e < 4; e++) *reinterpret_cast<int4 *>(kq + 4 * e) = reinterpret_cast<const int4 *>(kap + 16 * c)[e];
+        tmem_wait_ld(f);
+#pragma unroll
+        for (int e = 0; e < 16; e++) {   // (selects: a branch per entry costs more than the entry)
+            const int q = 16 * c + e;
+            const float2 m = make_float2(f[2 * e], f[2 * e + 1]);
+            st_global_f2_if(valid && q < n, gout + (unsigned)(kq[e] * a.ldg + i), m);
+            const float2 dd = make_float2(q == qd ? d.diag.x : q == qs ? d.sub.x : q == qp ? d.sup.x : 0.f,
+                                          q == qd ? d.diag.y : q == qs ? d.sub.y : q == qp ? d.sup.y : 0.f);
+            f[2 * e] = dd.x - (cc.x * m.x - cc.y * m.y);
+            f[2 * e + 1] = dd.y - (cc.x * m.y + cc.y * m.x);
+        }
+        if (more) tmem_st32(trow + (uint32_t)(32 * c), f);
+    }
+    tmem_wait_st();
 }
 
 // MID: the middle lines (one launch) instead of the halves: a kernel of its
@@ -202,9 +270,12 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
         sm.stepof[q] = -1;   // not pivoted in this line yet
     }
     if (tid == 0) {
-        mbar_init(sm.pan_bar, kF2RowWarps);   // the peer's 4 row warps
-        mbar_init(sm.y_bar, kF2RowWarps);
-        mbar_init(sm.b_ready, kF2RowWarps);
+        mbar_init(sm.pan_bar, kF2RowWarps);   // the peer's row warps
+        mbar_init(sm.yn_bar, kF2RowWarps);    // the peer's row warps
+        mbar_init(sm.bn_ready, kF2RowWarps);
+        mbar_init(sm.x_ready, kF2RowWarps);
+        mbar_init(sm.y_bar, kF2RowWarps);     // the peer's helpers
+        mbar_init(sm.y_free, kF2RowWarps);    // the peer's helpers
         mbar_init(sm.next_ready, 1);
         mbar_init(sm.rest_done, 1);
         mbar_init(sm.fin, 1);
@@ -215,13 +286,7 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
     tc_fence_after();
     const uint32_t tmem = *sm.tslot;
     bool dead = false;
-    auto wait_cta = [&](uint64_t *bar, uint32_t parity) {
-        if (!dead && !mbar_wait_bounded_cta(smem_u32(bar), parity, kF2WaitLimit)) {
-            dead = true;
-            atomicOr(a.status, 2);
-        }
-    };
-    // the row warps' waits, whole warps
+    // waits by whole warps
     auto wait_warp = [&](uint64_t *bar, uint32_t parity) {
         if (!dead && !mbar_wait_warp_cta(smem_u32(bar), parity, kF2WaitLimit)) {
             dead = true;
@@ -235,66 +300,158 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
         }
     };
 
-    if (warp == kF2RowWarps) {
-        // ---------------------------------------------------- MMA issuer
-        if (lane == 0) {
-            const uint32_t sbo = (uint32_t)(2 * kF2B / 4) * 128u;
-            const uint32_t bhi = smem_u32(sm.Bhi), blo = smem_u32(sm.Blo);
-            // D[:, c0 + [0, len)) += X B[c0 + [0, len), :]^T, 3xTF32, in chunks of N <= 256
-            auto issue = [&](int c0, int len) {
-                for (int off = 0; off < len; off += 256) {
-                    const int nn = len - off < 256 ? len - off : 256;
-                    const int col = c0 + off;
-                    const uint32_t idesc = umma_idesc_tf32(nn);
-                    const uint32_t boff = (uint32_t)(col / 8) * sbo;
+    const int t = tid & (kF2RowThreads - 1);      // TMEM lane t
+    const int g = gbase + t;                      // this CTA's physical row in lane t
+    const bool valid = t < nr;
+    const uint32_t trow = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+    const float2 kzv = a.kz2[kz];
+    int cur = 0;
+
+    if (warp >= kF2RowWarps) {
+        // ------------------------------------------------------- helpers
+        const bool issuer = warp == kF2RowWarps;   // its lane 0 issues the MMAs
+        const uint32_t sbo = (uint32_t)(2 * kF2B / 4) * 128u;
+        const uint32_t bhi = smem_u32(sm.Bhi), blo = smem_u32(sm.Blo);
+        const uint32_t ybar_peer = mapa_u32(smem_u32(sm.y_bar), peer);
+        const uint32_t yfree_peer = mapa_u32(smem_u32(sm.y_free), peer);
+        const uint32_t y_peer = mapa_u32(smem_u32(sm.Y), peer);
+        // D[:, c0 + [0, len)) += X B[c0 + [0, len), :]^T, 3xTF32, in chunks of N <= 256
+        auto issue = [&](int c0, int len) {
+            for (int off = 0; off < len; off += 256) {
+                const int nn = len - off < 256 ? len - off : 256;
+                const int col = c0 + off;
+                const uint32_t idesc = umma_idesc_tf32(nn);
+                const uint32_t boff = (uint32_t)(col / 8) * sbo;
 #pragma unroll
-                    for (int ks = 0; ks < 2 * kF2B / 8; ks++) {
-                        const uint32_t koff = (uint32_t)ks * 256u;
-                        const uint64_t dh = umma_desc(bhi + boff + koff, 128, sbo);
-                        const uint64_t dl = umma_desc(blo + boff + koff, 128, sbo);
-                        const uint32_t xh = tmem + kXhi + (uint32_t)(ks * 8), xl = tmem + kXlo + (uint32_t)(ks * 8);
-                        const uint32_t d = tmem + (uint32_t)col;
-                        umma_tf32_ts(d, xh, dh, idesc, 1u);
-                        umma_tf32_ts(d, xh, dl, idesc, 1u);
-                        umma_tf32_ts(d, xl, dh, idesc, 1u);
-                    }
-                }
-            };
-            uint32_t ph = 0;
-            for (int ls = 0; ls < lines; ls++) {
-                for (int p = 0; p < npan; p++) {
-                    wait_cta(sm.b_ready, ph);
-                    ph ^= 1u;
-                    tc_fence_after();
-                    if (p + 1 < npan) {
-                        issue(2 * kF2B * (p + 1), 2 * kF2B);
-                        umma_commit(sm.next_ready);
-                        issue(0, 2 * kF2B * p);
-                        issue(2 * kF2B * (p + 2), 2 * ncol - 2 * kF2B * (p + 2));
-                    } else {
-                        issue(0, 2 * kF2B * p);
-                    }
-                    umma_commit(sm.rest_done);
+                for (int ks = 0; ks < 2 * kF2B / 8; ks++) {
+                    const uint32_t koff = (uint32_t)ks * 256u;
+                    const uint64_t dh = umma_desc(bhi + boff + koff, 128, sbo);
+                    const uint64_t dl = umma_desc(blo + boff + koff, 128, sbo);
+                    const uint32_t xh = tmem + kXhi + (uint32_t)(ks * 8), xl = tmem + kXlo + (uint32_t)(ks * 8);
+                    const uint32_t d = tmem + (uint32_t)col;
+                    umma_tf32_ts(d, xh, dh, idesc, 1u);
+                    umma_tf32_ts(d, xh, dl, idesc, 1u);
+                    umma_tf32_ts(d, xl, dh, idesc, 1u);
                 }
             }
+        };
+        uint32_t ph_x = 0, ph_bn = 0, ph_y = 0, ph_free = 0, ph_rest = 0;
+        bool first = true;   // no panel before this one: Y is free
+        f2_all_barrier();    // the first block is in TMEM
+        for (int ls = 0; ls < lines; ls++) {
+            for (int p = 0; p < npan; p++) {
+                const int k0 = p * kF2B, bl = min(kF2B, n - k0);
+                const bool next = p + 1 < npan;
+                // the panel's steps are done and its X is in TMEM (the row
+                // warps have waited for the previous trailing GEMM)
+                wait_warp(sm.x_ready, ph_x);
+                ph_x ^= 1u;
+                if (issuer && next) {
+                    wait_warp(sm.bn_ready, ph_bn);
+                    ph_bn ^= 1u;
+                    tc_fence_after();
+                    if (lane == 0) {
+                        issue(2 * kF2B * (p + 1), 2 * kF2B);
+                        umma_commit(sm.next_ready);
+                    }
+                    __syncwarp();
+                }
+                tc_fence_after();
+                if (!first) {   // the peer has read the previous panel's Y
+                    wait_cluster(sm.y_free, ph_free);
+                    ph_free ^= 1u;
+                }
+                first = false;
+                // ---- this CTA's pivot rows (before the panel's update) in the
+                // columns outside panels p and p + 1 into Y of both CTAs, two
+                // 32-column loads in flight per wait
+                const int skip = next ? 2 : 1, nc = npan - skip;
+                const int my_step = valid ? sm.stepof[g] : -1;
+                const bool piv = valid && my_step >= k0 && my_step < k0 + bl;
+                if (__any_sync(0xffffffffu, piv)) {
+                    const int yr = piv ? my_step - k0 : 0;
+                    float2 *yrow = sm.Y + (size_t)yr * kF2Yld;
+                    const uint32_t yrp = y_peer + (uint32_t)(yr * kF2Yld * sizeof(float2));
+#pragma unroll 1
+                    for (int c = 0; c < nc; c += 2) {
+                        const int c0 = c < p ? c : c + skip, c1 = c + 1 < p ? c + 1 : c + 1 + skip;
+                        float f[2][32];
+                        tmem_ld32_nowait(trow + (uint32_t)(32 * c0), f[0]);
+                        if (c + 1 < nc) tmem_ld32_nowait(trow + (uint32_t)(32 * c1), f[1]);
+                        tmem_wait_ld(f[0]);
+                        tmem_wait_ld(f[1]);
+                        if (piv) {
+#pragma unroll
+                            for (int h = 0; h < 2; h++) {
+                                if (c + h >= nc) break;
+                                const int col = 16 * (h ? c1 : c0);
+#pragma unroll
+                                for (int e = 0; e < 8; e++) {
+                                    const float4 q4 = make_float4(f[h][4 * e], f[h][4 * e + 1], f[h][4 * e + 2],
+                                                                  f[h][4 * e + 3]);
+                                    reinterpret_cast<float4 *>(yrow + col)[e] = q4;
+                                    st_cluster_v4f32(yrp + (uint32_t)((col + 2 * e) * sizeof(float2)), q4);
+                                }
+                            }
+                        }
+                    }
+                }
+                tc_fence_before();
+                mbar_arrive_warp_cluster(ybar_peer);
+                f2_helper_barrier();
+                wait_cluster(sm.y_bar, ph_y);
+                ph_y ^= 1u;
+                // ---- their B, and the GEMM of every column outside panels p, p + 1
+                for (int c = 0; c < nc; c++) {
+                    const int v = 128 * (c < p ? c : c + skip) + t;
+                    const int kk0 = 2 * ((v >> 2) & 7), j = (v >> 5) * 4 + (v & 3);
+                    const float2 y0 = kk0 < bl ? sm.Y[(size_t)kk0 * kF2Yld + j] : make_float2(0.f, 0.f);
+                    const float2 y1 = kk0 + 1 < bl ? sm.Y[(size_t)(kk0 + 1) * kF2Yld + j] : make_float2(0.f, 0.f);
+                    f2_put_b(sm, v, y0, y1);
+                }
+                fence_proxy_async_smem();
+                mbar_arrive_warp_cluster(yfree_peer);
+                f2_helper_barrier();
+                tc_fence_after();
+                if (issuer && lane == 0) {
+                    issue(0, 2 * kF2B * p);
+                    if (next) issue(2 * kF2B * (p + 2), 2 * ncol - 2 * kF2B * (p + 2));
+                    umma_commit(sm.rest_done);
+                }
+                __syncwarp();
+                if (next) ph_rest ^= 1u;   // (waited for by the row warps)
+            }
+            wait_warp(sm.rest_done, ph_rest);
+            ph_rest ^= 1u;
+            tc_fence_after();
+            f2_all_barrier();   // the next frame
+            cur ^= 1;
+            {
+                const int i = valid ? sm.rho[cur * kF2Tab + g] : 0;
+                const bool more = ls + 1 < lines;
+                const int line = MID ? hc.mid : hc.line(ls), nl = more ? hc.line(ls + 1) : 0;
+                f2_line_out(a, sm, trow, valid, i, sm.kap + cur * kF2Tab,
+                            a.Gt + ((long)kz * a.ny + line) * (long)n * a.ldg, ncol, 1, more, nl,
+                            more ? cmul(cin[nl], cout[line]) : make_float2(0.f, 0.f), kzv);
+            }
+            tc_fence_before();
+            f2_all_barrier();   // the next line's block is in TMEM
+            tc_fence_after();
+        }
+        if (issuer && lane == 0) {
             umma_commit(sm.fin);
             mbar_wait_bounded_cta(smem_u32(sm.fin), 0u, kF2WaitLimit);
         }
+        __syncwarp();
     } else {
         // ----------------------------------------------------- row threads
-        const int t = tid;                       // TMEM lane t
-        const int g = gbase + t;                 // this CTA's physical row in lane t
-        const bool valid = t < nr;
         const int g1 = t + kF2RowThreads;        // the second row of the panel steps (g0 = t)
         const bool has1 = g1 < n;
-        const uint32_t trow = tmem + ((uint32_t)(32 * warp) << 16);
         const uint32_t panbar_peer = mapa_u32(smem_u32(sm.pan_bar), peer);
-        const uint32_t ybar_peer = mapa_u32(smem_u32(sm.y_bar), peer);
+        const uint32_t ynbar_peer = mapa_u32(smem_u32(sm.yn_bar), peer);
         const uint32_t pf_peer = mapa_u32(smem_u32(sm.PF), peer);
-        const uint32_t y_peer = mapa_u32(smem_u32(sm.Y), peer);
-        const float2 kzv = a.kz2[kz];
-        uint32_t ph_pan = 0, ph_y = 0, ph_next = 0, ph_rest = 0;
-        int cur = 0;
+        const uint32_t yn_peer = mapa_u32(smem_u32(sm.Yn), peer);
+        uint32_t ph_pan = 0, ph_yn = 0, ph_next = 0, ph_rest = 0;
 
         // ---- the first line's block in the identity frame: D, and for the
         // middle line both neighbours' terms, their G from global memory
@@ -327,6 +484,9 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
             }
             tmem_wait_st();
         }
+        tc_fence_before();
+        f2_all_barrier();
+        tc_fence_after();
 
         for (int ls = 0; ls < lines; ls++) {
             const int line = MID ? hc.mid : hc.line(ls);
@@ -519,71 +679,45 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                     tmem_st32(trow + (uint32_t)(2 * k0), f);
                     tmem_wait_st();
                 }
+                tc_fence_before();
+                mbar_arrive_warp(sm.x_ready);
+                if (p + 1 == npan) continue;   // no next panel
                 // every read of this panel's PF is done before this CTA's
                 // pivot rows go out (the peer writes the next panel's PF only
                 // after it has them)
                 f2_row_barrier();
                 // ---- the panel's pivot rows of this CTA (their values before
-                // the panel's update, outside the panel) into Y of both CTAs
+                // the panel's update) in the next panel's columns into Yn of
+                // both CTAs
                 if (__any_sync(0xffffffffu, piv)) {
                     const int yr = piv ? my_step - k0 : 0;
-                    float2 *yrow = sm.Y + (size_t)yr * kF2Yld;
-                    const uint32_t yrp = y_peer + (uint32_t)(yr * kF2Yld * sizeof(float2));
-                    // two 32-column loads in flight per wait
-                    const int nc = ncol / 16;
-#pragma unroll 1
-                    for (int c = 0; c < nc; c += 2) {
-                        float f[2][32];
-                        tmem_ld32_nowait(trow + (uint32_t)(32 * c), f[0]);
-                        if (c + 1 < nc) tmem_ld32_nowait(trow + (uint32_t)(32 * (c + 1)), f[1]);
-                        tmem_wait_ld(f[0]);
-                        tmem_wait_ld(f[1]);
-                        if (piv) {
+                    float4 *yrow = reinterpret_cast<float4 *>(sm.Yn + (size_t)yr * kF2PFld);
+                    const uint32_t yrp = yn_peer + (uint32_t)(yr * kF2PFld * sizeof(float2));
+                    float f[32];
+                    tmem_ld32_nowait(trow + (uint32_t)(32 * (p + 1)), f);
+                    tmem_wait_ld(f);
+                    if (piv) {
 #pragma unroll
-                            for (int h = 0; h < 2; h++) {
-                                if (c + h >= nc) break;
-#pragma unroll
-                                for (int e = 0; e < 8; e++) {
-                                    const float4 q4 = make_float4(f[h][4 * e], f[h][4 * e + 1], f[h][4 * e + 2],
-                                                                  f[h][4 * e + 3]);
-                                    reinterpret_cast<float4 *>(yrow + 16 * (c + h))[e] = q4;
-                                    st_cluster_v4f32(yrp + (uint32_t)((16 * (c + h) + 2 * e) * sizeof(float2)), q4);
-                                }
-                            }
+                        for (int e = 0; e < 8; e++) {
+                            const float4 q4 = make_float4(f[4 * e], f[4 * e + 1], f[4 * e + 2], f[4 * e + 3]);
+                            yrow[e] = q4;
+                            st_cluster_v4f32(yrp + 16u * (uint32_t)e, q4);
                         }
                     }
                 }
                 tc_fence_before();
-                mbar_arrive_warp_cluster(ybar_peer);
+                mbar_arrive_warp_cluster(ynbar_peer);
                 f2_row_barrier();
-                wait_cluster(sm.y_bar, ph_y);
-                ph_y ^= 1u;
-                // ---- B = real form of Y (rows 2j + c, K = 2kk + c'), hi and lo:
-                // each pair (column j of Y, K quad kq) gives the 16-byte units of
-                // rows 2j, (Re y, -Im y), and 2j + 1, (Im y, Re y), adjacent in
-                // address order (row & 7, K quad, 8-row group); the TF32 split
-                // is odd in its argument, so one split serves both rows
-#pragma unroll 2
-                for (int v = t; v < ncol * (2 * kF2B / 4); v += kF2RowThreads) {
-                    const int jlo = v & 3, kq = (v >> 2) & 7, j = (v >> 5) * 4 + jlo;
-                    const int kk0 = 2 * kq;
-                    const float2 y0 = kk0 < bl ? sm.Y[(size_t)kk0 * kF2Yld + j] : make_float2(0.f, 0.f);
-                    const float2 y1 = kk0 + 1 < bl ? sm.Y[(size_t)(kk0 + 1) * kF2Yld + j] : make_float2(0.f, 0.f);
-                    float4 h, l;   // split of (Re y0, Im y0, Re y1, Im y1)
-                    tf32_split_fast(y0.x, h.x, l.x);
-                    tf32_split_fast(y0.y, h.y, l.y);
-                    tf32_split_fast(y1.x, h.z, l.z);
-                    tf32_split_fast(y1.y, h.w, l.w);
-                    const int u0 = (v >> 5) * 64 + kq * 8 + 2 * jlo;
-                    float4 *bh = reinterpret_cast<float4 *>(sm.Bhi) + u0;
-                    float4 *bl4 = reinterpret_cast<float4 *>(sm.Blo) + u0;
-                    bh[0] = make_float4(h.x, -h.y, h.z, -h.w);
-                    bh[1] = make_float4(h.y, h.x, h.w, h.z);
-                    bl4[0] = make_float4(l.x, -l.y, l.z, -l.w);
-                    bl4[1] = make_float4(l.y, l.x, l.w, l.z);
+                wait_cluster(sm.yn_bar, ph_yn);
+                ph_yn ^= 1u;
+                // ---- their B: one unit per thread
+                {
+                    const int kk0 = 2 * ((t >> 2) & 7), j = (t >> 5) * 4 + (t & 3);
+                    const float2 *y = sm.Yn + (size_t)kk0 * kF2PFld + j;
+                    f2_put_b(sm, 128 * (p + 1) + t, y[0], y[kF2PFld]);
                 }
                 fence_proxy_async_smem();
-                mbar_arrive_warp(sm.b_ready);
+                mbar_arrive_warp(sm.bn_ready);
             }
 
             // ---- the line's last GEMM done: the next frame
@@ -605,49 +739,21 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                 sm.kapinv[kap2[q]] = q;
                 sm.stepof[q] = -1;   // for the next line
             }
-            f2_row_barrier();
             cur = nxt;
 
-            // ---- G_line^T to global in the new frame, and S_{line+1} in place
+            // ---- G_line^T to global in the new frame, and S_{line+1} in place,
+            // every other chunk by the helpers
+            f2_all_barrier();
             {
-                const int i = valid ? rho2[g] : 0;
                 const bool more = ls + 1 < lines;
-                float2 cc = make_float2(0.f, 0.f);
-                F2Drow d = {};
-                int qd = -1, qs = -1, qp = -1;
-                if (more) {
-                    const int nl = hc.line(ls + 1);
-                    cc = cmul(cin[nl], cout[line]);
-                    d = f2_drow(a, nl, i, kzv);
-                    qd = sm.kapinv[i];
-                    qs = i > 0 ? sm.kapinv[i - 1] : -1;
-                    qp = i + 1 < n ? sm.kapinv[i + 1] : -1;
-                }
-                float2 *gout = a.Gt + ((long)kz * a.ny + line) * (long)n * a.ldg;
-#pragma unroll 1
-                for (int c = 0; c < ncol / 16; c++) {
-                    float f[32];
-                    tmem_ld32_nowait(trow + (uint32_t)(32 * c), f);
-                    tmem_wait_ld(f);
-#pragma unroll
-                    for (int e = 0; e < 16; e++) {
-                        const int q = 16 * c + e;
-                        const float2 m = make_float2(f[2 * e], f[2 * e + 1]);
-                        float2 s = make_float2(0.f, 0.f);
-                        if (valid && q < n) {
-                            gout[(long)kap2[q] * a.ldg + i] = m;
-                            s = make_float2(-(cc.x * m.x - cc.y * m.y), -(cc.x * m.y + cc.y * m.x));
-                            if (q == qd) s = cadd(s, d.diag);
-                            else if (q == qs) s = cadd(s, d.sub);
-                            else if (q == qp) s = cadd(s, d.sup);
-                        }
-                        f[2 * e] = s.x;
-                        f[2 * e + 1] = s.y;
-                    }
-                    if (more) tmem_st32(trow + (uint32_t)(32 * c), f);
-                }
-                tmem_wait_st();
+                const int nl = more ? hc.line(ls + 1) : 0;
+                f2_line_out(a, sm, trow, valid, valid ? rho2[g] : 0, kap2,
+                            a.Gt + ((long)kz * a.ny + line) * (long)n * a.ldg, ncol, 0, more, nl,
+                            more ? cmul(cin[nl], cout[line]) : make_float2(0.f, 0.f), kzv);
             }
+            tc_fence_before();
+            f2_all_barrier();   // the next line's block is in TMEM
+            tc_fence_after();
         }
     }
     tc_fence_before();

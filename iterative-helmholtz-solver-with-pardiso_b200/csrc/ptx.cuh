@@ -207,6 +207,11 @@ __device__ __forceinline__ void st_shared_u32_if(bool p, uint32_t addr, uint32_t
                  "r"(addr), "r"(v)
                  : "memory");
 }
+__device__ __forceinline__ void st_global_f2_if(bool p, float2 *addr, float2 v) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q st.global.v2.f32 [%1], {%2, %3};\n\t}" ::"r"((uint32_t)p),
+                 "l"(addr), "f"(v.x), "f"(v.y)
+                 : "memory");
+}
 
 // this thread's warp in its (1-D) block, in a form the compiler knows to be warp-uniform
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
