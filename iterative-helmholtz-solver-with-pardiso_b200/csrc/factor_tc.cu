@@ -6,9 +6,10 @@
 // and DirFactFastDiagStructOnline, Source/HODLR/BinaryTreesHODLR.cpp:
 // 2870-2969), from both ends towards the middle line (chain.cuh: one launch
 // for the halves, one for the middle lines): S_0 = D_0, S_j = D_j - cin[j]
-// cout[prev] G_prev, G_j = S_j^{-1}, by Gauss-Jordan with partial pivoting (the pivot of column k is the row,
-// among those not yet pivoted, with the largest |re| + |im|; ties to the
-// lowest row), G_j^T written row-major for the sweep.
+// cout[prev] G_prev, G_j = S_j^{-1}, by Gauss-Jordan with partial pivoting
+// (the pivot of column k is the row, among those not yet pivoted, with the
+// largest |re| + |im|; ties to the lowest row), G_j^T written row-major for
+// the sweep.
 //
 // Blocking.  Step k of in-place Gauss-Jordan changes every column j != k by
 // M[:, j] -= c_k p_k[j] with c_k the current column k (its pivot entry minus
@@ -16,96 +17,86 @@
 // the columns outside it as M_J <- M_J + X M_J[R, :], R the panel's pivot
 // rows and X = (the panel's columns after its 16 steps) - E_R (E_R: ones
 // at (r_k, k)).  The panel's steps run on CUDA cores with the panel in
-// registers (thread i = row i); X M[R, :] is one tcgen05 GEMM per panel
-// (M = 128 rows, N = 2 n_pad real columns, K = 32) accumulated into the
-// block in TMEM; the panel's own columns, which that product does not
-// describe, are then rewritten from registers.
+// registers (thread i = row i).
+//
+// Look-ahead.  The chain of pivot steps bounds the factor, so the row warps
+// do nothing but what the next step needs: they form the next panel's columns
+// themselves (FP32, X from their registers, the 16 x 16 pivot entries from
+// shared memory) and run its steps, while four helper warps gather the pivot
+// rows' other columns, build the GEMM's operand and issue X M[R, :] for every
+// column outside panels p and p + 1 (M = 128 rows, K = 32 real), accumulated
+// into the block in TMEM.  The row warps wait for that GEMM only before they
+// write the next X.  A panel's own columns, which the product does not
+// describe, are rewritten from registers.
+//
+// Frames.  The block is never unscrambled: physical row t of M holds logical
+// row rho[t], physical column q logical column kap[q], and the next line's S
+// is formed in place in the frame that the pivots leave (the derivation stands
+// in factor_tc2.cu).
 //
 // Layout per CTA (one CTA per (kz, half), its lines in sequence):
-//   TMEM (512 columns x 128 lanes): the block M (lane i = row i, column
-//     2j / 2j + 1 = Re / Im M[i][j]) at [0, 256); X hi at [256, 288), X lo at
-//     [288, 320) (lane i, column 2kk + re/im);
-//   shared memory: G_{j-1} (row-major, padded rows) for the next Schur
-//     complement and the write-out; B = real form of M[R, :] (hi and lo,
-//     canonical no-swizzle K-major, 2 n_pad rows x 32); the gathered pivot
-//     rows; the per-warp pivot keys and rows (double-buffered by step
-//     parity, so one barrier per step); the pivot order.
-// Warps 0-3: row threads; warp 4, one lane: MMA issuer.  Every wait is
-// bounded: on expiry bit 1 of *status is set and the kernel runs on without
-// waiting (results invalid), waits (bounded) for its MMAs, frees its TMEM
-// and returns.  A zero pivot sets bit 0.
+//   TMEM (lane t = row t): the block at columns [0, 2 ncol) (2j / 2j + 1 = Re /
+//     Im of column j, ncol = n rounded up to 16), X hi at [2 ncol, + 32), X lo
+//     after it: 256 columns for n <= 96, so that two CTAs share an SM, else 512;
+//   shared memory: B = real form of M[R, :] (hi and lo, canonical no-swizzle
+//     K-major, 2 ncol rows x 32); the gathered pivot rows; the per-warp pivot
+//     keys and rows (double-buffered by step parity, so one barrier per step);
+//     the frame and the pivot order.
+// Every wait is bounded: on expiry bit 1 of *status is set and the kernel
+// runs on without waiting (results invalid), waits (bounded) for its MMAs,
+// frees its TMEM and returns.  A zero pivot, or a column without a finite
+// candidate, sets bit 0.
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
-#include "chain.cuh"
-#include "cplx.cuh"
-#include "helm3d_internal.h"
-#include "ptx.cuh"
-#include "tcgen05.cuh"
+#include "factor_tc.cuh"
 
 namespace h3d {
 
-constexpr int kFtRowWarps = 4;
-constexpr int kFtThreads = (kFtRowWarps + 1) * 32;
 constexpr int kFtNP = 128;              // rows = TMEM lanes, padded columns
-constexpr int kFtB = 16;                // panel width
-constexpr uint32_t kFtCols = 512;
-constexpr uint32_t kFtXhi = 256, kFtXlo = 288;
-constexpr int kFtGld = kFtNP + 1;       // padded row of G in shared memory (float2)
 constexpr int kFtYld = kFtNP + 2;       // padded row of the gathered pivot rows (float2)
-constexpr uint32_t kFtWaitLimit = 1u << 22;
-
-struct FactorTcK {
-    int n, ny, ldg;
-    float2 *Gt;
-    const float2 *cmx, *cpx, *cmy, *cpy, *base2d, *kz2;
-    int *status;
-    const int *kzslot;   // >= 0: a skipped mode (nothing to do), or null
-};
 
 struct FtSmem {
-    float2 *G;          // [kFtNP][kFtGld]
     float *Bhi, *Blo;   // [2 kFtNP rows][2 kFtB] canonical each
-    float2 *Y;          // [kFtB][kFtYld]
+    float2 *Y;          // [kFtB][kFtYld]: the panel's pivot rows (the helpers')
+    float2 *Yn;         // [kFtB][kFtB]: their entries in the next panel's columns (the row warps')
     float2 *wrow;       // [2][4][kFtB]
     uint32_t *ckey;     // [2][4]: each warp's pivot key, by step parity
-    int *perm;          // [kFtNP]
-    uint64_t *b_ready, *mma_done, *fin;
+    int *rho, *kap;     // [2][kFtNP] each: the frame, double-buffered by line
+    int *kapinv, *perm, *stepof;   // [kFtNP]; stepof[t]: the step that pivoted row t
+    uint64_t *x_ready, *rest_done, *fin;
     uint32_t *tslot;
 };
 
-constexpr size_t kFtSmemBytes = sizeof(float2) * kFtNP * kFtGld + 2 * sizeof(float) * 2 * kFtNP * 2 * kFtB +
-                                sizeof(float2) * kFtB * kFtYld + sizeof(float2) * 2 * 4 * kFtB +
-                                sizeof(float) * 8 + sizeof(int) * 8 + sizeof(int) * kFtNP + 3 * sizeof(uint64_t) +
-                                16 + 128;
+constexpr size_t kFtSmemBytes = 2 * sizeof(float) * 2 * kFtNP * 2 * kFtB + sizeof(float2) * kFtB * (kFtYld + kFtB) +
+                                sizeof(float2) * 2 * 4 * kFtB + sizeof(uint32_t) * 8 + sizeof(int) * 7 * kFtNP +
+                                3 * sizeof(uint64_t) + 16;
 
 __device__ __forceinline__ FtSmem ft_carve(unsigned char *raw) {
     FtSmem s;
     s.Bhi = reinterpret_cast<float *>(raw);                       // 1024-aligned base
     s.Blo = s.Bhi + 2 * kFtNP * 2 * kFtB;
-    s.G = reinterpret_cast<float2 *>(s.Blo + 2 * kFtNP * 2 * kFtB);
-    s.Y = s.G + kFtNP * kFtGld;
-    s.wrow = s.Y + kFtB * kFtYld;
+    s.Y = reinterpret_cast<float2 *>(s.Blo + 2 * kFtNP * 2 * kFtB);
+    s.Yn = s.Y + kFtB * kFtYld;
+    s.wrow = s.Yn + kFtB * kFtB;
     s.ckey = reinterpret_cast<uint32_t *>(s.wrow + 2 * 4 * kFtB);
-    s.perm = reinterpret_cast<int *>(s.ckey + 8);
-    uintptr_t b = reinterpret_cast<uintptr_t>(s.perm + kFtNP);
-    b = (b + 15) & ~uintptr_t(15);
-    s.b_ready = reinterpret_cast<uint64_t *>(b);
-    s.mma_done = s.b_ready + 1;
-    s.fin = s.b_ready + 2;
-    s.tslot = reinterpret_cast<uint32_t *>(s.b_ready + 3);
+    s.rho = reinterpret_cast<int *>(s.ckey + 8);
+    s.kap = s.rho + 2 * kFtNP;
+    s.kapinv = s.kap + 2 * kFtNP;
+    s.perm = s.kapinv + kFtNP;
+    s.stepof = s.perm + kFtNP;
+    s.x_ready = reinterpret_cast<uint64_t *>(s.stepof + kFtNP);   // (every part a multiple of 16 bytes)
+    s.rest_done = s.x_ready + 1;
+    s.fin = s.x_ready + 2;
+    s.tslot = reinterpret_cast<uint32_t *>(s.x_ready + 3);
     return s;
 }
 
-__device__ __forceinline__ void ft_row_barrier() {
-    asm volatile("bar.sync 1, %0;" ::"n"(kFtRowWarps * 32) : "memory");
-}
-
 // MID: the middle lines (one launch) instead of the halves: a kernel of its
-// own, so that the halves' loop does not carry the middle line\'s code
+// own, so that the halves' loop does not carry the middle line's code
 template <bool MID>
-__global__ void __launch_bounds__(kFtThreads, 1) factor_tc_kernel(FactorTcK a) {
+__global__ void __launch_bounds__(kFtThreads, 2) factor_tc_kernel(FtK a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     FtSmem sm = ft_carve(smem_raw);
     const int n = a.n;
@@ -116,12 +107,20 @@ __global__ void __launch_bounds__(kFtThreads, 1) factor_tc_kernel(FactorTcK a) {
     if (a.kzslot && a.kzslot[kz] >= 0) return;   // a skipped mode (kz_skip_ratio): not factored / swept
     const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
     const int npan = (n + kFtB - 1) / kFtB;
-    const int ncol = ((n + 7) / 8) * 8;          // complex columns the GEMM covers (N = 2 ncol, a multiple of 16)
+    const int ncol = npan * kFtB;
+    const uint32_t cols = 2 * ncol + 64 <= 256 ? 256u : 512u;
 
-    if (warp == 0) tmem_alloc(sm.tslot, kFtCols);
+    if (warp == 0) tmem_alloc(sm.tslot, cols);
+    for (int q = tid; q < kFtNP; q += kFtThreads) {
+        sm.rho[q] = sm.rho[kFtNP + q] = q;
+        sm.kap[q] = sm.kap[kFtNP + q] = q;
+        sm.kapinv[q] = q;
+        sm.perm[q] = 0;
+        sm.stepof[q] = -1;   // not pivoted in this line yet
+    }
     if (tid == 0) {
-        mbar_init(sm.b_ready, kFtRowWarps);
-        mbar_init(sm.mma_done, 1);
+        mbar_init(sm.x_ready, kFtRowWarps);
+        mbar_init(sm.rest_done, 1);
         mbar_init(sm.fin, 1);
         fence_mbar_init_cluster();
     }
@@ -129,110 +128,120 @@ __global__ void __launch_bounds__(kFtThreads, 1) factor_tc_kernel(FactorTcK a) {
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *sm.tslot;
+    const uint32_t xhi = tmem + 2u * ncol, xlo = xhi + 32u;
     bool dead = false;
-    auto wait = [&](uint64_t *bar, uint32_t parity) {
-        if (!dead && !mbar_wait_bounded_cta(smem_u32(bar), parity, kFtWaitLimit)) {
+    auto wait = [&](uint64_t *bar, uint32_t parity) {   // whole warps
+        if (!dead && !mbar_wait_warp_cta(smem_u32(bar), parity, kFtWaitLimit)) {
             dead = true;
-            atomicOr(a.status, 2);
+            if (lane == 0) atomicOr(a.status, 2);
         }
     };
+    const int t = tid & (kFtRowThreads - 1);      // row t, TMEM lane t
+    const bool valid = t < n;
+    const uint32_t trow = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+    const float2 kzv = a.kz2[kz];
+    const bool helper = warp >= kFtRowWarps;
+    int cur = 0;
 
-    if (warp == kFtRowWarps) {
-        // ---------------------------------------------------- MMA issuer
-        if (lane == 0) {
-            const uint32_t idesc = umma_idesc_tf32(2 * ncol);
-            const uint32_t sbo = (uint32_t)(2 * kFtB / 4) * 128u;
-            const uint32_t bhi = smem_u32(sm.Bhi), blo = smem_u32(sm.Blo);
-            uint32_t ph = 0;
-            for (int ls = 0; ls < lines; ls++) {
-                for (int p = 0; p < npan; p++) {
-                    wait(sm.b_ready, ph);
-                    tc_fence_after();
+    // every other 16-column chunk of the block by each kind of warp, here and
+    // at the end of a line
+    if (lines > 0) ft_first_block<MID>(a, trow, valid, t, kz, MID ? hc.mid : hc.line(0), ncol, helper ? 1 : 0, kzv);
+    tc_fence_before();
+    ft_all_barrier();
+    tc_fence_after();
+    auto line_out = [&](int ls, int which) {
+        const int line = MID ? hc.mid : hc.line(ls);
+        const bool more = ls + 1 < lines;
+        const int nl = more ? hc.line(ls + 1) : 0;
+        ft_line_out(a, trow, valid, valid ? sm.rho[cur * kFtNP + t] : 0, sm.kap + cur * kFtNP, sm.kapinv,
+                    a.Gt + ((long)kz * a.ny + line) * (long)n * a.ldg, ncol, which, more, nl,
+                    more ? cmul(cin[nl], cout[line]) : make_float2(0.f, 0.f), kzv);
+        tc_fence_before();
+        ft_all_barrier();   // the next line's block is in TMEM
+        tc_fence_after();
+    };
+
+    if (helper) {
+        // ------------------------------------------------------- helpers
+        const bool issuer = warp == kFtRowWarps && lane == 0;
+        const uint32_t bhi = smem_u32(sm.Bhi), blo = smem_u32(sm.Blo);
+        uint32_t ph_x = 0, ph_rest = 0;
+        for (int ls = 0; ls < lines; ls++) {
+            for (int p = 0; p < npan; p++) {
+                const int k0 = p * kFtB, bl = min(kFtB, n - k0);
+                const int skip = p + 1 < npan ? 2 : 1, nc = npan - skip;
+                // the panel's steps are done and its X is in TMEM (the row
+                // warps have waited for the previous GEMM)
+                wait(sm.x_ready, ph_x);
+                ph_x ^= 1u;
+                tc_fence_after();
+                // ---- the pivot rows (before the panel's update) in the columns
+                // outside panels p and p + 1 into Y
+                const int my_step = valid ? sm.stepof[t] : -1;
+                const bool piv = my_step >= k0 && my_step < k0 + bl;
+                if (__any_sync(0xffffffffu, piv)) {
+                    const uint32_t yrow = smem_u32(sm.Y + (size_t)(piv ? my_step - k0 : 0) * kFtYld);
+#pragma unroll 1
+                    for (int c = 0; c < nc; c++) {
+                        const int cc = c < p ? c : c + skip;
+                        float f[32];
+                        tmem_ld32_nowait(trow + (uint32_t)(32 * cc), f);
+                        tmem_wait_ld(f);
 #pragma unroll
-                    for (int ks = 0; ks < 2 * kFtB / 8; ks++) {
-                        const uint32_t koff = (uint32_t)ks * 256u;   // 8 K = two core matrices of 128 B
-                        const uint64_t dh = umma_desc(bhi + koff, 128, sbo), dl = umma_desc(blo + koff, 128, sbo);
-                        const uint32_t xh = tmem + kFtXhi + (uint32_t)(ks * 8), xl = tmem + kFtXlo + (uint32_t)(ks * 8);
-                        umma_tf32_ts(tmem, xh, dh, idesc, 1u);
-                        umma_tf32_ts(tmem, xh, dl, idesc, 1u);
-                        umma_tf32_ts(tmem, xl, dh, idesc, 1u);
+                        for (int e = 0; e < 8; e++)
+                            st_shared_v4_if(piv, yrow + 128u * (uint32_t)cc + 16u * (uint32_t)e,
+                                            make_float4(f[4 * e], f[4 * e + 1], f[4 * e + 2], f[4 * e + 3]));
                     }
-                    umma_commit(sm.mma_done);
-                    ph ^= 1u;
                 }
+                tc_fence_before();
+                ft_helper_barrier();
+                // ---- their B, and the GEMM
+                for (int c = 0; c < nc; c++) {
+                    const int v = 128 * (c < p ? c : c + skip) + t;
+                    const int kk0 = 2 * ((v >> 2) & 7), j = (v >> 5) * 4 + (v & 3);
+                    const float2 y0 = kk0 < bl ? sm.Y[(size_t)kk0 * kFtYld + j] : make_float2(0.f, 0.f);
+                    const float2 y1 = kk0 + 1 < bl ? sm.Y[(size_t)(kk0 + 1) * kFtYld + j] : make_float2(0.f, 0.f);
+                    ft_put_b(sm.Bhi, sm.Blo, v, y0, y1);
+                }
+                fence_proxy_async_smem();
+                ft_helper_barrier();
+                tc_fence_after();
+                if (issuer) {
+                    ft_issue(tmem, xhi, xlo, bhi, blo, 0, 2 * kFtB * p);
+                    if (skip == 2) ft_issue(tmem, xhi, xlo, bhi, blo, 2 * kFtB * (p + 2), 2 * ncol - 2 * kFtB * (p + 2));
+                    umma_commit(sm.rest_done);
+                }
+                __syncwarp();
+                if (skip == 2) ph_rest ^= 1u;   // (waited for by the row warps)
             }
+            wait(sm.rest_done, ph_rest);
+            ph_rest ^= 1u;
+            tc_fence_after();
+            ft_all_barrier();   // the next frame
+            cur ^= 1;
+            line_out(ls, 1);
+        }
+        if (issuer) {
             umma_commit(sm.fin);
             mbar_wait_bounded_cta(smem_u32(sm.fin), 0u, kFtWaitLimit);
         }
+        __syncwarp();
     } else {
         // ----------------------------------------------------- row threads
-        const int t = tid;                        // row t, TMEM lane t
-        const uint32_t trow = tmem + ((uint32_t)(32 * warp) << 16);
-        uint32_t ph = 0;
-        const float2 kzv = a.kz2[kz];
+        uint32_t ph_rest = 0;
         for (int ls = 0; ls < lines; ls++) {
-            const int line = MID ? hc.mid : hc.line(ls);
-            // ---- S_line = D_line - cin[line] cout[prev] G_prev into TMEM; the
-            // middle line: minus both neighbours' terms, their G from global memory
-            {
-                const float2 cyd = make_float2(-(a.cmy[line].x + a.cpy[line].x), -(a.cmy[line].y + a.cpy[line].y));
-                const float2 cc = ls > 0 ? cmul(cin[line], cout[hc.line(ls - 1)]) : make_float2(0.f, 0.f);
-                const bool lo = MID && line > 0, hi = MID && line + 1 < a.ny;
-                const float2 clo = lo ? cmul(a.cmy[line], a.cpy[line - 1]) : make_float2(0.f, 0.f);
-                const float2 chi = hi ? cmul(a.cpy[line], a.cmy[line + 1]) : make_float2(0.f, 0.f);
-                const float2 *glo = a.Gt + ((long)kz * a.ny + line - 1) * (long)n * a.ldg;
-                const float2 *ghi = glo + 2 * (long)n * a.ldg;
-                float2 diag = make_float2(0.f, 0.f), sub = diag, sup = diag;
-                if (t < n) {
-                    diag = cadd(cadd(cyd, a.base2d[(long)line * n + t]), kzv);
-                    diag.x -= a.cmx[t].x + a.cpx[t].x;
-                    diag.y -= a.cmx[t].y + a.cpx[t].y;
-                    sub = a.cmx[t];
-                    sup = a.cpx[t];
-                }
-                const float2 *grow = sm.G + (size_t)t * kFtGld;
-#pragma unroll 1
-                for (int q = 0; q < kFtNP / 16; q++) {
-                    float v[32];
-#pragma unroll
-                    for (int e = 0; e < 16; e++) {
-                        const int j = 16 * q + e;
-                        float2 s = make_float2(0.f, 0.f);
-                        if (t >= n || j >= n) {
-                            if (t == j) s = make_float2(1.f, 0.f);
-                        } else {
-                            if (ls > 0) {
-                                const float2 g = grow[j];
-                                s = make_float2(-(cc.x * g.x - cc.y * g.y), -(cc.x * g.y + cc.y * g.x));
-                            }
-                            if (lo) s = cfms(clo, glo[(long)j * a.ldg + t], s);
-                            if (hi) s = cfms(chi, ghi[(long)j * a.ldg + t], s);
-                            if (j == t) s = cadd(s, diag);
-                            else if (j == t + 1) s = cadd(s, sup);
-                            else if (j == t - 1) s = cadd(s, sub);
-                        }
-                        v[2 * e] = s.x;
-                        v[2 * e + 1] = s.y;
-                    }
-                    tmem_st32(trow + (uint32_t)(32 * q), v);
-                }
-                tmem_wait_st();
-            }
-
             bool used = false;
             int my_step = -1;
+            float2 P[kFtB];
+            {   // the first panel's columns
+                float f[32];
+                tmem_ld32_nowait(trow, f);
+                tmem_wait_ld(f);
+#pragma unroll
+                for (int e = 0; e < kFtB; e++) P[e] = make_float2(f[2 * e], f[2 * e + 1]);
+            }
             for (int p = 0; p < npan; p++) {
                 const int k0 = p * kFtB, bl = min(kFtB, n - k0);
-                // ---- the panel's columns into registers
-                float2 P[kFtB];
-                {
-                    float f[32];
-                    tc_fence_after();
-                    tmem_ld32_nowait(trow + (uint32_t)(2 * k0), f);
-                    tmem_wait_ld(f);
-#pragma unroll
-                    for (int e = 0; e < kFtB; e++) P[e] = make_float2(f[2 * e], f[2 * e + 1]);
-                }
                 // ---- the panel's steps (CUDA cores), in a rolled loop: the row
                 // rotates by one column per step, so that the column of step kk
                 // is always P[0]; after step kk, P[e] holds panel column
@@ -308,6 +317,7 @@ __global__ void __launch_bounds__(kFtThreads, 1) factor_tc_kernel(FactorTcK a) {
                     pivp |= ip;
                     my_step = ip ? k : my_step;
                     st_shared_u32_if(ip, smem_u32(&sm.perm[k]), (uint32_t)t);
+                    st_shared_u32_if(ip, smem_u32(&sm.stepof[t]), (uint32_t)k);
                     P[0] = cfms(sfac, prow[0], P[1]);
                     key = 0;
                     {
@@ -325,148 +335,114 @@ __global__ void __launch_bounds__(kFtThreads, 1) factor_tc_kernel(FactorTcK a) {
 #pragma unroll
                     for (int e = 0; e < kFtB; e++) P[e] = cmul(P[e], psc);
                 }
-                // back to column order (P[e] holds column (bl + e) mod 16;
-                // only a partial last panel is not back in order), through
-                // this thread's row of G, which holds nothing during the panels
-                if (bl < kFtB) {
-                    float2 *tmp = sm.G + (size_t)t * kFtGld;
+                // back to column order (P[e] holds column (bl + e) mod 16; only
+                // a partial last panel is not back in order): rotated by bl
 #pragma unroll
-                    for (int e = 0; e < kFtB; e++) tmp[(bl + e) & (kFtB - 1)] = P[e];
+                for (int b = 1; b < kFtB; b *= 2)
+                    if (bl & b) {
+                        float2 Q[kFtB];
 #pragma unroll
-                    for (int e = 0; e < kFtB; e++) P[e] = tmp[e];
-                }
+                        for (int e = 0; e < kFtB; e++) Q[(e + b) & (kFtB - 1)] = P[e];
+#pragma unroll
+                        for (int e = 0; e < kFtB; e++) P[e] = Q[e];
+                    }
 
-                // ---- X = panel - E_R into TMEM (tf32 hi / lo)
+                // ---- the previous panel's GEMM is done: X = panel - E_R (tf32
+                // hi / lo) and the panel's own columns into TMEM, the next
+                // panel's columns out of it
+                if (p > 0) {
+                    wait(sm.rest_done, ph_rest);
+                    ph_rest ^= 1u;
+                    tc_fence_after();
+                }
+                const bool next = p + 1 < npan;
                 {
-                    float xh[32], xl[32];
-#pragma unroll
-                    for (int e = 0; e < kFtB; e++) {
-                        float2 x = make_float2(0.f, 0.f);
-                        if (e < bl) {
-                            x = P[e];
-                            if (my_step == k0 + e) x.x -= 1.f;
-                        }
-                        tf32_split_fast(x.x, xh[2 * e], xl[2 * e]);
-                        tf32_split_fast(x.y, xh[2 * e + 1], xl[2 * e + 1]);
-                    }
-                    tmem_st32(trow + kFtXhi, xh);
-                    tmem_st32(trow + kFtXlo, xl);
-                }
-                // ---- the pivot rows of this panel (values before its update) into Y
-                const bool piv = my_step >= k0 && my_step < k0 + bl;
-                if (__any_sync(0xffffffffu, piv)) {
-                    float2 *yrow = sm.Y + (size_t)(piv ? my_step - k0 : 0) * kFtYld;
-#pragma unroll 1
-                    for (int q = 0; q < kFtNP / 16; q++) {
-                        float f[32];
-                        tmem_ld32_nowait(trow + (uint32_t)(32 * q), f);
-                        tmem_wait_ld(f);
-                        if (piv) {
-#pragma unroll
-                            for (int e = 0; e < 16; e++) yrow[16 * q + e] = make_float2(f[2 * e], f[2 * e + 1]);
-                        }
-                    }
-                }
-                tmem_wait_st();
-                tc_fence_before();
-                ft_row_barrier();
-                // ---- B = real form of Y (rows 2j + c, K = 2kk + c'), hi and lo,
-                // 16-byte units in address order (row & 7, K quad, 8-row group)
-#pragma unroll 4
-                for (int u = t; u < 2 * ncol * (2 * kFtB / 4); u += kFtRowWarps * 32) {
-                    const int rlo = u & 7, kq = (u >> 3) & 7, rg = u >> 6;
-                    const int row = rg * 8 + rlo, j = row >> 1;
-                    const int kk0 = 2 * kq;
-                    const float2 y0 = kk0 < bl ? sm.Y[(size_t)kk0 * kFtYld + j] : make_float2(0.f, 0.f);
-                    const float2 y1 = kk0 + 1 < bl ? sm.Y[(size_t)(kk0 + 1) * kFtYld + j] : make_float2(0.f, 0.f);
-                    float4 e;
-                    if ((row & 1) == 0) e = make_float4(y0.x, -y0.y, y1.x, -y1.y);   // (Re y, -Im y)
-                    else e = make_float4(y0.y, y0.x, y1.y, y1.x);                   // (Im y, Re y)
-                    float4 h, l;
-                    tf32_split_fast(e.x, h.x, l.x);
-                    tf32_split_fast(e.y, h.y, l.y);
-                    tf32_split_fast(e.z, h.z, l.z);
-                    tf32_split_fast(e.w, h.w, l.w);
-                    reinterpret_cast<float4 *>(sm.Bhi)[u] = h;
-                    reinterpret_cast<float4 *>(sm.Blo)[u] = l;
-                }
-                fence_proxy_async_smem();
-                mbar_arrive_warp(sm.b_ready);
-                // ---- M += X B^T done: rewrite the panel's own columns
-                if (!dead && !mbar_wait_warp_cta(smem_u32(sm.mma_done), ph, kFtWaitLimit)) {
-                    dead = true;
-                    atomicOr(a.status, 2);
-                }
-                ph ^= 1u;
-                tc_fence_after();
-                {
-                    float f[32];
+                    float f[32], xl[32];
 #pragma unroll
                     for (int e = 0; e < kFtB; e++) {
                         f[2 * e] = P[e].x;
                         f[2 * e + 1] = P[e].y;
                     }
                     tmem_st32(trow + (uint32_t)(2 * k0), f);
-                    tmem_wait_st();
-                }
-            }
-
-            // ---- G = M with rows and columns unscrambled: G[step of row t][perm[j]] = M[t][j]
-            ft_row_barrier();
-            {
-                const int rt = (t < n) ? my_step : t;
-                float2 *gdst = sm.G + (size_t)(rt >= 0 ? rt : 0) * kFtGld;
-#pragma unroll 1
-                for (int q = 0; q < kFtNP / 16; q++) {
-                    float f[32];
-                    tmem_ld32_nowait(trow + (uint32_t)(32 * q), f);
-                    tmem_wait_ld(f);
-                    if (t < n && rt >= 0) {
 #pragma unroll
-                        for (int e = 0; e < 16; e++) {
-                            const int j = 16 * q + e;
-                            if (j < n) gdst[sm.perm[j]] = make_float2(f[2 * e], f[2 * e + 1]);
-                        }
+                    for (int e = 0; e < kFtB; e++) {   // P becomes X
+                        const bool one = my_step == k0 + e;
+                        P[e].x = e >= bl ? 0.f : one ? P[e].x - 1.f : P[e].x;
+                        P[e].y = e >= bl ? 0.f : P[e].y;
+                        tf32_split_fast(P[e].x, f[2 * e], xl[2 * e]);
+                        tf32_split_fast(P[e].y, f[2 * e + 1], xl[2 * e + 1]);
+                    }
+                    tmem_st32(xhi + ((uint32_t)(32 * warp) << 16), f);
+                    tmem_st32(xlo + ((uint32_t)(32 * warp) << 16), xl);
+                }
+                float m[32];
+                if (next) {
+                    tmem_ld32_nowait(trow + (uint32_t)(32 * (p + 1)), m);
+                    tmem_wait_ld(m);
+                }
+                tmem_wait_st();
+                tc_fence_before();
+                mbar_arrive_warp(sm.x_ready);
+                if (!next) break;
+                // ---- the next panel after this one: M + X M[R, :], in FP32
+                {
+                    const uint32_t yrow = smem_u32(sm.Yn + (pivp ? my_step - k0 : 0) * kFtB);
+#pragma unroll
+                    for (int e = 0; e < 8; e++)
+                        st_shared_v4_if(pivp, yrow + 16u * (uint32_t)e,
+                                        make_float4(m[4 * e], m[4 * e + 1], m[4 * e + 2], m[4 * e + 3]));
+                }
+                ft_row_barrier();
+#pragma unroll
+                for (int k = 0; k < kFtB; k++) {
+                    const float4 *y = reinterpret_cast<const float4 *>(sm.Yn + k * kFtB);
+#pragma unroll
+                    for (int e = 0; e < kFtB / 2; e++) {
+                        const float4 q = y[e];
+                        const float2 m0 = cfma(P[k], make_float2(q.x, q.y), make_float2(m[4 * e], m[4 * e + 1]));
+                        const float2 m1 = cfma(P[k], make_float2(q.z, q.w), make_float2(m[4 * e + 2], m[4 * e + 3]));
+                        m[4 * e] = m0.x;
+                        m[4 * e + 1] = m0.y;
+                        m[4 * e + 2] = m1.x;
+                        m[4 * e + 3] = m1.y;
                     }
                 }
+#pragma unroll
+                for (int e = 0; e < kFtB; e++) P[e] = make_float2(m[2 * e], m[2 * e + 1]);
             }
-            tc_fence_before();
+
+            // ---- the line's last GEMM done: the next frame, G_line^T to global
+            // memory and S_{line+1} in place
+            wait(sm.rest_done, ph_rest);
+            ph_rest ^= 1u;
+            tc_fence_after();
             ft_row_barrier();
-            // ---- G_line^T to global: row m of G^T = column m of G
-            if (t < n) {
-                float2 *gout = a.Gt + ((long)kz * a.ny + line) * (long)n * a.ldg;
-                const float2 *grow = sm.G + (size_t)t * kFtGld;
-                for (int m = 0; m < n; m++) gout[(long)m * a.ldg + t] = grow[m];
-            }
+            const int nxt = cur ^ 1;
+            ft_next_frame(n, t, sm.rho + cur * kFtNP, sm.kap + cur * kFtNP, sm.rho + nxt * kFtNP, sm.kap + nxt * kFtNP,
+                          sm.kapinv, sm.perm, sm.stepof);
+            ft_all_barrier();
+            cur = nxt;
+            line_out(ls, 0);
         }
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 0) tmem_dealloc(tmem, kFtCols);
+    if (warp == 0) tmem_dealloc(tmem, cols);
 }
 
 bool factor_tc_supported(bool c64, int n) { return c64 && n >= 1 && n <= kFtNP; }
 
 int launch_factor_tc(const FactorArgs &fa, cudaStream_t st) {
     if (fa.n < 1 || fa.n > kFtNP) return HELM3D_ERR_ARG;
+    // n > 96 holds all of TMEM: one CTA per SM, by shared memory (a second one
+    // would only wait for the first's TMEM)
+    const int npan = (fa.n + kFtB - 1) / kFtB;
+    const size_t smem = 2 * npan * kFtB + 64 <= 256 ? kFtSmemBytes : device_info().smem_optin;
     if (kFtSmemBytes > device_info().smem_optin) return HELM3D_ERR_ARG;
-    FactorTcK k;
-    k.n = fa.n;
-    k.ny = fa.ny;
-    k.ldg = fa.ldg;
-    k.Gt = (float2 *)fa.Gt;
-    k.cmx = (const float2 *)fa.cmx;
-    k.cpx = (const float2 *)fa.cpx;
-    k.cmy = (const float2 *)fa.cmy;
-    k.cpy = (const float2 *)fa.cpy;
-    k.base2d = (const float2 *)fa.base2d;
-    k.kz2 = (const float2 *)fa.kz2;
-    k.status = fa.status;
-    k.kzslot = fa.kzslot;
-    void (*kern)(FactorTcK) = fa.middle ? factor_tc_kernel<true> : factor_tc_kernel<false>;
-    if (!smem_limit_max(kern, kFtSmemBytes)) return HELM3D_ERR_CUDA;
-    kern<<<dim3((unsigned)((fa.middle ? 1 : 2) * fa.nz)), kFtThreads, kFtSmemBytes, st>>>(k);
+    void (*kern)(FtK) = fa.middle ? factor_tc_kernel<true> : factor_tc_kernel<false>;
+    if (!smem_limit_max(kern, smem)) return HELM3D_ERR_CUDA;
+    kern<<<dim3((unsigned)((fa.middle ? 1 : 2) * fa.nz)), kFtThreads, smem, st>>>(ft_args(fa));
     return cudaGetLastError() == cudaSuccess ? HELM3D_OK : HELM3D_ERR_CUDA;
 }
 

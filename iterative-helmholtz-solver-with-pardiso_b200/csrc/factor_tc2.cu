@@ -63,66 +63,49 @@
 
 #include <cstdint>
 
-#include "chain.cuh"
-#include "cplx.cuh"
-#include "helm3d_internal.h"
-#include "ptx.cuh"
-#include "tcgen05.cuh"
+#include "factor_tc.cuh"
 
 namespace h3d {
 
-constexpr int kF2RowWarps = 4;
-constexpr int kF2RowThreads = kF2RowWarps * 32;
-constexpr int kF2Threads = 2 * kF2RowThreads;   // the row warps and as many helpers
-constexpr int kF2B = 16;                         // panel width
 constexpr int kF2MaxN = 224;                     // 2 ncol + 64 X columns <= 512
 constexpr int kF2Tab = 256;
 constexpr uint32_t kF2Cols = 512;
-constexpr uint32_t kF2WaitLimit = 1u << 22;
-
-struct F2K {
-    int n, ny, ldg;
-    float2 *Gt;
-    const float2 *cmx, *cpx, *cmy, *cpy, *base2d, *kz2;
-    int *status;
-    const int *kzslot;   // >= 0: a skipped mode (nothing to do, in both CTAs), or null
-};
 
 struct F2Smem {
-    float *Bhi, *Blo;   // [2 kF2MaxN rows][2 kF2B] canonical K-major each
-    float2 *Y;          // [kF2B][kF2Yld]: the panel's pivot rows (the helpers')
-    float2 *Yn;         // [kF2B][kF2PFld]: their entries in the next panel's columns (the row warps')
+    float *Bhi, *Blo;   // [2 kF2MaxN rows][2 kFtB] canonical K-major each
+    float2 *Y;          // [kFtB][kF2Yld]: the panel's pivot rows (the helpers')
+    float2 *Yn;         // [kFtB][kF2PFld]: their entries in the next panel's columns (the row warps')
     float2 *PF;         // [kF2MaxN][kF2PFld]: the panel's entries of every row
-    float2 *wrow;       // [2][kF2RowWarps][kF2B]: each warp's candidate row, by step parity
-    uint32_t *wkey;     // [2][kF2RowWarps]
+    float2 *wrow;       // [2][kFtRowWarps][kFtB]: each warp's candidate row, by step parity
+    uint32_t *wkey;     // [2][kFtRowWarps]
     int *rho, *kap;     // [2][kF2Tab] each: the frame, double-buffered by line
     int *kapinv, *perm, *stepof;   // [kF2Tab]; stepof[g]: the step that pivoted row g
     uint64_t *pan_bar, *yn_bar, *bn_ready, *x_ready, *y_bar, *y_free, *next_ready, *rest_done, *fin;
     uint32_t *tslot;
 };
 
-constexpr size_t kF2BBytes = sizeof(float) * 2 * kF2MaxN * 2 * kF2B;
+constexpr size_t kF2BBytes = sizeof(float) * 2 * kF2MaxN * 2 * kFtB;
 // row stride of PF: 18 complex (144 bytes) instead of 16, so that a warp's
 // row-per-thread accesses (16-byte and 8-byte) fall on distinct banks
-constexpr int kF2PFld = kF2B + 2;
+constexpr int kF2PFld = kFtB + 2;
 // row stride of Y: 226 complex, so that the B build's reads of four pivot
 // rows at the same column fall on distinct banks (16-byte aligned rows)
 constexpr int kF2Yld = kF2MaxN + 2;
-constexpr size_t kF2SmemBytes = 2 * kF2BBytes + sizeof(float2) * (kF2B * kF2Yld + kF2B * kF2PFld + kF2PFld * kF2MaxN) +
-                                sizeof(float2) * 2 * kF2RowWarps * kF2B + sizeof(uint32_t) * 2 * kF2RowWarps +
+constexpr size_t kF2SmemBytes = 2 * kF2BBytes + sizeof(float2) * (kFtB * kF2Yld + kFtB * kF2PFld + kF2PFld * kF2MaxN) +
+                                sizeof(float2) * 2 * kFtRowWarps * kFtB + sizeof(uint32_t) * 2 * kFtRowWarps +
                                 sizeof(int) * 7 * kF2Tab + 9 * sizeof(uint64_t) + 16 + 1024 + 16;
 
 __device__ __forceinline__ F2Smem f2_carve(unsigned char *raw) {
     F2Smem s;
     uintptr_t b = (reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023);
     s.Bhi = reinterpret_cast<float *>(b);
-    s.Blo = s.Bhi + 2 * kF2MaxN * 2 * kF2B;
-    s.Y = reinterpret_cast<float2 *>(s.Blo + 2 * kF2MaxN * 2 * kF2B);
-    s.Yn = s.Y + kF2B * kF2Yld;
-    s.PF = s.Yn + kF2B * kF2PFld;
+    s.Blo = s.Bhi + 2 * kF2MaxN * 2 * kFtB;
+    s.Y = reinterpret_cast<float2 *>(s.Blo + 2 * kF2MaxN * 2 * kFtB);
+    s.Yn = s.Y + kFtB * kF2Yld;
+    s.PF = s.Yn + kFtB * kF2PFld;
     s.wrow = s.PF + kF2MaxN * kF2PFld;
-    s.wkey = reinterpret_cast<uint32_t *>(s.wrow + 2 * kF2RowWarps * kF2B);
-    s.rho = reinterpret_cast<int *>(s.wkey + 2 * kF2RowWarps);
+    s.wkey = reinterpret_cast<uint32_t *>(s.wrow + 2 * kFtRowWarps * kFtB);
+    s.rho = reinterpret_cast<int *>(s.wkey + 2 * kFtRowWarps);
     s.kap = s.rho + 2 * kF2Tab;
     s.kapinv = s.kap + 2 * kF2Tab;
     s.perm = s.kapinv + kF2Tab;
@@ -142,107 +125,16 @@ __device__ __forceinline__ F2Smem f2_carve(unsigned char *raw) {
     return s;
 }
 
-__device__ __forceinline__ void f2_row_barrier() {
-    asm volatile("bar.sync 1, %0;" ::"n"(kF2RowThreads) : "memory");
-}
-
-__device__ __forceinline__ void f2_helper_barrier() {
-    asm volatile("bar.sync 2, %0;" ::"n"(kF2Threads - kF2RowThreads) : "memory");
-}
-__device__ __forceinline__ void f2_all_barrier() { asm volatile("bar.sync 3, %0;" ::"n"(kF2Threads) : "memory"); }
-
 __device__ __forceinline__ void st_cluster_v4f32(uint32_t addr, float4 v) {
     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z),
                  "f"(v.w)
                  : "memory");
 }
 
-// The tridiagonal D_line in logical row i: diagonal, and the couplings to
-// logical columns i - 1 (sub) and i + 1 (sup).
-struct F2Drow {
-    float2 diag, sub, sup;
-};
-__device__ __forceinline__ F2Drow f2_drow(const F2K &a, int line, int i, float2 kzv) {
-    F2Drow d;
-    const float2 cyd = make_float2(-(a.cmy[line].x + a.cpy[line].x), -(a.cmy[line].y + a.cpy[line].y));
-    d.diag = cadd(cadd(cyd, a.base2d[(long)line * a.n + i]), kzv);
-    d.diag.x -= a.cmx[i].x + a.cpx[i].x;
-    d.diag.y -= a.cmx[i].y + a.cpx[i].y;
-    d.sub = a.cmx[i];
-    d.sup = a.cpx[i];
-    return d;
-}
-
-// pivot key of an entry of row g (0 when the row is not a candidate)
-__device__ __forceinline__ uint32_t f2_key(float2 v, bool cand, int g) {
-    if (!cand) return 0u;
-    const float av = fabsf(v.x) + fabsf(v.y);
-    if (!(av == av)) return 0u;
-    return (__float_as_uint(av) & 0xFFFFFF00u) | (uint32_t)(255 - g);
-}
-
-// Unit v of the real form of Y (rows 2j + c, K = 2kk + c'), hi and lo, from the
-// pivot rows' entries y0, y1 in column j = (v >> 5) * 4 + (v & 3), K quad
-// kq = (v >> 2) & 7: the 16-byte units of rows 2j, (Re y, -Im y), and 2j + 1,
-// (Im y, Re y), adjacent in address order (row & 7, K quad, 8-row group); the
-// TF32 split is odd in its argument, so one split serves both rows.
-__device__ __forceinline__ void f2_put_b(const F2Smem &sm, int v, float2 y0, float2 y1) {
-    float4 h, l;   // split of (Re y0, Im y0, Re y1, Im y1)
-    tf32_split_fast(y0.x, h.x, l.x);
-    tf32_split_fast(y0.y, h.y, l.y);
-    tf32_split_fast(y1.x, h.z, l.z);
-    tf32_split_fast(y1.y, h.w, l.w);
-    const int u0 = (v >> 5) * 64 + ((v >> 2) & 7) * 8 + 2 * (v & 3);
-    float4 *bh = reinterpret_cast<float4 *>(sm.Bhi) + u0;
-    float4 *bl = reinterpret_cast<float4 *>(sm.Blo) + u0;
-    bh[0] = make_float4(h.x, -h.y, h.z, -h.w);
-    bh[1] = make_float4(h.y, h.x, h.w, h.z);
-    bl[0] = make_float4(l.x, -l.y, l.z, -l.w);
-    bl[1] = make_float4(l.y, l.x, l.w, l.z);
-}
-
-// G_line^T to global memory in the frame (kap, i = rho of the thread's row),
-// and, with more, the next line's S in place: the 16-column chunks c = which,
-// which + 2, ... of this thread's TMEM lane.
-__device__ __forceinline__ void f2_line_out(const F2K &a, const F2Smem &sm, uint32_t trow, bool valid, int i,
-                                            const int *kap, float2 *gout, int ncol, int which, bool more, int nl,
-                                            float2 cc, float2 kzv) {
-    const int n = a.n;
-    F2Drow d = {};
-    int qd = -1, qs = -1, qp = -1;
-    if (more && valid) {
-        d = f2_drow(a, nl, i, kzv);
-        qd = sm.kapinv[i];
-        qs = i > 0 ? sm.kapinv[i - 1] : -1;
-        qp = i + 1 < n ? sm.kapinv[i + 1] : -1;
-    }
-#pragma unroll 1
-    for (int c = which; c < ncol / 16; c += 2) {
-        float f[32];
-        tmem_ld32_nowait(trow + (uint32_t)(32 * c), f);
-        int kq[16];
-#pragma unroll
-        for (int e = 0; e < 4; e++) *reinterpret_cast<int4 *>(kq + 4 * e) = reinterpret_cast<const int4 *>(kap + 16 * c)[e];
-        tmem_wait_ld(f);
-#pragma unroll
-        for (int e = 0; e < 16; e++) {   // (selects: a branch per entry costs more than the entry)
-            const int q = 16 * c + e;
-            const float2 m = make_float2(f[2 * e], f[2 * e + 1]);
-            st_global_f2_if(valid && q < n, gout + (unsigned)(kq[e] * a.ldg + i), m);
-            const float2 dd = make_float2(q == qd ? d.diag.x : q == qs ? d.sub.x : q == qp ? d.sup.x : 0.f,
-                                          q == qd ? d.diag.y : q == qs ? d.sub.y : q == qp ? d.sup.y : 0.f);
-            f[2 * e] = dd.x - (cc.x * m.x - cc.y * m.y);
-            f[2 * e + 1] = dd.y - (cc.x * m.y + cc.y * m.x);
-        }
-        if (more) tmem_st32(trow + (uint32_t)(32 * c), f);
-    }
-    tmem_wait_st();
-}
-
 // MID: the middle lines (one launch) instead of the halves: a kernel of its
 // own, so that the halves' loop does not carry the middle line\'s code
 template <bool MID>
-__global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
+__global__ void __launch_bounds__(kFtThreads, 1) factor_tc2_kernel(FtK a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     F2Smem sm = f2_carve(smem_raw);
     const int n = a.n;
@@ -257,12 +149,12 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
     const int n0 = (n + 1) >> 1;
     const int nr = rank == 0 ? n0 : n - n0;       // rows of this CTA
     const int gbase = rank == 0 ? 0 : n0;
-    const int ncol = (n + kF2B - 1) / kF2B * kF2B;
-    const int npan = ncol / kF2B;
+    const int ncol = (n + kFtB - 1) / kFtB * kFtB;
+    const int npan = ncol / kFtB;
     const uint32_t kXhi = 2u * ncol, kXlo = 2u * ncol + 32u;
 
     if (warp == 0) tmem_alloc(sm.tslot, kF2Cols);
-    for (int q = tid; q < kF2Tab; q += kF2Threads) {
+    for (int q = tid; q < kF2Tab; q += kFtThreads) {
         sm.rho[q] = q;
         sm.kap[q] = q;
         sm.kapinv[q] = q;
@@ -270,12 +162,12 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
         sm.stepof[q] = -1;   // not pivoted in this line yet
     }
     if (tid == 0) {
-        mbar_init(sm.pan_bar, kF2RowWarps);   // the peer's row warps
-        mbar_init(sm.yn_bar, kF2RowWarps);    // the peer's row warps
-        mbar_init(sm.bn_ready, kF2RowWarps);
-        mbar_init(sm.x_ready, kF2RowWarps);
-        mbar_init(sm.y_bar, kF2RowWarps);     // the peer's helpers
-        mbar_init(sm.y_free, kF2RowWarps);    // the peer's helpers
+        mbar_init(sm.pan_bar, kFtRowWarps);   // the peer's row warps
+        mbar_init(sm.yn_bar, kFtRowWarps);    // the peer's row warps
+        mbar_init(sm.bn_ready, kFtRowWarps);
+        mbar_init(sm.x_ready, kFtRowWarps);
+        mbar_init(sm.y_bar, kFtRowWarps);     // the peer's helpers
+        mbar_init(sm.y_free, kFtRowWarps);    // the peer's helpers
         mbar_init(sm.next_ready, 1);
         mbar_init(sm.rest_done, 1);
         mbar_init(sm.fin, 1);
@@ -288,59 +180,42 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
     bool dead = false;
     // waits by whole warps
     auto wait_warp = [&](uint64_t *bar, uint32_t parity) {
-        if (!dead && !mbar_wait_warp_cta(smem_u32(bar), parity, kF2WaitLimit)) {
+        if (!dead && !mbar_wait_warp_cta(smem_u32(bar), parity, kFtWaitLimit)) {
             dead = true;
             atomicOr(a.status, 2);
         }
     };
     auto wait_cluster = [&](uint64_t *bar, uint32_t parity) {
-        if (!dead && !mbar_wait_warp_cluster(smem_u32(bar), parity, kF2WaitLimit)) {
+        if (!dead && !mbar_wait_warp_cluster(smem_u32(bar), parity, kFtWaitLimit)) {
             dead = true;
             atomicOr(a.status, 2);
         }
     };
 
-    const int t = tid & (kF2RowThreads - 1);      // TMEM lane t
+    const int t = tid & (kFtRowThreads - 1);      // TMEM lane t
     const int g = gbase + t;                      // this CTA's physical row in lane t
     const bool valid = t < nr;
     const uint32_t trow = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
     const float2 kzv = a.kz2[kz];
     int cur = 0;
 
-    if (warp >= kF2RowWarps) {
+    if (warp >= kFtRowWarps) {
         // ------------------------------------------------------- helpers
-        const bool issuer = warp == kF2RowWarps;   // its lane 0 issues the MMAs
-        const uint32_t sbo = (uint32_t)(2 * kF2B / 4) * 128u;
+        const bool issuer = warp == kFtRowWarps;   // its lane 0 issues the MMAs
         const uint32_t bhi = smem_u32(sm.Bhi), blo = smem_u32(sm.Blo);
         const uint32_t ybar_peer = mapa_u32(smem_u32(sm.y_bar), peer);
         const uint32_t yfree_peer = mapa_u32(smem_u32(sm.y_free), peer);
         const uint32_t y_peer = mapa_u32(smem_u32(sm.Y), peer);
-        // D[:, c0 + [0, len)) += X B[c0 + [0, len), :]^T, 3xTF32, in chunks of N <= 256
-        auto issue = [&](int c0, int len) {
-            for (int off = 0; off < len; off += 256) {
-                const int nn = len - off < 256 ? len - off : 256;
-                const int col = c0 + off;
-                const uint32_t idesc = umma_idesc_tf32(nn);
-                const uint32_t boff = (uint32_t)(col / 8) * sbo;
-#pragma unroll
-                for (int ks = 0; ks < 2 * kF2B / 8; ks++) {
-                    const uint32_t koff = (uint32_t)ks * 256u;
-                    const uint64_t dh = umma_desc(bhi + boff + koff, 128, sbo);
-                    const uint64_t dl = umma_desc(blo + boff + koff, 128, sbo);
-                    const uint32_t xh = tmem + kXhi + (uint32_t)(ks * 8), xl = tmem + kXlo + (uint32_t)(ks * 8);
-                    const uint32_t d = tmem + (uint32_t)col;
-                    umma_tf32_ts(d, xh, dh, idesc, 1u);
-                    umma_tf32_ts(d, xh, dl, idesc, 1u);
-                    umma_tf32_ts(d, xl, dh, idesc, 1u);
-                }
-            }
-        };
+        auto issue = [&](int c0, int len) { ft_issue(tmem, tmem + kXhi, tmem + kXlo, bhi, blo, c0, len); };
         uint32_t ph_x = 0, ph_bn = 0, ph_y = 0, ph_free = 0, ph_rest = 0;
         bool first = true;   // no panel before this one: Y is free
-        f2_all_barrier();    // the first block is in TMEM
+        if (lines > 0) ft_first_block<MID>(a, trow, valid, g, kz, MID ? hc.mid : hc.line(0), ncol, 1, kzv);
+        tc_fence_before();
+        ft_all_barrier();    // the first block is in TMEM
+        tc_fence_after();
         for (int ls = 0; ls < lines; ls++) {
             for (int p = 0; p < npan; p++) {
-                const int k0 = p * kF2B, bl = min(kF2B, n - k0);
+                const int k0 = p * kFtB, bl = min(kFtB, n - k0);
                 const bool next = p + 1 < npan;
                 // the panel's steps are done and its X is in TMEM (the row
                 // warps have waited for the previous trailing GEMM)
@@ -351,7 +226,7 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                     ph_bn ^= 1u;
                     tc_fence_after();
                     if (lane == 0) {
-                        issue(2 * kF2B * (p + 1), 2 * kF2B);
+                        issue(2 * kFtB * (p + 1), 2 * kFtB);
                         umma_commit(sm.next_ready);
                     }
                     __syncwarp();
@@ -398,7 +273,7 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                 }
                 tc_fence_before();
                 mbar_arrive_warp_cluster(ybar_peer);
-                f2_helper_barrier();
+                ft_helper_barrier();
                 wait_cluster(sm.y_bar, ph_y);
                 ph_y ^= 1u;
                 // ---- their B, and the GEMM of every column outside panels p, p + 1
@@ -407,15 +282,15 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                     const int kk0 = 2 * ((v >> 2) & 7), j = (v >> 5) * 4 + (v & 3);
                     const float2 y0 = kk0 < bl ? sm.Y[(size_t)kk0 * kF2Yld + j] : make_float2(0.f, 0.f);
                     const float2 y1 = kk0 + 1 < bl ? sm.Y[(size_t)(kk0 + 1) * kF2Yld + j] : make_float2(0.f, 0.f);
-                    f2_put_b(sm, v, y0, y1);
+                    ft_put_b(sm.Bhi, sm.Blo, v, y0, y1);
                 }
                 fence_proxy_async_smem();
                 mbar_arrive_warp_cluster(yfree_peer);
-                f2_helper_barrier();
+                ft_helper_barrier();
                 tc_fence_after();
                 if (issuer && lane == 0) {
-                    issue(0, 2 * kF2B * p);
-                    if (next) issue(2 * kF2B * (p + 2), 2 * ncol - 2 * kF2B * (p + 2));
+                    issue(0, 2 * kFtB * p);
+                    if (next) issue(2 * kFtB * (p + 2), 2 * ncol - 2 * kFtB * (p + 2));
                     umma_commit(sm.rest_done);
                 }
                 __syncwarp();
@@ -424,28 +299,28 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
             wait_warp(sm.rest_done, ph_rest);
             ph_rest ^= 1u;
             tc_fence_after();
-            f2_all_barrier();   // the next frame
+            ft_all_barrier();   // the next frame
             cur ^= 1;
             {
                 const int i = valid ? sm.rho[cur * kF2Tab + g] : 0;
                 const bool more = ls + 1 < lines;
                 const int line = MID ? hc.mid : hc.line(ls), nl = more ? hc.line(ls + 1) : 0;
-                f2_line_out(a, sm, trow, valid, i, sm.kap + cur * kF2Tab,
+                ft_line_out(a, trow, valid, i, sm.kap + cur * kF2Tab, sm.kapinv,
                             a.Gt + ((long)kz * a.ny + line) * (long)n * a.ldg, ncol, 1, more, nl,
                             more ? cmul(cin[nl], cout[line]) : make_float2(0.f, 0.f), kzv);
             }
             tc_fence_before();
-            f2_all_barrier();   // the next line's block is in TMEM
+            ft_all_barrier();   // the next line's block is in TMEM
             tc_fence_after();
         }
         if (issuer && lane == 0) {
             umma_commit(sm.fin);
-            mbar_wait_bounded_cta(smem_u32(sm.fin), 0u, kF2WaitLimit);
+            mbar_wait_bounded_cta(smem_u32(sm.fin), 0u, kFtWaitLimit);
         }
         __syncwarp();
     } else {
         // ----------------------------------------------------- row threads
-        const int g1 = t + kF2RowThreads;        // the second row of the panel steps (g0 = t)
+        const int g1 = t + kFtRowThreads;        // the second row of the panel steps (g0 = t)
         const bool has1 = g1 < n;
         const uint32_t panbar_peer = mapa_u32(smem_u32(sm.pan_bar), peer);
         const uint32_t ynbar_peer = mapa_u32(smem_u32(sm.yn_bar), peer);
@@ -453,46 +328,16 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
         const uint32_t yn_peer = mapa_u32(smem_u32(sm.Yn), peer);
         uint32_t ph_pan = 0, ph_yn = 0, ph_next = 0, ph_rest = 0;
 
-        // ---- the first line's block in the identity frame: D, and for the
-        // middle line both neighbours' terms, their G from global memory
-        if (lines > 0) {
-            const int line = MID ? hc.mid : hc.line(0);
-            F2Drow d = f2_drow(a, line, valid ? g : 0, kzv);
-            const bool lo = MID && line > 0, hi = MID && line + 1 < a.ny;
-            const float2 clo = lo ? cmul(a.cmy[line], a.cpy[line - 1]) : make_float2(0.f, 0.f);
-            const float2 chi = hi ? cmul(a.cpy[line], a.cmy[line + 1]) : make_float2(0.f, 0.f);
-            const float2 *glo = a.Gt + ((long)kz * a.ny + line - 1) * (long)n * a.ldg + g;
-            const float2 *ghi = glo + 2 * (long)n * a.ldg;
-#pragma unroll 1
-            for (int c = 0; c < ncol / 16; c++) {
-                float f[32];
-#pragma unroll
-                for (int e = 0; e < 16; e++) {
-                    const int q = 16 * c + e;
-                    float2 s = make_float2(0.f, 0.f);
-                    if (valid && q < n) {
-                        if (q == g) s = d.diag;
-                        else if (q == g - 1) s = d.sub;
-                        else if (q == g + 1) s = d.sup;
-                        if (lo) s = cfms(clo, glo[(long)q * a.ldg], s);
-                        if (hi) s = cfms(chi, ghi[(long)q * a.ldg], s);
-                    }
-                    f[2 * e] = s.x;
-                    f[2 * e + 1] = s.y;
-                }
-                tmem_st32(trow + (uint32_t)(32 * c), f);
-            }
-            tmem_wait_st();
-        }
+        if (lines > 0) ft_first_block<MID>(a, trow, valid, g, kz, MID ? hc.mid : hc.line(0), ncol, 0, kzv);
         tc_fence_before();
-        f2_all_barrier();
+        ft_all_barrier();
         tc_fence_after();
 
         for (int ls = 0; ls < lines; ls++) {
             const int line = MID ? hc.mid : hc.line(ls);
             bool used0 = false, used1 = false;
             for (int p = 0; p < npan; p++) {
-                const int k0 = p * kF2B, bl = min(kF2B, n - k0);
+                const int k0 = p * kFtB, bl = min(kFtB, n - k0);
                 if (p > 0) {
                     wait_warp(sm.next_ready, ph_next);
                     ph_next ^= 1u;
@@ -507,7 +352,7 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                         float4 *dst = reinterpret_cast<float4 *>(sm.PF + (size_t)g * kF2PFld);
                         const uint32_t rdst = pf_peer + (uint32_t)(g * kF2PFld * sizeof(float2));
 #pragma unroll
-                        for (int e = 0; e < kF2B / 2; e++) {
+                        for (int e = 0; e < kFtB / 2; e++) {
                             const float4 q4 = make_float4(f[4 * e], f[4 * e + 1], f[4 * e + 2], f[4 * e + 3]);
                             dst[e] = q4;
                             st_cluster_v4f32(rdst + 16u * (uint32_t)e, q4);
@@ -515,15 +360,15 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                     }
                     mbar_arrive_warp_cluster(panbar_peer);
                 }
-                f2_row_barrier();
+                ft_row_barrier();
                 wait_cluster(sm.pan_bar, ph_pan);
                 ph_pan ^= 1u;
-                float2 P0[kF2B], P1[kF2B];
+                float2 P0[kFtB], P1[kFtB];
                 {
                     const float4 *s0 = reinterpret_cast<const float4 *>(sm.PF + (size_t)t * kF2PFld);
                     const float4 *s1 = reinterpret_cast<const float4 *>(sm.PF + (size_t)(has1 ? g1 : t) * kF2PFld);
 #pragma unroll
-                    for (int e = 0; e < kF2B / 2; e++) {
+                    for (int e = 0; e < kFtB / 2; e++) {
                         const float4 x0 = s0[e], x1 = s1[e];
                         P0[2 * e] = make_float2(x0.x, x0.y);
                         P0[2 * e + 1] = make_float2(x0.z, x0.w);
@@ -543,8 +388,8 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                 // the next pivot column, before the other columns.
                 float2 sc0 = make_float2(1.f, 0.f), sc1 = sc0;
                 bool piv0 = false, piv1 = false, bad = false;
-                uint32_t key0 = f2_key(P0[0], !used0, t);
-                uint32_t key1 = f2_key(P1[0], has1 && !used1, g1);
+                uint32_t key0 = ft_key(P0[0], !used0, t);
+                uint32_t key1 = ft_key(P1[0], has1 && !used1, g1);
                 uint32_t key = key0 > key1 ? key0 : key1;
                 uint32_t kw = __reduce_max_sync(0xffffffffu, key);
                 // every row's 1 / candidate, under the reduction's latency: the
@@ -554,31 +399,31 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
 #pragma unroll 1
                 for (int kk = 0; kk < bl; kk++) {
                     const int k = k0 + kk, buf = k & 1;
-                    st_shared_u32_if(lane == 0, smem_u32(&sm.wkey[buf * kF2RowWarps + warp]), kw);
+                    st_shared_u32_if(lane == 0, smem_u32(&sm.wkey[buf * kFtRowWarps + warp]), kw);
                     {
                         // the winning row in register order, w[1 + e] = prow[e], with
                         // 1 / pivot in the pivot's place
                         const bool win = kw != 0u && key == kw, first = key0 == kw;
-                        const uint32_t w = smem_u32(sm.wrow + (size_t)(buf * kF2RowWarps + warp) * kF2B);
+                        const uint32_t w = smem_u32(sm.wrow + (size_t)(buf * kFtRowWarps + warp) * kFtB);
                         const float2 h0 = make_float2(first ? inv0.x : inv1.x, first ? inv0.y : inv1.y);
 #pragma unroll
-                        for (int e = 0; e < kF2B / 2; e++)
+                        for (int e = 0; e < kFtB / 2; e++)
                             st_shared_v4_if(win, w + 16u * (uint32_t)e,
                                             make_float4(e == 0 ? h0.x : first ? P0[2 * e].x : P1[2 * e].x,
                                                         e == 0 ? h0.y : first ? P0[2 * e].y : P1[2 * e].y,
                                                         first ? P0[2 * e + 1].x : P1[2 * e + 1].x,
                                                         first ? P0[2 * e + 1].y : P1[2 * e + 1].y));
                     }
-                    f2_row_barrier();
-                    const uint4 kv = *reinterpret_cast<const uint4 *>(sm.wkey + buf * kF2RowWarps);
+                    ft_row_barrier();
+                    const uint4 kv = *reinterpret_cast<const uint4 *>(sm.wkey + buf * kFtRowWarps);
                     const uint32_t kmax = max(max(kv.x, kv.y), max(kv.z, kv.w));
                     const int r = kmax != 0u ? 255 - (int)(kmax & 0xFFu) : -1;
-                    const int wsel = (r & (kF2RowThreads - 1)) >> 5;   // the warp that holds row r
+                    const int wsel = (r & (kFtRowThreads - 1)) >> 5;   // the warp that holds row r
                     // the pivot row, rotated like the rows: prow[e] = column (kk + 1 + e) mod 16
-                    const float4 *w = reinterpret_cast<const float4 *>(sm.wrow + (size_t)(buf * kF2RowWarps + wsel) * kF2B);
-                    float2 prow[kF2B], pinv = make_float2(0.f, 0.f);
+                    const float4 *w = reinterpret_cast<const float4 *>(sm.wrow + (size_t)(buf * kFtRowWarps + wsel) * kFtB);
+                    float2 prow[kFtB], pinv = make_float2(0.f, 0.f);
 #pragma unroll
-                    for (int e = 0; e < kF2B / 2; e++) {
+                    for (int e = 0; e < kFtB / 2; e++) {
                         const float4 q4 = w[e];
                         if (e == 0) pinv = make_float2(r < 0 ? 0.f : q4.x, r < 0 ? 0.f : q4.y);
                         else prow[2 * e - 1] = make_float2(q4.x, q4.y);
@@ -602,29 +447,29 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                     st_shared_u32_if(ip0 || ip1, smem_u32(&sm.stepof[r >= 0 ? r : 0]), (uint32_t)k);
                     P0[0] = cfms(s0, prow[0], P0[1]);
                     P1[0] = cfms(s1, prow[0], P1[1]);
-                    key0 = f2_key(P0[0], !used0, t);
-                    key1 = f2_key(P1[0], has1 && !used1, g1);
+                    key0 = ft_key(P0[0], !used0, t);
+                    key1 = ft_key(P1[0], has1 && !used1, g1);
                     key = key0 > key1 ? key0 : key1;
                     kw = __reduce_max_sync(0xffffffffu, key);
                     inv0 = pivot_inv0(P0[0]);
                     inv1 = pivot_inv0(P1[0]);
 #pragma unroll
-                    for (int e = 1; e < kF2B - 1; e++) {
+                    for (int e = 1; e < kFtB - 1; e++) {
                         P0[e] = cfms(s0, prow[e], P0[e + 1]);
                         P1[e] = cfms(s1, prow[e], P1[e + 1]);
                     }
-                    P0[kF2B - 1] = ip0 ? make_float2(1.f, 0.f) : make_float2(-s0.x, -s0.y);
-                    P1[kF2B - 1] = ip1 ? make_float2(1.f, 0.f) : make_float2(-s1.x, -s1.y);
+                    P0[kFtB - 1] = ip0 ? make_float2(1.f, 0.f) : make_float2(-s0.x, -s0.y);
+                    P1[kFtB - 1] = ip1 ? make_float2(1.f, 0.f) : make_float2(-s1.x, -s1.y);
                 }
                 if (bad && t == 0 && rank == 0) atomicOr(a.status, 1);
                 // the panel's pivot rows scaled by their 1 / pv
                 if (piv0) {
 #pragma unroll
-                    for (int e = 0; e < kF2B; e++) P0[e] = cmul(P0[e], sc0);
+                    for (int e = 0; e < kFtB; e++) P0[e] = cmul(P0[e], sc0);
                 }
                 if (piv1) {
 #pragma unroll
-                    for (int e = 0; e < kF2B; e++) P1[e] = cmul(P1[e], sc1);
+                    for (int e = 0; e < kFtB; e++) P1[e] = cmul(P1[e], sc1);
                 }
                 // ---- the panel after its steps back into PF, in column order
                 // (P[e] holds column (bl + e) mod 16)
@@ -632,13 +477,13 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                     float2 *d0 = sm.PF + (size_t)t * kF2PFld;
                     float2 *d1 = sm.PF + (size_t)(has1 ? g1 : t) * kF2PFld;
 #pragma unroll
-                    for (int e = 0; e < kF2B; e++) d0[(bl + e) & (kF2B - 1)] = P0[e];
+                    for (int e = 0; e < kFtB; e++) d0[(bl + e) & (kFtB - 1)] = P0[e];
                     if (has1) {
 #pragma unroll
-                        for (int e = 0; e < kF2B; e++) d1[(bl + e) & (kF2B - 1)] = P1[e];
+                        for (int e = 0; e < kFtB; e++) d1[(bl + e) & (kFtB - 1)] = P1[e];
                     }
                 }
-                f2_row_barrier();
+                ft_row_barrier();
 
                 // ---- the previous panel's trailing GEMM is done: X and the
                 // panel's own columns of this CTA's rows into TMEM
@@ -653,7 +498,7 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                     float xh[32], xl[32], f[32];
                     const float4 *src = reinterpret_cast<const float4 *>(sm.PF + (size_t)(valid ? g : 0) * kF2PFld);
 #pragma unroll
-                    for (int e = 0; e < kF2B / 2; e++) {
+                    for (int e = 0; e < kFtB / 2; e++) {
                         const float4 q4 = src[e];
                         f[4 * e] = q4.x;
                         f[4 * e + 1] = q4.y;
@@ -665,7 +510,7 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                         for (int e = 0; e < 32; e++) f[e] = 0.f;
                     }
 #pragma unroll
-                    for (int e = 0; e < kF2B; e++) {
+                    for (int e = 0; e < kFtB; e++) {
                         float2 x = make_float2(0.f, 0.f);
                         if (e < bl) {
                             x = make_float2(f[2 * e], f[2 * e + 1]);
@@ -685,7 +530,7 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                 // every read of this panel's PF is done before this CTA's
                 // pivot rows go out (the peer writes the next panel's PF only
                 // after it has them)
-                f2_row_barrier();
+                ft_row_barrier();
                 // ---- the panel's pivot rows of this CTA (their values before
                 // the panel's update) in the next panel's columns into Yn of
                 // both CTAs
@@ -707,14 +552,14 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
                 }
                 tc_fence_before();
                 mbar_arrive_warp_cluster(ynbar_peer);
-                f2_row_barrier();
+                ft_row_barrier();
                 wait_cluster(sm.yn_bar, ph_yn);
                 ph_yn ^= 1u;
                 // ---- their B: one unit per thread
                 {
                     const int kk0 = 2 * ((t >> 2) & 7), j = (t >> 5) * 4 + (t & 3);
                     const float2 *y = sm.Yn + (size_t)kk0 * kF2PFld + j;
-                    f2_put_b(sm, 128 * (p + 1) + t, y[0], y[kF2PFld]);
+                    ft_put_b(sm.Bhi, sm.Blo, 128 * (p + 1) + t, y[0], y[kF2PFld]);
                 }
                 fence_proxy_async_smem();
                 mbar_arrive_warp(sm.bn_ready);
@@ -724,35 +569,25 @@ __global__ void __launch_bounds__(kF2Threads, 1) factor_tc2_kernel(F2K a) {
             wait_warp(sm.rest_done, ph_rest);
             ph_rest ^= 1u;
             tc_fence_after();
-            f2_row_barrier();
+            ft_row_barrier();
             const int nxt = cur ^ 1;
             const int *rho = sm.rho + cur * kF2Tab, *kap = sm.kap + cur * kF2Tab;
             int *rho2 = sm.rho + nxt * kF2Tab, *kap2 = sm.kap + nxt * kF2Tab;
-            for (int q = t; q < n; q += kF2RowThreads) {
-                int st = sm.stepof[q];
-                st = (st >= 0 && st < n) ? st : 0;   // a failed step leaves rows unpivoted (status set)
-                rho2[q] = kap[st];
-                kap2[q] = rho[sm.perm[q]];
-            }
-            f2_row_barrier();
-            for (int q = t; q < n; q += kF2RowThreads) {
-                sm.kapinv[kap2[q]] = q;
-                sm.stepof[q] = -1;   // for the next line
-            }
+            ft_next_frame(n, t, rho, kap, rho2, kap2, sm.kapinv, sm.perm, sm.stepof);
             cur = nxt;
 
             // ---- G_line^T to global in the new frame, and S_{line+1} in place,
             // every other chunk by the helpers
-            f2_all_barrier();
+            ft_all_barrier();
             {
                 const bool more = ls + 1 < lines;
                 const int nl = more ? hc.line(ls + 1) : 0;
-                f2_line_out(a, sm, trow, valid, valid ? rho2[g] : 0, kap2,
+                ft_line_out(a, trow, valid, valid ? rho2[g] : 0, kap2, sm.kapinv,
                             a.Gt + ((long)kz * a.ny + line) * (long)n * a.ldg, ncol, 0, more, nl,
                             more ? cmul(cin[nl], cout[line]) : make_float2(0.f, 0.f), kzv);
             }
             tc_fence_before();
-            f2_all_barrier();   // the next line's block is in TMEM
+            ft_all_barrier();   // the next line's block is in TMEM
             tc_fence_after();
         }
     }
@@ -768,21 +603,8 @@ bool factor_tc2_supported(bool c64, int n) { return c64 && n > 128 && n <= kF2Ma
 int launch_factor_tc2(const FactorArgs &fa, cudaStream_t st) {
     if (fa.n <= 128 || fa.n > kF2MaxN) return HELM3D_ERR_ARG;
     if (kF2SmemBytes > device_info().smem_optin) return HELM3D_ERR_ARG;
-    F2K k;
-    k.n = fa.n;
-    k.ny = fa.ny;
-    k.ldg = fa.ldg;
-    k.Gt = (float2 *)fa.Gt;
-    k.cmx = (const float2 *)fa.cmx;
-    k.cpx = (const float2 *)fa.cpx;
-    k.cmy = (const float2 *)fa.cmy;
-    k.cpy = (const float2 *)fa.cpy;
-    k.base2d = (const float2 *)fa.base2d;
-    k.kz2 = (const float2 *)fa.kz2;
-    k.status = fa.status;
-    k.kzslot = fa.kzslot;
     return launch_pairs(fa.middle ? factor_tc2_kernel<true> : factor_tc2_kernel<false>, (fa.middle ? 1 : 2) * fa.nz,
-                        kF2Threads, kF2SmemBytes, k, st);
+                        kFtThreads, kF2SmemBytes, ft_args(fa), st);
 }
 
 }  // namespace h3d
