@@ -35,13 +35,13 @@
 // in factor_tc2.cu).
 //
 // Layout per CTA (one CTA per (kz, half), its lines in sequence):
-//   TMEM (lane t = row t): the block at columns [0, 2 ncol) (2j / 2j + 1 = Re /
-//     Im of column j, ncol = n rounded up to 16), X hi at [2 ncol, + 32), X lo
-//     after it: 256 columns for n <= 96, so that two CTAs share an SM, else 512;
-//   shared memory: B = real form of M[R, :] (hi and lo, canonical no-swizzle
-//     K-major, 2 ncol rows x 32); the gathered pivot rows; the per-warp pivot
-//     keys and rows (double-buffered by step parity, so one barrier per step);
-//     the frame and the pivot order.
+//   TMEM (256 columns, lane t = row t): the block (columns 2j / 2j + 1 = Re /
+//     Im of column j);
+//   shared memory: X (A of the GEMM) and B = real form of M[R, :] (hi and lo,
+//     canonical no-swizzle K-major, 128 and 2 ncol rows x 32); the pivot rows
+//     in the next panel's columns; the per-warp pivot keys and rows (double-
+//     buffered by step parity, so one barrier per step); the frame and the
+//     pivot order.  Half of TMEM and of shared memory: two CTAs share an SM.
 // Every wait is bounded: on expiry bit 1 of *status is set and the kernel
 // runs on without waiting (results invalid), waits (bounded) for its MMAs,
 // frees its TMEM and returns.  A zero pivot, or a column without a finite
@@ -55,12 +55,14 @@
 namespace h3d {
 
 constexpr int kFtNP = 128;              // rows = TMEM lanes, padded columns
-constexpr int kFtYld = kFtNP + 2;       // padded row of the gathered pivot rows (float2)
+constexpr int kFtYld = kFtB + 2;        // row of Y: reads of four rows at a column fall on distinct banks
+constexpr uint32_t kFtCols = 2 * kFtNP; // TMEM columns: two CTAs per SM
 
 struct FtSmem {
     float *Bhi, *Blo;   // [2 kFtNP rows][2 kFtB] canonical each
-    float2 *Y;          // [kFtB][kFtYld]: the panel's pivot rows (the helpers')
-    float2 *Yn;         // [kFtB][kFtB]: their entries in the next panel's columns (the row warps')
+    float *Xhi, *Xlo;   // [kFtNP rows][2 kFtB] canonical each
+    float2 *Yn;         // [kFtB][kFtB]: the pivot rows in the next panel's columns (the row warps')
+    float2 *Y;          // [2][kFtB][kFtYld]: ... in one panel's columns, by turns (the helpers')
     float2 *wrow;       // [2][4][kFtB]
     uint32_t *ckey;     // [2][4]: each warp's pivot key, by step parity
     int *rho, *kap;     // [2][kFtNP] each: the frame, double-buffered by line
@@ -69,7 +71,7 @@ struct FtSmem {
     uint32_t *tslot;
 };
 
-constexpr size_t kFtSmemBytes = 2 * sizeof(float) * 2 * kFtNP * 2 * kFtB + sizeof(float2) * kFtB * (kFtYld + kFtB) +
+constexpr size_t kFtSmemBytes = 2 * sizeof(float) * 3 * kFtNP * 2 * kFtB + sizeof(float2) * kFtB * (kFtB + 2 * kFtYld) +
                                 sizeof(float2) * 2 * 4 * kFtB + sizeof(uint32_t) * 8 + sizeof(int) * 7 * kFtNP +
                                 3 * sizeof(uint64_t) + 16;
 
@@ -77,9 +79,11 @@ __device__ __forceinline__ FtSmem ft_carve(unsigned char *raw) {
     FtSmem s;
     s.Bhi = reinterpret_cast<float *>(raw);                       // 1024-aligned base
     s.Blo = s.Bhi + 2 * kFtNP * 2 * kFtB;
-    s.Y = reinterpret_cast<float2 *>(s.Blo + 2 * kFtNP * 2 * kFtB);
-    s.Yn = s.Y + kFtB * kFtYld;
-    s.wrow = s.Yn + kFtB * kFtB;
+    s.Xhi = s.Blo + 2 * kFtNP * 2 * kFtB;
+    s.Xlo = s.Xhi + kFtNP * 2 * kFtB;
+    s.Yn = reinterpret_cast<float2 *>(s.Xlo + kFtNP * 2 * kFtB);
+    s.Y = s.Yn + kFtB * kFtB;
+    s.wrow = s.Y + 2 * kFtB * kFtYld;
     s.ckey = reinterpret_cast<uint32_t *>(s.wrow + 2 * 4 * kFtB);
     s.rho = reinterpret_cast<int *>(s.ckey + 8);
     s.kap = s.rho + 2 * kFtNP;
@@ -108,9 +112,8 @@ __global__ void __launch_bounds__(kFtThreads, 2) factor_tc_kernel(FtK a) {
     const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
     const int npan = (n + kFtB - 1) / kFtB;
     const int ncol = npan * kFtB;
-    const uint32_t cols = 2 * ncol + 64 <= 256 ? 256u : 512u;
 
-    if (warp == 0) tmem_alloc(sm.tslot, cols);
+    if (warp == 0) tmem_alloc(sm.tslot, kFtCols);
     for (int q = tid; q < kFtNP; q += kFtThreads) {
         sm.rho[q] = sm.rho[kFtNP + q] = q;
         sm.kap[q] = sm.kap[kFtNP + q] = q;
@@ -128,7 +131,6 @@ __global__ void __launch_bounds__(kFtThreads, 2) factor_tc_kernel(FtK a) {
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *sm.tslot;
-    const uint32_t xhi = tmem + 2u * ncol, xlo = xhi + 32u;
     bool dead = false;
     auto wait = [&](uint64_t *bar, uint32_t parity) {   // whole warps
         if (!dead && !mbar_wait_warp_cta(smem_u32(bar), parity, kFtWaitLimit)) {
@@ -164,51 +166,66 @@ __global__ void __launch_bounds__(kFtThreads, 2) factor_tc_kernel(FtK a) {
     if (helper) {
         // ------------------------------------------------------- helpers
         const bool issuer = warp == kFtRowWarps && lane == 0;
-        const uint32_t bhi = smem_u32(sm.Bhi), blo = smem_u32(sm.Blo);
+        const uint32_t bhi = smem_u32(sm.Bhi), blo = smem_u32(sm.Blo), xhi = smem_u32(sm.Xhi), xlo = smem_u32(sm.Xlo);
+        // D[:, c0 + [0, len)) += X B[c0 + [0, len), :]^T, 3xTF32
+        auto issue = [&](int c0, int len) {
+            if (len <= 0) return;
+            const uint32_t sbo = (uint32_t)(2 * kFtB / 4) * 128u, idesc = umma_idesc_tf32(len);
+            const uint32_t boff = (uint32_t)(c0 / 8) * sbo, d = tmem + (uint32_t)c0;
+#pragma unroll
+            for (int ks = 0; ks < 2 * kFtB / 8; ks++) {
+                const uint32_t koff = (uint32_t)ks * 256u;   // 8 K = two core matrices of 128 B
+                const uint64_t dh = umma_desc(bhi + boff + koff, 128, sbo), dl = umma_desc(blo + boff + koff, 128, sbo);
+                const uint64_t xh = umma_desc(xhi + koff, 128, sbo), xl = umma_desc(xlo + koff, 128, sbo);
+                umma_tf32(d, xh, dh, idesc, 1u);
+                umma_tf32(d, xh, dl, idesc, 1u);
+                umma_tf32(d, xl, dh, idesc, 1u);
+            }
+        };
         uint32_t ph_x = 0, ph_rest = 0;
         for (int ls = 0; ls < lines; ls++) {
             for (int p = 0; p < npan; p++) {
                 const int k0 = p * kFtB, bl = min(kFtB, n - k0);
                 const int skip = p + 1 < npan ? 2 : 1, nc = npan - skip;
-                // the panel's steps are done and its X is in TMEM (the row
+                // the panel's steps are done and its X is in place (the row
                 // warps have waited for the previous GEMM)
                 wait(sm.x_ready, ph_x);
                 ph_x ^= 1u;
                 tc_fence_after();
                 // ---- the pivot rows (before the panel's update) in the columns
-                // outside panels p and p + 1 into Y
+                // outside panels p and p + 1 through Y into B, a panel's columns
+                // at a time, the next ones on their way out of TMEM meanwhile
                 const int my_step = valid ? sm.stepof[t] : -1;
                 const bool piv = my_step >= k0 && my_step < k0 + bl;
-                if (__any_sync(0xffffffffu, piv)) {
-                    const uint32_t yrow = smem_u32(sm.Y + (size_t)(piv ? my_step - k0 : 0) * kFtYld);
+                const bool any = __any_sync(0xffffffffu, piv);
+                const uint32_t yrow = smem_u32(sm.Y + (piv ? my_step - k0 : 0) * kFtYld);
+                const int kk0 = 2 * ((t >> 2) & 7);
+                float f[32];
+                if (any && nc > 0) tmem_ld32_nowait(trow + (uint32_t)(32 * (p > 0 ? 0 : skip)), f);
 #pragma unroll 1
-                    for (int c = 0; c < nc; c++) {
-                        const int cc = c < p ? c : c + skip;
-                        float f[32];
-                        tmem_ld32_nowait(trow + (uint32_t)(32 * cc), f);
+                for (int c = 0; c < nc; c++) {
+                    const int cc = c < p ? c : c + skip;
+                    const uint32_t half = (uint32_t)((c & 1) * kFtB * kFtYld * sizeof(float2));
+                    if (any) {
                         tmem_wait_ld(f);
 #pragma unroll
                         for (int e = 0; e < 8; e++)
-                            st_shared_v4_if(piv, yrow + 128u * (uint32_t)cc + 16u * (uint32_t)e,
+                            st_shared_v4_if(piv, yrow + half + 16u * (uint32_t)e,
                                             make_float4(f[4 * e], f[4 * e + 1], f[4 * e + 2], f[4 * e + 3]));
+                        if (c + 1 < nc) tmem_ld32_nowait(trow + (uint32_t)(32 * (c + 1 < p ? c + 1 : c + 1 + skip)), f);
                     }
+                    ft_helper_barrier();
+                    const float2 *y = sm.Y + ((c & 1) * kFtB + kk0) * kFtYld + (t >> 5) * 4 + (t & 3);
+                    ft_put_b(sm.Bhi, sm.Blo, 128 * cc + t, kk0 < bl ? y[0] : make_float2(0.f, 0.f),
+                             kk0 + 1 < bl ? y[kFtYld] : make_float2(0.f, 0.f));
                 }
                 tc_fence_before();
-                ft_helper_barrier();
-                // ---- their B, and the GEMM
-                for (int c = 0; c < nc; c++) {
-                    const int v = 128 * (c < p ? c : c + skip) + t;
-                    const int kk0 = 2 * ((v >> 2) & 7), j = (v >> 5) * 4 + (v & 3);
-                    const float2 y0 = kk0 < bl ? sm.Y[(size_t)kk0 * kFtYld + j] : make_float2(0.f, 0.f);
-                    const float2 y1 = kk0 + 1 < bl ? sm.Y[(size_t)(kk0 + 1) * kFtYld + j] : make_float2(0.f, 0.f);
-                    ft_put_b(sm.Bhi, sm.Blo, v, y0, y1);
-                }
                 fence_proxy_async_smem();
                 ft_helper_barrier();
                 tc_fence_after();
                 if (issuer) {
-                    ft_issue(tmem, xhi, xlo, bhi, blo, 0, 2 * kFtB * p);
-                    if (skip == 2) ft_issue(tmem, xhi, xlo, bhi, blo, 2 * kFtB * (p + 2), 2 * ncol - 2 * kFtB * (p + 2));
+                    issue(0, 2 * kFtB * p);
+                    if (skip == 2) issue(2 * kFtB * (p + 2), 2 * ncol - 2 * kFtB * (p + 2));
                     umma_commit(sm.rest_done);
                 }
                 __syncwarp();
@@ -347,9 +364,9 @@ __global__ void __launch_bounds__(kFtThreads, 2) factor_tc_kernel(FtK a) {
                         for (int e = 0; e < kFtB; e++) P[e] = Q[e];
                     }
 
-                // ---- the previous panel's GEMM is done: X = panel - E_R (tf32
-                // hi / lo) and the panel's own columns into TMEM, the next
-                // panel's columns out of it
+                // ---- the previous panel's GEMM is done: X = panel - E_R into
+                // shared memory (tf32 hi / lo), the panel's own columns into TMEM,
+                // the next panel's columns out of it
                 if (p > 0) {
                     wait(sm.rest_done, ph_rest);
                     ph_rest ^= 1u;
@@ -357,24 +374,31 @@ __global__ void __launch_bounds__(kFtThreads, 2) factor_tc_kernel(FtK a) {
                 }
                 const bool next = p + 1 < npan;
                 {
-                    float f[32], xl[32];
+                    float f[32];
 #pragma unroll
                     for (int e = 0; e < kFtB; e++) {
                         f[2 * e] = P[e].x;
                         f[2 * e + 1] = P[e].y;
                     }
                     tmem_st32(trow + (uint32_t)(2 * k0), f);
+                    float *xh = sm.Xhi + canon_off(t, 0, 2 * kFtB) / 4, *xl = sm.Xlo + canon_off(t, 0, 2 * kFtB) / 4;
 #pragma unroll
-                    for (int e = 0; e < kFtB; e++) {   // P becomes X
-                        const bool one = my_step == k0 + e;
-                        P[e].x = e >= bl ? 0.f : one ? P[e].x - 1.f : P[e].x;
-                        P[e].y = e >= bl ? 0.f : P[e].y;
-                        tf32_split_fast(P[e].x, f[2 * e], xl[2 * e]);
-                        tf32_split_fast(P[e].y, f[2 * e + 1], xl[2 * e + 1]);
+                    for (int e = 0; e < kFtB; e += 2) {
+#pragma unroll
+                        for (int h = e; h < e + 2; h++) {   // P becomes X
+                            P[h].x = h >= bl ? 0.f : my_step == k0 + h ? P[h].x - 1.f : P[h].x;
+                            P[h].y = h >= bl ? 0.f : P[h].y;
+                        }
+                        float4 h4, l4;
+                        tf32_split_fast(P[e].x, h4.x, l4.x);
+                        tf32_split_fast(P[e].y, h4.y, l4.y);
+                        tf32_split_fast(P[e + 1].x, h4.z, l4.z);
+                        tf32_split_fast(P[e + 1].y, h4.w, l4.w);
+                        *reinterpret_cast<float4 *>(xh + 16 * e) = h4;
+                        *reinterpret_cast<float4 *>(xl + 16 * e) = l4;
                     }
-                    tmem_st32(xhi + ((uint32_t)(32 * warp) << 16), f);
-                    tmem_st32(xlo + ((uint32_t)(32 * warp) << 16), xl);
                 }
+                fence_proxy_async_smem();
                 float m[32];
                 if (next) {
                     tmem_ld32_nowait(trow + (uint32_t)(32 * (p + 1)), m);
@@ -428,21 +452,17 @@ __global__ void __launch_bounds__(kFtThreads, 2) factor_tc_kernel(FtK a) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 0) tmem_dealloc(tmem, cols);
+    if (warp == 0) tmem_dealloc(tmem, kFtCols);
 }
 
 bool factor_tc_supported(bool c64, int n) { return c64 && n >= 1 && n <= kFtNP; }
 
 int launch_factor_tc(const FactorArgs &fa, cudaStream_t st) {
     if (fa.n < 1 || fa.n > kFtNP) return HELM3D_ERR_ARG;
-    // n > 96 holds all of TMEM: one CTA per SM, by shared memory (a second one
-    // would only wait for the first's TMEM)
-    const int npan = (fa.n + kFtB - 1) / kFtB;
-    const size_t smem = 2 * npan * kFtB + 64 <= 256 ? kFtSmemBytes : device_info().smem_optin;
     if (kFtSmemBytes > device_info().smem_optin) return HELM3D_ERR_ARG;
     void (*kern)(FtK) = fa.middle ? factor_tc_kernel<true> : factor_tc_kernel<false>;
-    if (!smem_limit_max(kern, smem)) return HELM3D_ERR_CUDA;
-    kern<<<dim3((unsigned)((fa.middle ? 1 : 2) * fa.nz)), kFtThreads, smem, st>>>(ft_args(fa));
+    if (!smem_limit_max(kern, kFtSmemBytes)) return HELM3D_ERR_CUDA;
+    kern<<<dim3((unsigned)((fa.middle ? 1 : 2) * fa.nz)), kFtThreads, kFtSmemBytes, st>>>(ft_args(fa));
     return cudaGetLastError() == cudaSuccess ? HELM3D_OK : HELM3D_ERR_CUDA;
 }
 

@@ -202,6 +202,11 @@ __device__ __forceinline__ void st_shared_v4_if(bool p, uint32_t addr, float4 v)
         "r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
         : "memory");
 }
+__device__ __forceinline__ void st_shared_v2_if(bool p, uint32_t addr, float2 v) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q st.shared.v2.f32 [%1], {%2, %3};\n\t}" ::"r"((uint32_t)p),
+                 "r"(addr), "f"(v.x), "f"(v.y)
+                 : "memory");
+}
 __device__ __forceinline__ void st_shared_u32_if(bool p, uint32_t addr, uint32_t v) {
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q st.shared.u32 [%1], %2;\n\t}" ::"r"((uint32_t)p),
                  "r"(addr), "r"(v)
