@@ -61,19 +61,19 @@ constexpr uint32_t kFtCols = 2 * kFtNP; // TMEM columns: two CTAs per SM
 struct FtSmem {
     float *Bhi, *Blo;   // [2 kFtNP rows][2 kFtB] canonical each
     float *Xhi, *Xlo;   // [kFtNP rows][2 kFtB] canonical each
-    float2 *Yn;         // [kFtB][kFtB]: the pivot rows in the next panel's columns (the row warps')
+    float2 *Yn;         // [kFtB][kFtYld]: the pivot rows in the next panel's columns (the row warps')
     float2 *Y;          // [2][kFtB][kFtYld]: ... in one panel's columns, by turns (the helpers')
     float2 *wrow;       // [2][4][kFtB]
     uint32_t *ckey;     // [2][4]: each warp's pivot key, by step parity
     int *rho, *kap;     // [2][kFtNP] each: the frame, double-buffered by line
     int *kapinv, *perm, *stepof;   // [kFtNP]; stepof[t]: the step that pivoted row t
-    uint64_t *x_ready, *rest_done, *fin;
+    uint64_t *x_ready, *next_done, *rest_done, *fin;
     uint32_t *tslot;
 };
 
-constexpr size_t kFtSmemBytes = 2 * sizeof(float) * 3 * kFtNP * 2 * kFtB + sizeof(float2) * kFtB * (kFtB + 2 * kFtYld) +
+constexpr size_t kFtSmemBytes = 2 * sizeof(float) * 3 * kFtNP * 2 * kFtB + sizeof(float2) * 3 * kFtB * kFtYld +
                                 sizeof(float2) * 2 * 4 * kFtB + sizeof(uint32_t) * 8 + sizeof(int) * 7 * kFtNP +
-                                3 * sizeof(uint64_t) + 16;
+                                4 * sizeof(uint64_t) + 16;
 
 __device__ __forceinline__ FtSmem ft_carve(unsigned char *raw) {
     FtSmem s;
@@ -82,7 +82,7 @@ __device__ __forceinline__ FtSmem ft_carve(unsigned char *raw) {
     s.Xhi = s.Blo + 2 * kFtNP * 2 * kFtB;
     s.Xlo = s.Xhi + kFtNP * 2 * kFtB;
     s.Yn = reinterpret_cast<float2 *>(s.Xlo + kFtNP * 2 * kFtB);
-    s.Y = s.Yn + kFtB * kFtB;
+    s.Y = s.Yn + kFtB * kFtYld;
     s.wrow = s.Y + 2 * kFtB * kFtYld;
     s.ckey = reinterpret_cast<uint32_t *>(s.wrow + 2 * 4 * kFtB);
     s.rho = reinterpret_cast<int *>(s.ckey + 8);
@@ -91,9 +91,10 @@ __device__ __forceinline__ FtSmem ft_carve(unsigned char *raw) {
     s.perm = s.kapinv + kFtNP;
     s.stepof = s.perm + kFtNP;
     s.x_ready = reinterpret_cast<uint64_t *>(s.stepof + kFtNP);   // (every part a multiple of 16 bytes)
-    s.rest_done = s.x_ready + 1;
-    s.fin = s.x_ready + 2;
-    s.tslot = reinterpret_cast<uint32_t *>(s.x_ready + 3);
+    s.next_done = s.x_ready + 1;
+    s.rest_done = s.x_ready + 2;
+    s.fin = s.x_ready + 3;
+    s.tslot = reinterpret_cast<uint32_t *>(s.x_ready + 4);
     return s;
 }
 
@@ -123,6 +124,7 @@ __global__ void __launch_bounds__(kFtThreads, 2) factor_tc_kernel(FtK a) {
     }
     if (tid == 0) {
         mbar_init(sm.x_ready, kFtRowWarps);
+        mbar_init(sm.next_done, 1);
         mbar_init(sm.rest_done, 1);
         mbar_init(sm.fin, 1);
         fence_mbar_init_cluster();
@@ -163,25 +165,26 @@ __global__ void __launch_bounds__(kFtThreads, 2) factor_tc_kernel(FtK a) {
         tc_fence_after();
     };
 
+    const uint32_t bhi = smem_u32(sm.Bhi), blo = smem_u32(sm.Blo), xhi = smem_u32(sm.Xhi), xlo = smem_u32(sm.Xlo);
+    // D[:, c0 + [0, len)) += X B[c0 + [0, len), :]^T, 3xTF32
+    auto issue = [&](int c0, int len) {
+        if (len <= 0) return;
+        const uint32_t sbo = (uint32_t)(2 * kFtB / 4) * 128u, idesc = umma_idesc_tf32(len);
+        const uint32_t boff = (uint32_t)(c0 / 8) * sbo, d = tmem + (uint32_t)c0;
+#pragma unroll
+        for (int ks = 0; ks < 2 * kFtB / 8; ks++) {
+            const uint32_t koff = (uint32_t)ks * 256u;   // 8 K = two core matrices of 128 B
+            const uint64_t dh = umma_desc(bhi + boff + koff, 128, sbo), dl = umma_desc(blo + boff + koff, 128, sbo);
+            const uint64_t xh = umma_desc(xhi + koff, 128, sbo), xl = umma_desc(xlo + koff, 128, sbo);
+            umma_tf32(d, xh, dh, idesc, 1u);
+            umma_tf32(d, xh, dl, idesc, 1u);
+            umma_tf32(d, xl, dh, idesc, 1u);
+        }
+    };
+
     if (helper) {
         // ------------------------------------------------------- helpers
         const bool issuer = warp == kFtRowWarps && lane == 0;
-        const uint32_t bhi = smem_u32(sm.Bhi), blo = smem_u32(sm.Blo), xhi = smem_u32(sm.Xhi), xlo = smem_u32(sm.Xlo);
-        // D[:, c0 + [0, len)) += X B[c0 + [0, len), :]^T, 3xTF32
-        auto issue = [&](int c0, int len) {
-            if (len <= 0) return;
-            const uint32_t sbo = (uint32_t)(2 * kFtB / 4) * 128u, idesc = umma_idesc_tf32(len);
-            const uint32_t boff = (uint32_t)(c0 / 8) * sbo, d = tmem + (uint32_t)c0;
-#pragma unroll
-            for (int ks = 0; ks < 2 * kFtB / 8; ks++) {
-                const uint32_t koff = (uint32_t)ks * 256u;   // 8 K = two core matrices of 128 B
-                const uint64_t dh = umma_desc(bhi + boff + koff, 128, sbo), dl = umma_desc(blo + boff + koff, 128, sbo);
-                const uint64_t xh = umma_desc(xhi + koff, 128, sbo), xl = umma_desc(xlo + koff, 128, sbo);
-                umma_tf32(d, xh, dh, idesc, 1u);
-                umma_tf32(d, xh, dl, idesc, 1u);
-                umma_tf32(d, xl, dh, idesc, 1u);
-            }
-        };
         uint32_t ph_x = 0, ph_rest = 0;
         for (int ls = 0; ls < lines; ls++) {
             for (int p = 0; p < npan; p++) {
@@ -245,7 +248,7 @@ __global__ void __launch_bounds__(kFtThreads, 2) factor_tc_kernel(FtK a) {
         __syncwarp();
     } else {
         // ----------------------------------------------------- row threads
-        uint32_t ph_rest = 0;
+        uint32_t ph_rest = 0, ph_next = 0;
         for (int ls = 0; ls < lines; ls++) {
             bool used = false;
             int my_step = -1;
@@ -408,29 +411,34 @@ __global__ void __launch_bounds__(kFtThreads, 2) factor_tc_kernel(FtK a) {
                 tc_fence_before();
                 mbar_arrive_warp(sm.x_ready);
                 if (!next) break;
-                // ---- the next panel after this one: M + X M[R, :], in FP32
+                // ---- the next panel's columns: their pivot entries, B (one unit per
+                // thread) and GEMM by the row warps, which wait for nothing else
                 {
-                    const uint32_t yrow = smem_u32(sm.Yn + (pivp ? my_step - k0 : 0) * kFtB);
+                    const uint32_t yrow = smem_u32(sm.Yn + (pivp ? my_step - k0 : 0) * kFtYld);
 #pragma unroll
                     for (int e = 0; e < 8; e++)
                         st_shared_v4_if(pivp, yrow + 16u * (uint32_t)e,
                                         make_float4(m[4 * e], m[4 * e + 1], m[4 * e + 2], m[4 * e + 3]));
                 }
                 ft_row_barrier();
-#pragma unroll
-                for (int k = 0; k < kFtB; k++) {
-                    const float4 *y = reinterpret_cast<const float4 *>(sm.Yn + k * kFtB);
-#pragma unroll
-                    for (int e = 0; e < kFtB / 2; e++) {
-                        const float4 q = y[e];
-                        const float2 m0 = cfma(P[k], make_float2(q.x, q.y), make_float2(m[4 * e], m[4 * e + 1]));
-                        const float2 m1 = cfma(P[k], make_float2(q.z, q.w), make_float2(m[4 * e + 2], m[4 * e + 3]));
-                        m[4 * e] = m0.x;
-                        m[4 * e + 1] = m0.y;
-                        m[4 * e + 2] = m1.x;
-                        m[4 * e + 3] = m1.y;
-                    }
+                {
+                    const float2 *y = sm.Yn + 2 * ((t >> 2) & 7) * kFtYld + (t >> 5) * 4 + (t & 3);
+                    ft_put_b(sm.Bhi, sm.Blo, 128 * (p + 1) + t, y[0], y[kFtYld]);
                 }
+                fence_proxy_async_smem();
+                tc_fence_before();
+                ft_row_barrier();
+                tc_fence_after();
+                if (t == 0) {
+                    issue(2 * kFtB * (p + 1), 2 * kFtB);
+                    umma_commit(sm.next_done);
+                }
+                __syncwarp();
+                wait(sm.next_done, ph_next);
+                ph_next ^= 1u;
+                tc_fence_after();
+                tmem_ld32_nowait(trow + (uint32_t)(32 * (p + 1)), m);
+                tmem_wait_ld(m);
 #pragma unroll
                 for (int e = 0; e < kFtB; e++) P[e] = make_float2(m[2 * e], m[2 * e + 1]);
             }
