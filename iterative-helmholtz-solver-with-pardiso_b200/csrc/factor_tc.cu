@@ -19,15 +19,17 @@
 // at (r_k, k)).  The panel's steps run on CUDA cores with the panel in
 // registers (thread i = row i).
 //
-// Look-ahead.  The chain of pivot steps bounds the factor, so the row warps
-// do nothing but what the next step needs: they form the next panel's columns
-// themselves (FP32, X from their registers, the 16 x 16 pivot entries from
-// shared memory) and run its steps, while four helper warps gather the pivot
-// rows' other columns, build the GEMM's operand and issue X M[R, :] for every
-// column outside panels p and p + 1 (M = 128 rows, K = 32 real), accumulated
-// into the block in TMEM.  The row warps wait for that GEMM only before they
-// write the next X.  A panel's own columns, which the product does not
-// describe, are rewritten from registers.
+// Look-ahead.  The chain of pivot steps bounds the factor, so the four row warps
+// do only what the next step needs: they gather the pivot rows' entries in the
+// next panel's columns, build their B, issue their GEMM and run that panel's
+// steps.  Four helper warps meanwhile gather the other columns (a panel's at a
+// time through two small buffers), build B and issue X M[R, :] for every column
+// outside panels p and p + 1 (M = 128 rows, K = 32 real), accumulated into the
+// block in TMEM, which the row warps wait for only before they write the next X.
+// A panel's own columns, which the product does not describe, are rewritten
+// from registers.  All columns by the same 3xTF32 product: the next panel's in
+// FP32 was no slower, but raised the preconditioner's error at 96^3 from 2.16e-6
+// to 2.98e-6.
 //
 // Frames.  The block is never unscrambled: physical row t of M holds logical
 // row rho[t], physical column q logical column kap[q], and the next line's S
@@ -42,6 +44,10 @@
 //     in the next panel's columns; the per-warp pivot keys and rows (double-
 //     buffered by step parity, so one barrier per step); the frame and the
 //     pivot order.  Half of TMEM and of shared memory: two CTAs share an SM.
+// Two chains on an SM hide each other's latencies, which is why X is in shared
+// memory and not in TMEM.  In ms, one CTA per SM with a whole GEMM after each
+// panel and the block unscrambled through shared memory -> look-ahead, frames and
+// two CTAs per SM: 40^3 0.60 -> 0.38, 96^3 5.13 -> 2.95, 128^3 9.66 -> 5.85.
 // Every wait is bounded: on expiry bit 1 of *status is set and the kernel
 // runs on without waiting (results invalid), waits (bounded) for its MMAs,
 // frees its TMEM and returns.  A zero pivot, or a column without a finite

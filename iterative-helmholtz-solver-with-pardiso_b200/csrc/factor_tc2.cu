@@ -33,7 +33,7 @@
 // alternating by step parity, one CTA barrier per step.  After the steps
 // each CTA keeps X and the panel of its own rows, and the panel's pivot
 // rows (their other columns live in their owner's TMEM) are exchanged the
-// same way as the panel entries.  Two exchanges between the CTAs per panel.
+// same way as the panel entries.
 //
 // Frames.  The block is never unscrambled.  Physical row g of M holds
 // logical row rho[g], physical column q logical column kap[q].  In-place
@@ -47,12 +47,21 @@
 // G^T[kap'[q]][rho'[g]] = M[g][q] (the 8-byte stores of a warp scatter
 // within one row of G^T and merge in L2).
 //
-// Look-ahead.  After panel p's pivot rows are in place, the MMA warp first
-// updates the next panel's 16 columns (commit: next_ready), then every other
-// column outside panels p and p+1 (commit: rest_done).  The row threads run
-// panel p+1's pivot steps as soon as next_ready arrives; rest_done is waited
-// for only before panel p+1's X and pivot rows are written, so the trailing
-// GEMM runs under the next panel's pivot chain.
+// Look-ahead.  The chain of pivot steps bounds the factor, so the four row
+// warps do only what the next step needs: after panel p's steps they exchange
+// its pivot rows in the next panel's 16 columns, build those columns' B and,
+// when their GEMM is done (next_ready), run panel p+1's steps.  Four helper
+// warps meanwhile exchange the pivot rows' other columns, build their B and
+// issue the GEMM of every column outside panels p and p+1 (rest_done), which the
+// row warps wait for only before they write panel p+1's X.  A finished line is
+// written, and the next one formed, by all eight warps.
+//
+// 200 x 200 x 74 in ms: the row warps alone, with branches 39.7; steps without
+// branches 36.9, 1 / pivot before the barrier 35.8, helpers 32.3, a line's
+// entries by selects and predicated stores 30.6, the first block by all warps
+// 29.6.  A step is 725 cycles: store the candidate 130, barrier 25, keys 105, the
+// row 85, the next column's update and reduction 180, the other columns 160.
+// Eight row warps of one row each took 36.9 -> 38.7: more warps at each barrier.
 //
 // Every wait is bounded: on expiry bit 1 of *status is set and the kernel
 // runs on without waiting (results invalid), waits (bounded) for its MMAs,
@@ -132,7 +141,7 @@ __device__ __forceinline__ void st_cluster_v4f32(uint32_t addr, float4 v) {
 }
 
 // MID: the middle lines (one launch) instead of the halves: a kernel of its
-// own, so that the halves' loop does not carry the middle line\'s code
+// own, so that the halves' loop does not carry the middle line's code
 template <bool MID>
 __global__ void __launch_bounds__(kFtThreads, 1) factor_tc2_kernel(FtK a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
