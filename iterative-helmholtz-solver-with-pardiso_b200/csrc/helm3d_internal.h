@@ -122,7 +122,6 @@ struct SweepArgs {
     const void *cmy, *cpy;
     void *planes;             // PlaneLayout with R right-hand sides
     int R;
-    int rstride = 0;          // right-hand sides of the planes, where they hold more than this launch's (0: R)
     const void *dxy;          // null: S^{-1}; else S^{-H} with the [2][ny][n] alpha_x alpha_y table
     int *status;              // device flag: bit 2 = a bounded wait expired
     int stage_kb = 32;        // bulk-copy stage of G^T rows (KB, about)

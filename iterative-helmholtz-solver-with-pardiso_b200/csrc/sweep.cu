@@ -36,7 +36,7 @@ namespace h3d {
 
 template <typename R> struct SweepK {
     int n, ny, ldg, nrhs;
-    int rstride;         // right-hand sides of the planes, nrhs of which from planes on are this launch's
+    int groups, gsize;   // the right-hand sides in groups of gsize, a cluster of its own for each (kz, group)
     const cplx<R> *Gt;
     const cplx<R> *cmy, *cpy;
     cplx<R> *planes;
@@ -153,8 +153,9 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) sweep_kernel(SweepK<R> a) {
     typedef cplx<R> Cx;
     constexpr int RW = 32 / G;  // rows of y per warp
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    const int n = a.n, ldg = a.ldg, Rn = a.nrhs, Rs = a.rstride;
-    const int kz = blockIdx.x >> 1;
+    const int n = a.n, ldg = a.ldg, Rs = a.nrhs;
+    const int kz = (blockIdx.x >> 1) / a.groups, rg = (blockIdx.x >> 1) % a.groups * a.gsize;
+    const int Rn = min(a.gsize, Rs - rg);   // this cluster's right-hand sides, rg, rg + 1, ...
     if (a.kzslot && a.kzslot[kz] >= 0) return;   // a skipped mode (kz_skip_ratio), in both CTAs
     const uint32_t rank = blockIdx.x & 1u, peer = rank ^ 1u;   // the rank in the cluster of two
     const HalfChain hc(a.ny, (int)rank);
@@ -165,7 +166,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) sweep_kernel(SweepK<R> a) {
     uint64_t *empty = full + a.nstage;
     uint64_t *never = empty + a.nstage;         // no thread arrives on it
     uint64_t *met = never + 1, *read = never + 2;   // the peer's consumer warps arrive on them
-    Cx *P = a.planes + (long)kz * a.ny * Rs * n;  // line j, rhs r, row i at ((j*Rs + r)*n + i)
+    Cx *P = a.planes + ((long)kz * a.ny * Rs + rg) * n;  // line j, rhs rg + r, row i at ((j*Rs + r)*n + i)
     const int cpl = (n + a.rows_per_stage - 1) / a.rows_per_stage;
 
     if (threadIdx.x == 0) {
@@ -383,7 +384,7 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 // G^T; the G partial sums of a row meet by halving, which leaves each group g
 // the right-hand sides from g RR / G on to finish.  Everything else as in
 // sweep_kernel.  Sixteen sources, one row per thread -> this kernel: 32^3 84 ->
-// 50 us, 64^3 291 -> 197, 96^3 1425 -> 1032, 128^3 2461 -> 2030, 200 x 128 x 60
+// 50 us, 64^3 291 -> 197, 96^3 1425 -> 830, 128^3 2461 -> 2030, 200 x 128 x 60
 // 3080 -> 2880; eight: 64^3 141 -> 122, 96^3 765 -> 567, 128^3 1409 -> 1120.
 // elements between the rows of v: the G rows that a warp reads at once lie in
 // banks of their own
@@ -396,8 +397,9 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) sweep_batch_kernel(SweepK<fl
     constexpr int VS = RR + kBatchPad;                       // row stride of v
     constexpr int FS = RR >= G ? RR / G : 1;         // right-hand sides a thread finishes
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    const int n = a.n, ldg = a.ldg, Rn = a.nrhs, Rs = a.rstride;
-    const int kz = blockIdx.x >> 1;
+    const int n = a.n, ldg = a.ldg, Rs = a.nrhs;
+    const int kz = (blockIdx.x >> 1) / a.groups, rg = (blockIdx.x >> 1) % a.groups * a.gsize;
+    const int Rn = min(a.gsize, Rs - rg);   // this cluster's right-hand sides, rg, rg + 1, ...
     if (a.kzslot && a.kzslot[kz] >= 0) return;   // a skipped mode (kz_skip_ratio), in both CTAs
     const uint32_t rank = blockIdx.x & 1u, peer = rank ^ 1u;   // the rank in the cluster of two
     const HalfChain hc(a.ny, (int)rank);
@@ -408,7 +410,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) sweep_batch_kernel(SweepK<fl
     uint64_t *empty = full + a.nstage;
     uint64_t *never = empty + a.nstage;         // no thread arrives on it
     uint64_t *met = never + 1, *read = never + 2;   // the peer's consumer warps arrive on them
-    Cx *P = a.planes + (long)kz * a.ny * Rs * n;  // line j, rhs r, row i at ((j*Rs + r)*n + i)
+    Cx *P = a.planes + ((long)kz * a.ny * Rs + rg) * n;  // line j, rhs rg + r, row i at ((j*Rs + r)*n + i)
     const int cpl = (n + a.rows_per_stage - 1) / a.rows_per_stage;
 
     if (threadIdx.x == 0) {
@@ -603,16 +605,18 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) sweep_batch_kernel(SweepK<fl
 }
 
 // A launch of kern: CW consumer warps, rows of v of vs elements; even > 0: the
-// stages of a line are the same multiple of that many rows.
+// stages of a line are the same multiple of that many rows; the right-hand
+// sides in so many groups.
 template <typename R, int CW>
-static int sweep_go(void (*kern)(SweepK<R>), int vs, int even, const SweepArgs &sa, cudaStream_t st) {
+static int sweep_go(void (*kern)(SweepK<R>), int vs, int even, int groups, const SweepArgs &sa, cudaStream_t st) {
     typedef cplx<R> Cx;
     SweepK<R> k;
     k.n = sa.n;
     k.ny = sa.ny;
     k.ldg = sa.ldg;
     k.nrhs = sa.R;
-    k.rstride = sa.rstride ? sa.rstride : sa.R;
+    k.groups = groups;
+    k.gsize = (sa.R + groups - 1) / groups;
     k.Gt = (const Cx *)sa.Gt;
     k.cmy = (const Cx *)sa.cmy;
     k.cpy = (const Cx *)sa.cpy;
@@ -650,18 +654,25 @@ static int sweep_go(void (*kern)(SweepK<R>), int vs, int even, const SweepArgs &
     if (nst < 2) return HELM3D_ERR_ARG;
     k.nstage = nst;
     const size_t smem = (size_t)nst * k.stage_bytes + vbytes + (2 * nst + 3) * sizeof(uint64_t);
-    return launch_pairs(kern, sa.nz, (CW + 1) * 32, smem, k, st);
+    return launch_pairs(kern, sa.nz * groups, (CW + 1) * 32, smem, k, st);
 }
 
-template <typename R, int G, int RR, bool ADJ, int CW> static int sweep_impl(const SweepArgs &sa, cudaStream_t st) {
-    return sweep_go<R, CW>(sweep_kernel<R, G, RR, ADJ, CW>, RR, 0, sa, st);
+template <typename R, int G, int RR, bool ADJ, int CW> static int sweep_impl(const SweepArgs &sa, cudaStream_t st, int groups = 1) {
+    return sweep_go<R, CW>(sweep_kernel<R, G, RR, ADJ, CW>, RR, 0, groups, sa, st);
 }
 
-// complex64 batches: 64 / G rows per warp
+// complex64 batches: 64 / G rows per warp.  More than 8 right-hand sides as two
+// groups where that fills the last wave of CTAs (one to an SM above 64 rows): a
+// group of 8 takes 0.55 of the time of 16 (96 x 96 x 64, one wave: 293 of 526
+// us), so 96^3 x 16 as three waves of 8 instead of two of 16: 1032 ->
+// 830 us (128^3, 4 waves of 8 for 2 of 16, stays).
 template <int G, bool ADJ, int CW> static int sweep_batch(const SweepArgs &sa, cudaStream_t st) {
-    if (sa.R <= 4) return sweep_go<float, CW>(sweep_batch_kernel<G, 4, ADJ, CW>, 4 + kBatchPad, G, sa, st);
-    if (sa.R <= 8) return sweep_go<float, CW>(sweep_batch_kernel<G, 8, ADJ, CW>, 8 + kBatchPad, G, sa, st);
-    return sweep_go<float, CW>(sweep_batch_kernel<G, 16, ADJ, CW>, 16 + kBatchPad, G, sa, st);
+    if (sa.R <= 4) return sweep_go<float, CW>(sweep_batch_kernel<G, 4, ADJ, CW>, 4 + kBatchPad, G, 1, sa, st);
+    if (sa.R <= 8) return sweep_go<float, CW>(sweep_batch_kernel<G, 8, ADJ, CW>, 8 + kBatchPad, G, 1, sa, st);
+    const int sms = device_info().sm_count, one = (2 * sa.nz + sms - 1) / sms, two = (4 * sa.nz + sms - 1) / sms;
+    if (sa.n > 64 && 11 * two < 20 * one)
+        return sweep_go<float, CW>(sweep_batch_kernel<G, 8, ADJ, CW>, 8 + kBatchPad, G, 2, sa, st);
+    return sweep_go<float, CW>(sweep_batch_kernel<G, 16, ADJ, CW>, 16 + kBatchPad, G, 1, sa, st);
 }
 
 // The split of a line over the consumer warps: 32 / G rows per warp, CW warps.
@@ -675,15 +686,8 @@ template <typename R, bool ADJ, int G1, int CW1, int G2> static int sweep_rr(con
     if constexpr (sizeof(R) == 8) {
         if (sa.R <= 8) return sweep_impl<R, G2, 8, ADJ, 8>(sa, s);
         // sums of 16 right-hand sides do not fit the registers (spilled, 64^3:
-        // 957 us; two launches 2 x 269, although they read G twice)
-        SweepArgs h = sa;
-        h.rstride = sa.R;
-        h.R = 8;
-        const int rc = sweep_impl<R, G2, 8, ADJ, 8>(h, s);
-        if (rc) return rc;
-        h.R = sa.R - 8;
-        h.planes = (cplx<R> *)sa.planes + 8 * (long)sa.n;
-        return sweep_rr<R, ADJ, G1, CW1, G2>(h, s);
+        // 957 us; two groups of 8, although they read G twice, 530)
+        return sweep_impl<R, G2, 8, ADJ, 8>(sa, s, 2);
     }
     return HELM3D_ERR_ARG;   // (complex64 batches are sweep_batch's)
 }

@@ -1,7 +1,8 @@
 """Batches of right-hand sides in the block sweep, at the edges of its splits:
 rows per warp and warps per line (8, 16 or 32 rows; odd counts, whose last
 thread owns one row), one and several stages to a line, right-hand sides below,
-at and above the padded counts 4, 8 and 16 (complex128: two launches above 8),
+at and above the padded counts 4, 8 and 16 (above 8 in two groups: complex128, and
+complex64 where that fills the last wave),
 forward and adjoint, against the FP64 oracle (needs a B200).  Tolerances as in
 test_gpu_parity: 1e-9 (complex128 preconditioner), 5e-5 (complex64)."""
 import numpy as np
@@ -13,11 +14,7 @@ from oracle import mode_n
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nx,batches", [(5, (3, 16)), (31, (5, 9)), (33, (4, 8)), (64, (5, 16)), (65, (3, 8)), (96, (16,)),
-                                        (97, (4, 9)), (128, (16,)), (129, (3, 16)), (193, (8,)), (240, (9,)), (255, (5, 16))])
-@pytest.mark.parametrize("prec", [0, 1])
-def test_batches_match_the_oracle(nx, batches, prec):
-    ny, nz = 3, 4
+def check(nx, ny, nz, batches, prec):
     p = small_problem(nx, ny, nz, pml=1, seed=nx)
     on = mode_n.setup(p, beta_prec=0.25)
     X = np.stack([rand_c(p.shape, seed=300 + r) for r in range(max(batches))])
@@ -31,3 +28,15 @@ def test_batches_match_the_oracle(nx, batches, prec):
             assert rel(Y[r], ref[r]) < tol, (k, r)
             assert rel(Yh[r], refh[r]) < tol, (k, r)
     s.close()
+
+
+@pytest.mark.parametrize("nx,batches", [(5, (3, 16)), (31, (5, 9)), (33, (4, 8)), (64, (5, 16)), (65, (3, 8)), (96, (16,)),
+                                        (97, (4, 9)), (128, (16,)), (129, (3, 16)), (193, (8,)), (240, (9,)), (255, (5, 16))])
+@pytest.mark.parametrize("prec", [0, 1])
+def test_batches_match_the_oracle(nx, batches, prec):
+    check(nx, 3, 4, batches, prec)
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+def test_groups_of_right_hand_sides(prec):
+    check(70, 3, 80, (9, 16), prec)
