@@ -546,6 +546,11 @@ __global__ void base2d_kernel(const double *__restrict__ s2, int nz, long plane,
 
 static inline bool ok() { return cudaGetLastError() == cudaSuccess; }
 
+// Dynamic shared memory above this is opted in to: with the kernel's own (up to
+// 16 KB of sums in dots_kernel, 144 bytes in the others) it may pass the 48 KB
+// that a launch gets without.
+constexpr size_t kSmemOptIn = 24 * 1024;
+
 static int grid_for(long N, int R = 1) {
     const long b = (N + kRedThreads - 1) / kRedThreads;
     const long cap = (4L * device_info().sm_count + R - 1) / R;
@@ -562,7 +567,7 @@ static int go_dots(const DotsK &a, int items, bool two, const Reduce &red, int R
     if (items * (two ? 2 : 1) > red.cap || R > red.rmax) return HELM3D_ERR_ARG;
     const size_t smem = sizeof(double2) * scratch;
     auto go = [&](void (*kern)(DotsK), int ul) -> int {
-        if (smem > 24 * 1024 && !smem_limit_max(kern, smem)) return HELM3D_ERR_CUDA;
+        if (smem > kSmemOptIn && !smem_limit_max(kern, smem)) return HELM3D_ERR_CUDA;
         kern<<<dim3(pass_blocks(red, a.N, 32 * ul * kRedWarps), R), kRedThreads, smem, s>>>(a);
         return ok() ? HELM3D_OK : HELM3D_ERR_CUDA;
     };
@@ -618,7 +623,7 @@ int launch_cycle_end(const VecBatch &V, long ldv, const ArnState &arn, bool tail
     const size_t scratch = arn_scratch(arn.m + 1) + kBacksubTri * kBacksubTri;
     if (!tail) {
         const size_t smem = sizeof(double2) * scratch;
-        if (smem > 48 * 1024 && !smem_limit_max(backsub_kernel, smem)) return HELM3D_ERR_CUDA;
+        if (smem > kSmemOptIn && !smem_limit_max(backsub_kernel, smem)) return HELM3D_ERR_CUDA;
         backsub_kernel<<<R, kRedThreads, smem, s>>>(arn, red.tickets + red.rmax);
         return ok() ? HELM3D_OK : HELM3D_ERR_CUDA;
     }
@@ -668,7 +673,7 @@ int launch_update(const VecBatch &V, long ldv, const ScaleBatch &vs, int nv, con
     }
     const int nb = post ? pass_blocks(red, N, kRedThreads) : grid_for(N, R);
     const size_t smem = sizeof(double2) * (arn ? arn_scratch(nv) : nv > 0 ? (size_t)nv : 1);
-    if (smem > 48 * 1024 && !smem_limit_max(update_kernel, smem)) return HELM3D_ERR_CUDA;
+    if (smem > kSmemOptIn && !smem_limit_max(update_kernel, smem)) return HELM3D_ERR_CUDA;
     update_kernel<<<dim3(nb, R), kRedThreads, smem, s>>>(a);
     return ok() ? HELM3D_OK : HELM3D_ERR_CUDA;
 }
