@@ -488,8 +488,10 @@ static int cycle_tail(helm3d_ctx *c, int m, int B, bool adjoint, const ArnState 
 // node j holding step j, then the tail.  Step 0 always runs; the bookkeeping
 // kernel of step j sets the condition of step j + 1.  The chain's kernels
 // are recorded on c's launch count per step (per_step) and at the tail.
-// Every allocation happens before the captures.
-static bool add_cycle(cudaGraph_t G, helm3d_ctx *c, int m, int B, bool adjoint, long long &per_step,
+// Every allocation happens before the captures.  A capture that CUDA
+// invalidates takes the graph it was recorded into with it: G is then null, not
+// to be destroyed again.
+static bool add_cycle(cudaGraph_t &G, helm3d_ctx *c, int m, int B, bool adjoint, long long &per_step,
                       long long &tail) {
     if (ensure_planes(c, B)) return false;
     const ArnState a = arn_state(c, m, B);
@@ -504,6 +506,17 @@ static bool add_cycle(cudaGraph_t G, helm3d_ctx *c, int m, int B, bool adjoint, 
     c->stream = cap;
     c->prof = false;
     bool ok = true;
+    // HELM3D_TEST_FAIL_CAPTURE: a call that captures do not allow, so that
+    // they are invalidated (tests of the way back to launched steps)
+    const char *te = std::getenv("HELM3D_TEST_FAIL_CAPTURE");
+    const bool fail_test = te && *te && *te != '0';
+    auto end_capture = [&]() {
+        if (fail_test) cudaStreamSynchronize(cap);
+        cudaGraph_t out = nullptr;
+        if (cudaStreamEndCapture(cap, &out) == cudaSuccess) return true;
+        G = nullptr;
+        return false;
+    };
     std::vector<cudaGraphConditionalHandle> hs(m);
     for (int j = 0; ok && j < m; j++)
         ok = cudaGraphConditionalHandleCreate(&hs[j], G, j == 0 ? 1u : 0u, cudaGraphCondAssignDefault) == cudaSuccess;
@@ -523,8 +536,7 @@ static bool add_cycle(cudaGraph_t G, helm3d_ctx *c, int m, int B, bool adjoint, 
         if (!ok) break;
         const long long l0 = c->launches;
         const int rc = arnoldi_step(c, m, B, j, adjoint, a, j + 1 < m, j + 1 < m ? hs[j + 1] : 0);
-        cudaGraph_t out = nullptr;
-        ok = cudaStreamEndCapture(cap, &out) == cudaSuccess && rc == HELM3D_OK;
+        ok = end_capture() && rc == HELM3D_OK;
         per_step = c->launches - l0;
         prev = node;
     }
@@ -533,8 +545,7 @@ static bool add_cycle(cudaGraph_t G, helm3d_ctx *c, int m, int B, bool adjoint, 
         if (ok) {
             const long long l0 = c->launches;
             const int rc = cycle_tail(c, m, B, adjoint, a);
-            cudaGraph_t out = nullptr;
-            ok = cudaStreamEndCapture(cap, &out) == cudaSuccess && rc == HELM3D_OK;
+            ok = end_capture() && rc == HELM3D_OK;
             tail = c->launches - l0;
         }
     }
@@ -1172,10 +1183,10 @@ int fgmres_group(helm3d_ctx *const *cs, int n, const double2 *const *f, double2 
             helm3d_ctx *c = cs[i];
             const int g1 = run.graphs_usable() ? cycle_graph(c, run.m, run.B, false) : -1;
             if (g1 >= 0) {
-                    RC(cuda_check(c, cudaGraphLaunch(c->graphs[g1].exec, c->stream), "cycle graph"));
+                RC(cuda_check(c, cudaGraphLaunch(c->graphs[g1].exec, c->stream), "cycle graph"));
                 RC(run.cycle_end_device(c->graphs[g1].kernels_per_step, c->graphs[g1].tail_kernels));
             } else if (lowsync(c)) {
-                    RC(run.run_steps());
+                RC(run.run_steps());
                 RC(run.cycle_end_device(-1, 0));
             } else {
                 RC(run.run_host_cycle());
