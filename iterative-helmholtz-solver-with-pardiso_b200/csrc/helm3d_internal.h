@@ -102,7 +102,9 @@ struct FactorArgs {
     const int *kzslot = nullptr;   // [nz]: >= 0 for a skipped mode (not factored), or null
     int middle = 0;           // set by launch_factor: 0 the two halves of every kz, 1 the middle lines (chain.cuh)
 };
-// variant: one of the factor_variants(c64, n) launch shapes (0: the default)
+// variant: one of the factor_variants(c64, n) launch shapes (0: the default);
+// kFactorLaunches kernels (the halves, the middle lines)
+constexpr int kFactorLaunches = 2;
 int launch_factor(bool c64, const FactorArgs &a, cudaStream_t s, int variant = 0);
 int factor_variants(bool c64, int n);
 // the tensor-core factor (complex64, n <= 128): the last factor variant

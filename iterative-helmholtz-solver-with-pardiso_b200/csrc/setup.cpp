@@ -607,7 +607,7 @@ int ctx_factor(helm3d_ctx *c) {
     } else {
         c->tv_factor = 0;
     }
-    rc = timed(c, HELM3D_K_FACTOR, 1, [&] { return launch_factor(c->c64, a, c->stream, c->tv_factor); });
+    rc = timed(c, HELM3D_K_FACTOR, kFactorLaunches, [&] { return launch_factor(c->c64, a, c->stream, c->tv_factor); });
     if (rc) return set_error(c, rc, std::string("factor launch failed: ") + cudaGetErrorString(cudaGetLastError()));
     // complex64: the blocks' power-of-two scales for the FP16 sweep
     if (c->c64) {
