@@ -344,6 +344,7 @@ int tune_forced(const char *family);
 // z points per thread 8, 1, 2, 4, 6, 12 (1, 2: the register kernel, else blocks in
 // shared memory); source-major (0-5) or source-minor (6-11) grid
 constexpr int kStencilVariants = 12;
+constexpr int kAnyBatch = -1;
 constexpr int kReduceVariants = 3;    // reduction blocks 2, 1, 4 per SM
 constexpr int kUpdateVariants = 2;    // DCGS2 update pass: basis loads one by one, 8 batched
 int stencil_zblock(int v);
@@ -453,7 +454,8 @@ struct helm3d_ctx {
     int tv_factor = 0;
     int tv_sweep[2] = {0, 0};
     int tv_sweep_R[2] = {0, 0};                 // the batch tv_sweep was chosen for (0: none yet, sweep_default)
-    int tv_stencil = -1;                        // -1: not tuned, stencil_default
+    int tv_stencil = 0;
+    int tv_stencil_R = 0;                       // ... for tv_stencil (0: stencil_default; kAnyBatch: forced)
     int tv_update = 0;
     size_t f_cap = 0, u_cap = 0;                // staging capacities (vectors) of d_f, d_u
     double *d_vs = nullptr;

@@ -295,8 +295,14 @@ static StencilArgs stencil_args(helm3d_ctx *c, const VecBatch &x, double xscale,
     a.y = y;
     a.f = f;
     a.R = R;
-    a.zblock = c->tv_stencil >= 0 ? stencil_zblock(c->tv_stencil) : stencil_default(a.nx, a.ny, a.nz, R);
-    a.src_fast = stencil_src_fast(c->tv_stencil);
+    // the forced shape; the tuned one for the batch it was timed with, and for
+    // others to which the default rule gives as many planes per block (what is
+    // left of a batch whose others have retired; not one vector of a grid that
+    // only the batch filled the SMs with); else the default
+    const int dflt = stencil_default(a.nx, a.ny, a.nz, R), tR = c->tv_stencil_R;
+    const bool tuned = tR == kAnyBatch || (tR > 0 && (tR == R || stencil_default(a.nx, a.ny, a.nz, tR) == dflt));
+    a.zblock = tuned ? stencil_zblock(c->tv_stencil) : dflt;
+    a.src_fast = tuned ? stencil_src_fast(c->tv_stencil) : 0;
     return a;
 }
 
@@ -585,7 +591,7 @@ int tune_solve(helm3d_ctx *c, int R, bool adjoint) {
                             std::getenv("HELM3D_FORCE_REDUCE") || std::getenv("HELM3D_FORCE_UPDATE");
     if (!tune_enabled() && !any_forced) {
         c->tv_sweep_R[0] = c->tv_sweep_R[1] = 0;   // sweep_default
-        c->tv_stencil = -1;
+        c->tv_stencil_R = 0;                       // stencil_default
         c->tv_update = 0;
         c->red_blocks = reduce_blocks(0);
         return HELM3D_OK;
@@ -619,6 +625,7 @@ int tune_solve(helm3d_ctx *c, int R, bool adjoint) {
             t.src_fast = stencil_src_fast(v);
             return launch_stencil(t, adjoint, c->stream);
         });
+        c->tv_stencil_R = tune_forced("STENCIL") >= 0 ? kAnyBatch : tune_enabled() ? R : 0;
     }
     // the Gram-Schmidt reduction at mid-cycle depth (read-only on V)
     const int j = std::min(m - 1, std::max(0, m / 2));
