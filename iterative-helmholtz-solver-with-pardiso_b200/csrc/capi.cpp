@@ -58,42 +58,24 @@ struct VecArg {
     }
 };
 
-// the misfit gradient's wavefields given back (synchronizes the stream)
-void release_grad(helm3d_ctx *c) {
-    if (!c->d_grad) return;
-    cudaStreamSynchronize(c->stream);
-    cudaFree(c->d_grad);
-    c->bytes -= c->grad_bytes;
-    c->d_grad = nullptr;
-    c->grad_bytes = 0;
-}
-
 // Right-hand sides per lockstep batch: at most kMaxBatch, and as many as the
 // Krylov bases (V, Z), packed iterates, planes, staging and `extra` further
 // vectors of each fit in 85% of the free device memory (plus what the
-// context's Krylov workspace and, for the gradient's extra vectors, its
-// wavefields already hold).  A kept wavefield buffer that would make a solve's
-// batch smaller is given back.
+// context's Krylov workspace already holds).
 int batch_size(helm3d_ctx *c, int nrhs, bool staged, int extra = 0) {
     const int m = std::max(1, c->opts.restart);
     const size_t vb = sizeof(double2) * (size_t)c->N;
     const size_t per =
         vb * ((size_t)(m + 1) + (c->opts.mode == HELM3D_MODE_N ? m : 0) + 2 + (staged ? 2 : 0) + extra) +
         (c->c64 ? 8 : 16) * (size_t)c->N;
-    for (;;) {
-        size_t fr = 0, tot = 0;
-        if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
-            cudaGetLastError();
-            return 1;
-        }
-        const size_t avail = (size_t)(0.85 * (double)(fr + c->kry_bytes + (extra ? c->grad_bytes : 0)));
-        const int R = (int)std::min<size_t>(avail / std::max<size_t>(per, 1), (size_t)kMaxBatch);
-        if (R < std::min(nrhs, kMaxBatch) && !extra && c->d_grad) {
-            release_grad(c);
-            continue;
-        }
-        return std::max(1, std::min(R, nrhs));
+    size_t fr = 0, tot = 0;
+    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
+        cudaGetLastError();
+        return 1;
     }
+    const size_t avail = (size_t)(0.85 * (double)(fr + c->kry_bytes));
+    const int R = (int)std::min<size_t>(avail / std::max<size_t>(per, 1), (size_t)kMaxBatch);
+    return std::max(1, std::min(R, nrhs));
 }
 
 int validate(const helm3d_grid *g, const helm3d_opts *o) {
@@ -566,7 +548,7 @@ int helm3d_misfit_grad(helm3d_ctx *c, const double *f, int nsrc, const long long
     int rc;
     // receivers: checked on the host, used from the device
     std::vector<long long> hrecv((size_t)nrecv);
-    DevBuf d_recv, d_data, d_grad, d_res;
+    DevBuf d_recv, d_data, d_grad, d_u, d_lam, d_res;
     if (nrecv > 0) {
         if ((rc = cuda_check(c, cudaMemcpy(hrecv.data(), recv, sizeof(long long) * nrecv, cudaMemcpyDefault),
                              "receivers")))
@@ -594,18 +576,14 @@ int helm3d_misfit_grad(helm3d_ctx *c, const double *f, int nsrc, const long long
     }
     if ((rc = cuda_check(c, cudaMemsetAsync(g, 0, sizeof(double) * N, c->stream), "gradient zero"))) return rc;
     const bool fstaged = !is_device_ptr(f);
-    const int B = batch_size(c, nsrc, fstaged, 3);
+    const int B = batch_size(c, nsrc, fstaged, 2);
     const size_t vb = sizeof(double2) * (size_t)N;
-    // the wavefields are kept by the context (allocating and freeing them
-    // took longer than a small gradient's kernels)
-    if (c->grad_bytes < 3 * vb * B) {
-        release_grad(c);
-        if ((rc = cuda_check(c, cudaMalloc(&c->d_grad, 3 * vb * B), "wavefields"))) return rc;
-        c->grad_bytes = 3 * vb * B;
-        c->bytes += c->grad_bytes;
-    }
-    if (nrecv > 0 && (rc = d_res.alloc(c, sizeof(double2) * (size_t)B * nrecv, "receiver residuals"))) return rc;
-    double2 *U = (double2 *)c->d_grad, *Lam = U + (size_t)B * N, *Adj = Lam + (size_t)B * N, *Res = (double2 *)d_res.p;
+    // given back at the end of the call (1.4 of 25.7 ms at 96^3 with 8 sources):
+    // kept by the context, other contexts and the caller would lose them
+    if ((rc = d_u.alloc(c, vb * B, "wavefields")) || (rc = d_lam.alloc(c, vb * B, "adjoint wavefields")) ||
+        (nrecv > 0 && (rc = d_res.alloc(c, sizeof(double2) * (size_t)B * nrecv, "receiver residuals"))))
+        return rc;
+    double2 *U = (double2 *)d_u.p, *Lam = (double2 *)d_lam.p, *Res = (double2 *)d_res.p;
     std::vector<double2> hres((size_t)B * std::max(nrecv, 0));
     const double w2 = c->grid.omega * c->grid.omega;
     double J = 0.0;
@@ -618,14 +596,15 @@ int helm3d_misfit_grad(helm3d_ctx *c, const double *f, int nsrc, const long long
         rc = fgmres(c, fa.dev, U, R, false, st);
         if (rc && rc != HELM3D_ERR_NOT_CONVERGED) return rc;
         if (rc) worst = rc;
-        // receiver residuals P u - d, misfit, adjoint sources P^T (d - P u)
-        if ((rc = cuda_check(c, cudaMemsetAsync(Adj, 0, vb * R, c->stream), "adjoint source zero"))) return rc;
+        // receiver residuals P u - d, misfit, adjoint sources P^T (d - P u), where
+        // the adjoint wavefields go (fgmres copies its right-hand sides first)
+        if ((rc = cuda_check(c, cudaMemsetAsync(Lam, 0, vb * R, c->stream), "adjoint source zero"))) return rc;
         if (nrecv > 0) {
             rc = timed(c, HELM3D_K_KRYLOV, 2, [&] {
                 int r1 = launch_receiver_residual(VecBatch{U, N}, R, (const long long *)d_recv.p, nrecv,
                                                   dd + (size_t)r0 * nrecv, nrecv, Res, c->stream);
                 if (r1) return r1;
-                return launch_adjoint_source(Res, R, (const long long *)d_recv.p, nrecv, -1.0, VecBatch{Adj, N},
+                return launch_adjoint_source(Res, R, (const long long *)d_recv.p, nrecv, -1.0, VecBatch{Lam, N},
                                              c->stream);
             });
             if (rc) return set_error(c, rc, "misfit_grad: receiver kernels");
@@ -637,7 +616,7 @@ int helm3d_misfit_grad(helm3d_ctx *c, const double *f, int nsrc, const long long
             for (size_t q = 0; q < (size_t)R * nrecv; q++) J += 0.5 * (hres[q].x * hres[q].x + hres[q].y * hres[q].y);
         }
         // adjoint wavefields A^H lam = P^T (d - P u)
-        rc = fgmres(c, Adj, Lam, R, true, st);
+        rc = fgmres(c, Lam, Lam, R, true, st);
         if (rc && rc != HELM3D_ERR_NOT_CONVERGED) return rc;
         if (rc) worst = rc;
         rc = timed(c, HELM3D_K_KRYLOV, 1, [&] {
@@ -668,7 +647,6 @@ int helm3d_destroy(helm3d_ctx *c) {
         if (p) cudaFree(p);
     for (auto &g : c->graphs) cudaGraphExecDestroy(g.exec);
     for (auto &g : c->groups) cudaGraphExecDestroy(g.exec);
-    if (c->d_grad) cudaFree(c->d_grad);
     if (c->d_arn) cudaFree(c->d_arn);
     for (auto &e : c->prof_ev) {
         cudaEventDestroy(e.a);

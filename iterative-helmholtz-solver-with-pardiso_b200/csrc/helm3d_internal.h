@@ -466,8 +466,6 @@ struct helm3d_ctx {
     long red_stride = 0;           // partials of one right-hand side
     double2 *d_f = nullptr, *d_u = nullptr, *d_r = nullptr, *d_t = nullptr, *d_t2 = nullptr;
     double2 *d_bic = nullptr;      // BiCGStab vectors
-    void *d_grad = nullptr;        // misfit gradient: wavefields, adjoint wavefields and sources
-    size_t grad_bytes = 0;
     size_t bytes = 0;
 
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -513,6 +511,7 @@ int apply_op_adjoint(helm3d_ctx *c, const VecBatch &x, double xscale, const Scal
 int apply_prec_adjoint(helm3d_ctx *c, const VecBatch &x, double xscale, const ScaleBatch &sc, const VecBatch &y,
                        int R);
 // FGMRES on R right-hand sides f + r N -> u + r N (device), iterated in lockstep
+// (f is copied before u is first written: they may be the same)
 int fgmres(helm3d_ctx *c, const double2 *f, double2 *u, int R, bool adjoint, helm3d_stats *st);
 // FGMRES on n contexts at once (R[i] <= kMaxBatch right-hand sides of device
 // vectors f[i] -> u[i] each): every restart cycle of every context in one
