@@ -58,7 +58,6 @@ template <typename R> struct FactorK {
     const cplx<R> *kz2;  // complex shift of mode kz
     int *status;
     const int *kzslot;   // >= 0: a skipped mode (nothing to do), or null
-    int middle;          // 0: the halves, 1: the middle lines
 };
 
 template <typename R> __device__ __forceinline__ R cabs1(cplx<R> a) { return fabs(a.x) + fabs(a.y); }
@@ -132,7 +131,10 @@ template <typename R, int NP, int NPC> constexpr size_t factor_smem_bytes() {
 
 // MB: CTAs per SM the register budget is planned for (2 lets two kz chains
 // share an SM and hide each other's pivot-step latency)
-template <typename R, int NP, int NW, int CB, int C, int MB>
+// MID: the middle lines (one launch) instead of the halves: a kernel of its own,
+// so that the halves' loop does not carry the middle line's code (with both in one
+// kernel complex128 blocks of up to 32 rows took 146 registers, one CTA per SM)
+template <typename R, int NP, int NW, int CB, int C, int MB, bool MID>
 __global__ void __launch_bounds__(NW * 32, MB) factor_kernel(FactorK<R> a) {
     constexpr int RB = NP / 32;
     constexpr int NPC = NP / C;
@@ -144,11 +146,11 @@ __global__ void __launch_bounds__(NW * 32, MB) factor_kernel(FactorK<R> a) {
 
     const uint32_t rank = (C > 1) ? cluster_ctarank() : 0u;
     const int piece = blockIdx.x / C;
-    const int kz = a.middle ? piece : piece >> 1;
-    const HalfChain hc(a.ny, a.middle ? 0 : piece & 1);
+    const int kz = MID ? piece : piece >> 1;
+    const HalfChain hc(a.ny, MID ? 0 : piece & 1);
     if (a.kzslot && a.kzslot[kz] >= 0) return;   // a skipped mode (kz_skip_ratio): not factored / swept
     const int lane = threadIdx.x & 31, warp = warp_index();
-    const int n = a.n, lines = a.middle ? 1 : hc.K;
+    const int n = a.n, lines = MID ? 1 : hc.K;
     const Cx *cin = hc.half ? a.cpy : a.cmy, *cout = hc.half ? a.cmy : a.cpy;
     const int col0 = (int)rank * NPC + warp * CB;
     bool dead = false;
@@ -168,13 +170,13 @@ __global__ void __launch_bounds__(NW * 32, MB) factor_kernel(FactorK<R> a) {
     long t = 0;  // global pivot step counter (line * n + k)
 
     for (int ls = 0; ls < lines; ls++) {
-        const int line = a.middle ? hc.mid : hc.line(ls);
+        const int line = MID ? hc.mid : hc.line(ls);
         // ---- S_line = D_line - cin[line] cout[prev] G_prev; the middle
         // line: minus both neighbours' terms, their G read from global memory
         {
             const Cx cyd = mkc<R>(-(a.cmy[line].x + a.cpy[line].x), -(a.cmy[line].y + a.cpy[line].y));
             const Cx cc = ls > 0 ? cmul(cin[line], cout[hc.line(ls - 1)]) : mkc<R>(0, 0);
-            const bool lo = a.middle && line > 0, hi = a.middle && line + 1 < a.ny;
+            const bool lo = MID && line > 0, hi = MID && line + 1 < a.ny;
             const Cx clo = lo ? cmul(a.cmy[line], a.cpy[line - 1]) : mkc<R>(0, 0);
             const Cx chi = hi ? cmul(a.cpy[line], a.cmy[line + 1]) : mkc<R>(0, 0);
             const Cx *glo = a.Gt + ((long)kz * a.ny + line - 1) * (long)n * a.ldg;
@@ -193,8 +195,10 @@ __global__ void __launch_bounds__(NW * 32, MB) factor_kernel(FactorK<R> a) {
                             Cx gij = sm.sGT[(warp * CB + b) * NP + i];
                             v = mkc<R>(-(cc.x * gij.x - cc.y * gij.y), -(cc.x * gij.y + cc.y * gij.x));
                         }
-                        if (lo) v = cfms(clo, glo[(long)j * a.ldg + i], v);
-                        if (hi) v = cfms(chi, ghi[(long)j * a.ldg + i], v);
+                        if constexpr (MID) {
+                            if (lo) v = cfms(clo, glo[(long)j * a.ldg + i], v);
+                            if (hi) v = cfms(chi, ghi[(long)j * a.ldg + i], v);
+                        }
                         if (i == j) {
                             Cx d = cadd(cadd(cyd, a.base2d[(long)line * n + i]), kzv);
                             d.x -= a.cmx[i].x + a.cpx[i].x;
@@ -400,7 +404,6 @@ __global__ void __launch_bounds__(NW * 32, MB) factor_kernel(FactorK<R> a) {
 template <typename R, int NP, int NW, int CB, int C, int MB>
 static int launch_cfg(const FactorArgs &fa, cudaStream_t st) {
     FactorK<R> k;
-    k.middle = fa.middle;
     k.n = fa.n;
     k.ny = fa.ny;
     k.nz = fa.nz;
@@ -415,7 +418,7 @@ static int launch_cfg(const FactorArgs &fa, cudaStream_t st) {
     k.kzslot = fa.kzslot;
     k.status = fa.status;
     constexpr size_t smem = factor_smem_bytes<R, NP, NP / C>();
-    auto kern = factor_kernel<R, NP, NW, CB, C, MB>;
+    auto kern = fa.middle ? factor_kernel<R, NP, NW, CB, C, MB, true> : factor_kernel<R, NP, NW, CB, C, MB, false>;
     if (!smem_limit_max(kern, smem))
         return HELM3D_ERR_CUDA;
     cudaLaunchConfig_t cfg = {};
