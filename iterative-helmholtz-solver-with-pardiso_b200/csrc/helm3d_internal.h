@@ -150,8 +150,11 @@ int launch_kzinv(bool c64, const int *kzlist, int nskip, int nx, int ny, const v
 int launch_kzskip_apply(bool c64, const SweepArgs &a, cudaStream_t s);
 // the sweep's launch variants the autotuner times: stage and ring sizes of
 // the CUDA-core kernel (0-5), the tensor-core kernel on the packed factor
-// planned for two CTAs per SM (6, 7) or one (8, 9), ring depths 8 and 4
+// planned for two CTAs per SM (6, 7: ring depths 8 and 4) or one (8, 9: 4 and 8)
 constexpr int kSweepVariants = 10;
+// whether variant v is another launch than those before it: complex128 has no
+// tensor-core kernel, and with more than 128 rows that one has an SM to itself
+bool sweep_variant_own(bool c64, int n, int v);
 int sweep_default(bool c64, int n, int R);   // the variant of an untuned batch
 // power-of-two scale of every complex64 block G_j for the FP16 products
 int launch_gscale(const void *Gt, int n, int ny, int nz, int ldg, float *gscale, cudaStream_t s);

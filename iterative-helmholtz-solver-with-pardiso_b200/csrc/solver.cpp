@@ -608,6 +608,7 @@ int tune_solve(helm3d_ctx *c, int R, bool adjoint) {
     std::snprintf(shape, sizeof(shape), "t2|%d|%d|%d|%d|%d|%d", c->c64 ? 64 : 128, g.nx, g.ny, g.nz, R, adj);
     const SweepArgs s0 = sweep_args(c, R, adjoint);
     c->tv_sweep[adj] = tune_pick(c, "SWEEP", shape, kSweepVariants, [&](int v) {
+        if (!sweep_variant_own(c->c64, g.nx, v)) return (int)HELM3D_ERR_ARG;   // (not timed)
         SweepArgs t = s0;
         sweep_variant(v, t);
         return launch_sweep(c->c64, t, c->stream);

@@ -728,6 +728,8 @@ void sweep_variant(int v, SweepArgs &a) {
     a.tc_stages = kTcStages[v];
 }
 
+bool sweep_variant_own(bool c64, int n, int v) { return v < 6 || (c64 && (n <= 128 || v < 8)); }
+
 // The variant of a batch that no solve of this context has been tuned for:
 // the CUDA-core kernel, whose products are FP32 (the tensor cores' FP16 hi/lo
 // products add about a fifth to the complex64 preconditioner's error, 3.1e-6
