@@ -98,6 +98,7 @@ extern "C" int helm3d_apply_prec_noalloc(helm3d_ctx *c, const double *x, double 
     s.R = 1;
     s.dxy = nullptr;
     s.status = c->d_status;
+    sweep_variant(sweep_default(c->c64, s.n, 1), s);   // as an apply_prec that no solve was tuned for
     if (c->nskip > 0) {
         s.kzslot = c->d_kzslot;
         s.kzlist = c->d_kzlist;
