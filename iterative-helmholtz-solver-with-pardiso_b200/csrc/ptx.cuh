@@ -37,26 +37,9 @@ __device__ __forceinline__ void fence_mbar_init_cluster() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
-// arrive (release, cluster scope) on an mbarrier given by its cluster address
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-
 // local arrive (release, CTA scope)
 __device__ __forceinline__ void mbar_arrive_local(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t addr, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    return ok != 0;
 }
 
 __device__ __forceinline__ bool mbar_try_wait_cta(uint32_t addr, uint32_t parity) {
@@ -116,11 +99,6 @@ __device__ __forceinline__ void st_cluster_c(uint32_t addr, float2 v) { st_clust
 __device__ __forceinline__ void st_cluster_c(uint32_t addr, double2 v) { st_cluster_v2f64(addr, v.x, v.y); }
 
 // bounded wait: gives up after `limit` polls and reports false
-__device__ __forceinline__ bool mbar_wait_bounded_cluster(uint32_t addr, uint32_t parity, uint32_t limit) {
-    for (uint32_t it = 0; it < limit; ++it)
-        if (mbar_try_wait_cluster(addr, parity)) return true;
-    return false;
-}
 __device__ __forceinline__ bool mbar_wait_bounded_cta(uint32_t addr, uint32_t parity, uint32_t limit) {
     for (uint32_t it = 0; it < limit; ++it)
         if (mbar_try_wait_cta(addr, parity)) return true;
@@ -201,11 +179,6 @@ __device__ __forceinline__ void st_shared_v4_if(bool p, uint32_t addr, float4 v)
         "@q st.shared.v4.f32 [%1], {%2, %3, %4, %5};\n\t}" ::"r"((uint32_t)p),
         "r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
         : "memory");
-}
-__device__ __forceinline__ void st_shared_v2_if(bool p, uint32_t addr, float2 v) {
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q st.shared.v2.f32 [%1], {%2, %3};\n\t}" ::"r"((uint32_t)p),
-                 "r"(addr), "f"(v.x), "f"(v.y)
-                 : "memory");
 }
 __device__ __forceinline__ void st_shared_u32_if(bool p, uint32_t addr, uint32_t v) {
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q st.shared.u32 [%1], %2;\n\t}" ::"r"((uint32_t)p),

@@ -38,10 +38,6 @@ __host__ __device__ inline void tf32_split(double v, float &hi, float &lo) {
     hi = tf32_round((float)v);
     lo = tf32_round((float)(v - (double)hi));
 }
-__host__ __device__ inline void tf32_split_f(float v, float &hi, float &lo) {
-    hi = tf32_round(v);
-    lo = tf32_round(v - hi);
-}
 // the same split with lo left in FP32: v - hi is exact, and the tensor core
 // reads only its tf32 part, which drops less than 2^-21 |v|
 __host__ __device__ inline void tf32_split_fast(float v, float &hi, float &lo) {
@@ -118,17 +114,6 @@ __device__ __forceinline__ void umma_tf32_ts(uint32_t tmem_d, uint32_t tmem_a, u
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-        :
-        : "r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
-}
-
-// kind::f16: D (TMEM) (+)= A (TMEM: lane = row, two fp16 per column) B^T (shared memory), K = 16
-__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
-                                            uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
         :
         : "r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
 }
@@ -221,16 +206,8 @@ __device__ __forceinline__ void tmem_wait_ld(float (&v)[8]) {
                  : "memory");
 }
 
-// 16 / 32 consecutive fp32 columns into this warp's 32 TMEM lanes (lane =
-// thread); complete once tmem_wait_st() returns
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-        "%14, %15, %16};" ::"r"(taddr),
-        "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]),
-        "f"(v[9]), "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15])
-        : "memory");
-}
+// 32 consecutive fp32 columns into this warp's 32 TMEM lanes (lane = thread);
+// complete once tmem_wait_st() returns
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float (&v)[32]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
