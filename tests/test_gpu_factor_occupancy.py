@@ -4,17 +4,18 @@ SM (complex128, 256 threads) and for a fourth (complex64, 128 threads): at most
 B200)."""
 import pytest
 
-from cuda_kernels import kernels
-from helpers import mode_n_solver, small_problem
+from cuda_kernels import in_child
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("prec", [0, 1])
-def test_registers(prec, tmp_path, monkeypatch):
-    monkeypatch.setenv("HELM3D_FORCE_FACTOR", "0")
-    p = small_problem(20, 12, 8, pml=3, seed=6)
-    s = mode_n_solver(p, precision=prec)
-    ran = [k for k in kernels(lambda: s.set_medium(p.s2), tmp_path) if "factor_kernel" in k[0]]
-    s.close()
-    assert len(ran) == 2 and all(regs <= 128 for _, regs in ran), ran
+def test_registers():
+    got = in_child("""
+        out = []
+        for prec in (0, 1):
+            p = small_problem(20, 12, 8, pml=3, seed=6)
+            s = mode_n_solver(p, precision=prec)
+            out.append([k for k in kernels(lambda: s.set_medium(p.s2)) if "factor_kernel" in k[0]])
+        """, HELM3D_FORCE_FACTOR="0")
+    for ran in got:
+        assert len(ran) == 2 and all(regs <= 128 for _, regs in ran), ran
