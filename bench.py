@@ -308,9 +308,10 @@ def roofline_table(p, prof, its_per_source, nsrc, peaks):
 # DRAM read + write of one launch (ncu: dram__bytes_read.sum +
 # dram__bytes_write.sum of one captured launch), per (family, grid, sources)
 TRAFFIC = {
-    ("sweep", 128, 16): 5.273e9,
-    # the 200 x 200 x 32 capture of the packed sweep (4.825 GB) scaled by the kz chains, 200 / 32
-    ("sweep", 200, 16): 30.16e9,
+    # captures of the packed sweep on 128 x 128 x 32 (1.246 GB) and 200 x 200 x 32
+    # (4.838 GB), scaled by the kz chains: 128 / 32, 200 / 32
+    ("sweep", 128, 16): 4.99e9,
+    ("sweep", 200, 16): 30.24e9,
 }
 
 

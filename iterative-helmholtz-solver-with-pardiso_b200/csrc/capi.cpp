@@ -98,9 +98,9 @@ int validate(const helm3d_grid *g, const helm3d_opts *o) {
 
 // Start of a call that runs the operator or the preconditioner: refused
 // after a failed set-up or factor of this context (that error again), else
-// the device status word is cleared (unless it was last read as zero), so that a bounded wait that expired or
-// an index check that failed in an earlier call is not reported again (the
-// factor's own bits were reported when it ran).
+// the device status word is cleared (unless it was last read as zero), so that
+// a bounded wait that expired or an index check that failed in an earlier call
+// is not reported again (the factor's own bits were reported when it ran).
 int h3d::begin_call(helm3d_ctx *c) {
     if (c->factor_rc)
         return set_error(c, c->factor_rc,

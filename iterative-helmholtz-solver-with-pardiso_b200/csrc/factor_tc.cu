@@ -45,9 +45,8 @@
 //     buffered by step parity, so one barrier per step); the frame and the
 //     pivot order.  Half of TMEM and of shared memory: two CTAs share an SM.
 // Two chains on an SM hide each other's latencies, which is why X is in shared
-// memory and not in TMEM.  In ms, one CTA per SM with a whole GEMM after each
-// panel and the block unscrambled through shared memory -> look-ahead, frames and
-// two CTAs per SM: 40^3 0.60 -> 0.38, 96^3 5.13 -> 2.95, 128^3 9.66 -> 5.85.
+// memory and not in TMEM (96^3 2.95 ms, 128^3 5.85; one CTA per SM with a whole
+// GEMM after each panel and the block unscrambled 5.13, 9.66).
 // Every wait is bounded: on expiry bit 1 of *status is set and the kernel
 // runs on without waiting (results invalid), waits (bounded) for its MMAs,
 // frees its TMEM and returns.  A zero pivot, or a column without a finite

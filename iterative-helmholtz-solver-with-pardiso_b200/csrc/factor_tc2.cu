@@ -56,12 +56,16 @@
 // row warps wait for only before they write panel p+1's X.  A finished line is
 // written, and the next one formed, by all eight warps.
 //
-// 200 x 200 x 74 in ms: the row warps alone, with branches 39.7; steps without
-// branches 36.9, 1 / pivot before the barrier 35.8, helpers 32.3, a line's
-// entries by selects and predicated stores 30.6, the first block by all warps
-// 29.6.  A step is 725 cycles: store the candidate 130, barrier 25, keys 105, the
-// row 85, the next column's update and reduction 180, the other columns 160.
-// Eight row warps of one row each took 36.9 -> 38.7: more warps at each barrier.
+// 200 x 200 x 74: 39.7 ms by the row warps alone with branches in a step, 29.6 so.
+// A step is 725 cycles: store the candidate 130, barrier 25, keys 105, the row 85,
+// the next column's update and reduction 180, the other columns 160.  Eight row
+// warps of one row each were slower by 5 %: more warps at each barrier.
+//
+// Tensor memory.  Two kernels whose clusters hold some on one SM while they wait
+// for some on another could wait for each other.  The only other cluster kernel
+// with tensor memory is the packed sweep (352 threads of at least 80 registers),
+// and beside a CTA of this one (256 threads of at least 168) an SM has registers
+// for 64 each: the two never share an SM.
 //
 // Every wait is bounded: on expiry bit 1 of *status is set and the kernel
 // runs on without waiting (results invalid), waits (bounded) for its MMAs,

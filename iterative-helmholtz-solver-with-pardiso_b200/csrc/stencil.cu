@@ -9,9 +9,9 @@
 // plane's loads in flight, or three in a ring of shared-memory planes, reached
 // 37-46 % of it.  stencil_block_kernel: a CTA owns 32 x 8 x ZB points, copies
 // them with their halo into shared memory at once (asynchronous copies,
-// zero-filled off the grid, which is the operator's u = 0 there), s2 and f into
+// zero-filled off the grid, which is the operator's u = 0 there), s2 into
 // registers meanwhile, and goes through the ZB planes from shared memory, the z
-// neighbours in registers.  stencil_kernel: the same from registers and L1
+// neighbours in registers, f (a residual's) read as its plane comes.  stencil_kernel: the same from registers and L1
 // without a barrier, a thread per ZB points of a column, for grids too small to
 // fill the SMs with such blocks.  The grid's z dimension enumerates (source, z
 // block) pairs, source-major or source-minor (autotuned, with ZB).  The input x

@@ -696,9 +696,9 @@ template <typename R, bool ADJ> static int sweep_n(const SweepArgs &sa, cudaStre
     if constexpr (sizeof(R) == 4) {
         // (three or four sources of up to 64 rows: 88 us by sweep_kernel at 64^3,
         // 93 by this.)  Warps of 8 or 16 rows by whichever leaves the four
-        // schedulers of an SM the same number: 96 rows as 12 warps of 8 rows,
-        // 16 sources, 1075 us, as 6 of 16 rows 1290; 160 rows (x 128 x 60) as
-        // 10 of 16 1980, as 5 of 32 2550; 200 rows as 13 2873, as 7 2922
+        // schedulers of an SM the same number: 16 sources of 96 rows are 1.2
+        // times slower as 6 warps of 16 rows than as 12 of 8, of 160 rows 1.3
+        // times as 5 of 32 than as 10 of 16, of 200 rows the same either way
         if (sa.R > 4 || (sa.R > 2 && sa.n > 64)) {
             if (sa.n <= 32) return sweep_batch<8, ADJ, 4>(sa, s);
             if (sa.n <= 64) return sweep_batch<8, ADJ, 8>(sa, s);
