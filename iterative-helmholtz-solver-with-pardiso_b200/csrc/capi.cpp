@@ -548,7 +548,7 @@ int helm3d_misfit_grad(helm3d_ctx *c, const double *f, int nsrc, const long long
     int rc;
     // receivers: checked on the host, used from the device
     std::vector<long long> hrecv((size_t)nrecv);
-    DevBuf d_recv, d_data, d_grad, d_u, d_lam, d_res;
+    DevBuf d_recv, d_data, d_grad, d_u, d_res;
     if (nrecv > 0) {
         if ((rc = cuda_check(c, cudaMemcpy(hrecv.data(), recv, sizeof(long long) * nrecv, cudaMemcpyDefault),
                              "receivers")))
@@ -578,12 +578,12 @@ int helm3d_misfit_grad(helm3d_ctx *c, const double *f, int nsrc, const long long
     const bool fstaged = !is_device_ptr(f);
     const int B = batch_size(c, nsrc, fstaged, 2);
     const size_t vb = sizeof(double2) * (size_t)N;
-    // given back at the end of the call (1.4 of 25.7 ms at 96^3 with 8 sources):
+    // given back at the end of the call (0.8 of 25.2 ms at 96^3 with 8 sources, 1.4 by two allocations):
     // kept by the context, other contexts and the caller would lose them
-    if ((rc = d_u.alloc(c, vb * B, "wavefields")) || (rc = d_lam.alloc(c, vb * B, "adjoint wavefields")) ||
+    if ((rc = d_u.alloc(c, 2 * vb * B, "wavefields")) ||
         (nrecv > 0 && (rc = d_res.alloc(c, sizeof(double2) * (size_t)B * nrecv, "receiver residuals"))))
         return rc;
-    double2 *U = (double2 *)d_u.p, *Lam = (double2 *)d_lam.p, *Res = (double2 *)d_res.p;
+    double2 *U = (double2 *)d_u.p, *Lam = U + (size_t)B * N, *Res = (double2 *)d_res.p;
     std::vector<double2> hres((size_t)B * std::max(nrecv, 0));
     const double w2 = c->grid.omega * c->grid.omega;
     double J = 0.0;
